@@ -337,12 +337,12 @@ static int enqueue_step(harm_ctx* c, int precision, int guess, double* d_P, bool
   // bound_prim (post_advance step_ch.c:288-330)
   if (hp_bound(c, c->d_pk, c->d_pflag)) return 1;
   if (hp_fixup(c, c->d_pk, c->d_pflag, 0, false)) return 1;
-  if (hp_bound(c, c->d_pk, nullptr)) return 1;
+  if (hp_bound(c, c->d_pk, nullptr, c->d_nrec)) return 1;
   if (substep(c, precision, guess, 1, 2, d_P, c->d_pk, d_P, c->d_pflag, CUf[1], Cun[1], c->d_dtslots + 3, with_stats))
     return 1;
   if (hp_bound(c, d_P, c->d_pflag)) return 1;
   if (hp_fixup(c, d_P, c->d_pflag, 1, false)) return 1;
-  if (hp_bound(c, d_P, nullptr)) return 1;
+  if (hp_bound(c, d_P, nullptr, c->d_nrec)) return 1;
   return hp_finalize_dt(c, c->d_dt, c->d_ndt, 2);
 }
 

@@ -53,8 +53,20 @@ __global__ void k_copy_ghosts(Dims d, const double* __restrict__ pb, double* __r
 //       (POLEDEATH 1, POLEINTERPTYPE 3) and POLEGAMMADEATH's Lorentz-factor limit there,
 //       over every i of the extended grid;
 //   x3: periodic (:1114), over every (i,j) of the extended grid.
-// One thread per boundary line; the arithmetic is the oracle's (oracle/orc_bound.c) in the
-// same order.
+// k_bound does all three in one launch: one thread per written cell, each pulling its value
+// through the directions in reverse (x3: the periodic partner's plane; x2: the mirrored row, or
+// for the two pole rows the second active row; x1: the extrapolation of that row), so nothing
+// it reads is written by the launch: the pole rewrites only the density, energy and velocity
+// (in 2-D also B3) of the first active rows, and those are replaced from the second row in
+// every cell that derives from them.  The chain of one cell is what bounds it (a few dependent
+// loads, the logarithms of the slopes).  As three or four kernels of one thread per boundary
+// line with a serial loop over its ghost cells a full step took 403 us at 128x128x1 (MC, FP64)
+// and 1764 us at 192x96x64 (PARALINE, mixed); with k_bound 293 and 1584 us, results the same
+// bit for bit.
+// The mirrored and periodic sources have to be active cells that the launch does not write
+// (n2 > ng, n3 >= ng); smaller grids take the directions as separate launches (k_bound_x1,
+// k_bound_x2_reflect, k_bound_x2_pole, k_bound_x3).  The arithmetic is the oracle's
+// (oracle/orc_bound.c) in the same order.
 
 #define BMINMOD(a, b) (((a) * (b) <= 0) ? 0.0 : ((fabs(a) < fabs(b)) ? (a) : (b)))
 
@@ -63,20 +75,19 @@ __device__ __forceinline__ void cent_geo(const Dims& d, const double* __restrict
   load_geo<double, double>(geom + (size_t)HARM_LOC_CENT * HARM_NGF * d.plane, d.plane, (size_t)jj * d.n1e + ii, g);
 }
 
-// extrapfunc for the ghost cells of the x1 line (jj,kk) on one side
-__global__ void k_bound_x1_extrap(Dims d, Phys ph, double* __restrict__ P, const double* __restrict__ geom) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2LL * d.n2 * d.n3) return;
-  const int up = (int)(t & 1);
-  long long r = t >> 1;
-  const int jj = (int)(r % d.n2) + d.ng, kk = (int)(r / d.n2) + d.ng3;
+// extrapfunc for the x1 ghost cell ii of the active line (jj,kk), with the outer boundary's
+// inflow check and Lorentz-factor limit
+__device__ __forceinline__ void x1_ghost(const Dims& d, const Phys& ph, const double* P, const double* __restrict__ geom,
+                                         int ii, int jj, int kk, double* p) {
+  const int up = ii >= d.ng + d.n1;
   const int ri = up ? d.ng + d.n1 - 1 : d.ng;
   const int ri2 = up ? ri - 1 : ri + 1, ri3 = up ? ri - 2 : ri + 2;
   const double signdq = up ? -1.0 : 1.0;
-  Geo<double> gr, g2, g3;
+  Geo<double> gr, g2, g3, gi;
   cent_geo(d, geom, ri, jj, gr);
   cent_geo(d, geom, ri2, jj, g2);
   cent_geo(d, geom, ri3, jj, g3);
+  cent_geo(d, geom, ii, jj, gi);
   double p1[NPR], p2[NPR], p3[NPR];
   const size_t c1 = cidx(d, ri, jj, kk), c2 = cidx(d, ri2, jj, kk), c3 = cidx(d, ri3, jj, kk);
 #pragma unroll
@@ -86,29 +97,37 @@ __global__ void k_bound_x1_extrap(Dims d, Phys ph, double* __restrict__ P, const
     p3[pl] = P[(size_t)pl * d.cells + c3];
   }
   double Bd3 = 0.0, Bd3ri2 = 0.0, Bd3ri3 = 0.0;
+#pragma unroll
   for (int a = 1; a <= 3; a++) Bd3 += p1[HARM_B1 + a - 1] * gr.gcov[sym(3, a)];
+#pragma unroll
   for (int a = 1; a <= 3; a++) Bd3ri2 += p2[HARM_B1 + a - 1] * g2.gcov[sym(3, a)];
+#pragma unroll
   for (int a = 1; a <= 3; a++) Bd3ri3 += p3[HARM_B1 + a - 1] * g3.gcov[sym(3, a)];
   double Dqp = Bd3ri3 - Bd3ri2, Dqm = Bd3ri2 - Bd3, Dqc = Bd3ri3 - Bd3;
   const double dqBd3 = signdq * BMINMOD(BMINMOD(Dqp, Dqm), Dqc);
   double ucref[4], ucref2[4], gam, qsq;
   ucon_of<double>(p1, gr, ucref, gam, qsq);
   ucon_of<double>(p2, g2, ucref2, gam, qsq);
-  double dq[NPR], dqlog[NPR], dqgd[NPR];
+  double dq[NPR], dqlog[HARM_UU + 1], lp1[HARM_UU + 1], dqgd[NPR];
 #pragma unroll
   for (int pl = 0; pl < NPR; pl++) {
     Dqp = p3[pl] - p2[pl];
     Dqm = p2[pl] - p1[pl];
     Dqc = p3[pl] - p1[pl];
     dq[pl] = signdq * BMINMOD(BMINMOD(Dqp, Dqm), Dqc);
-    Dqp = log(1.e-300 + fabs(p3[pl])) - log(1.e-300 + fabs(p2[pl]));
-    Dqm = log(1.e-300 + fabs(p2[pl])) - log(1.e-300 + fabs(p1[pl]));
-    Dqc = log(1.e-300 + fabs(p3[pl])) - log(1.e-300 + fabs(p1[pl]));
-    dqlog[pl] = signdq * BMINMOD(BMINMOD(Dqp, Dqm), Dqc);
     Dqp = g3.gdet * p3[pl] - g2.gdet * p2[pl];
     Dqm = g2.gdet * p2[pl] - gr.gdet * p1[pl];
     Dqc = g3.gdet * p3[pl] - gr.gdet * p1[pl];
     dqgd[pl] = signdq * BMINMOD(BMINMOD(Dqp, Dqm), Dqc);
+  }
+#pragma unroll
+  for (int pl = HARM_RHO; pl <= HARM_UU; pl++) {
+    const double l1 = log(1.e-300 + fabs(p1[pl])), l2 = log(1.e-300 + fabs(p2[pl])), l3 = log(1.e-300 + fabs(p3[pl]));
+    Dqp = l3 - l2;
+    Dqm = l2 - l1;
+    Dqc = l3 - l1;
+    dqlog[pl] = signdq * BMINMOD(BMINMOD(Dqp, Dqm), Dqc);
+    lp1[pl] = l1;
   }
   // the slopes of u and the velocities fade out where u^t jumps between ri and ri2
   const double xdqfrac = fabs(ucref[0] - ucref2[0]) / ucref[0];
@@ -117,69 +136,192 @@ __global__ void k_bound_x1_extrap(Dims d, Phys ph, double* __restrict__ P, const
   else if (xdqfrac < 0.2) ydqfrac = (0.0 + (1.0 - 0.0) / (0.2 - 0.1) * (xdqfrac - 0.1));
   else ydqfrac = 1.0;
 #pragma unroll
-  for (int a = 0; a < 4; a++) {
-    dq[HARM_UU + a] = dq[HARM_UU + a] * (1.0 - ydqfrac);
-    dqlog[HARM_UU + a] = dqlog[HARM_UU + a] * (1.0 - ydqfrac);
-  }
+  for (int a = 0; a < 4; a++) dq[HARM_UU + a] = dq[HARM_UU + a] * (1.0 - ydqfrac);
+  dqlog[HARM_UU] = dqlog[HARM_UU] * (1.0 - ydqfrac);
   const double powerratio = (1.0 + (0.1));
-  for (int q = 1; q <= d.ng; q++) {
-    const int ii = up ? ri + q : ri - q;
-    const double di = (double)(ii - ri);
-    Geo<double> gi;
-    cent_geo(d, geom, ii, jj, gi);
-    double p[NPR];
+  const double di = (double)(ii - ri);
 #pragma unroll
-    for (int pl = 0; pl < NPR; pl++) p[pl] = p1[pl];
+  for (int pl = 0; pl < NPR; pl++) p[pl] = p1[pl];
 #pragma unroll
-    for (int pl = HARM_RHO; pl <= HARM_UU; pl++) {
-      double ftemp = exp(-signdq * dqlog[pl]) - powerratio, mydqlog;
-      if (ftemp >= 0.0) mydqlog = log(powerratio) / (-signdq);
-      else mydqlog = dqlog[pl];
-      p[pl] = exp(log(1.e-300 + fabs(p1[pl])) + mydqlog * di);
+  for (int pl = HARM_RHO; pl <= HARM_UU; pl++) {
+    double ftemp = exp(-signdq * dqlog[pl]) - powerratio, mydqlog;
+    if (ftemp >= 0.0) mydqlog = log(powerratio) / (-signdq);
+    else mydqlog = dqlog[pl];
+    p[pl] = exp(lp1[pl] + mydqlog * di);
+  }
+#pragma unroll
+  for (int pl = HARM_U1; pl <= HARM_U3; pl++) p[pl] = p1[pl] + dq[pl] * di;
+#pragma unroll
+  for (int pl = HARM_B1; pl <= HARM_B2; pl++) {
+    const double igd = copysign(1.0, gi.gdet) / (fabs(gi.gdet) + 1.e-300);
+    p[pl] = (p1[pl] * fabs(gr.gdet + dqgd[pl] * di)) * igd;
+  }
+  {
+    const double Bu1 = p[HARM_B1], Bu2 = p[HARM_B2];
+    const double gcon03 = gi.gcon[sym(0, 3)], gcon13 = gi.gcon[sym(1, 3)], gcon23 = gi.gcon[sym(2, 3)],
+                 gcon33 = gi.gcon[sym(3, 3)];
+    const double gcov01 = gi.gcov[sym(0, 1)], gcov02 = gi.gcov[sym(0, 2)], gcov11 = gi.gcov[sym(1, 1)],
+                 gcov12 = gi.gcov[sym(1, 2)], gcov21 = gcov12, gcov22 = gi.gcov[sym(2, 2)],
+                 gcov03 = gi.gcov[sym(0, 3)], gcov13 = gi.gcov[sym(1, 3)], gcov23 = gi.gcov[sym(2, 3)];
+    const double myBd3 = Bd3 + dqBd3 * di;
+    const double ftemp = (1.0 - gcon03 * gcov03 - gcon13 * gcov13 - gcon23 * gcov23);
+    const double igd = copysign(1.0, ftemp) / (fabs(ftemp) + 1.e-300);
+    p[HARM_B3] = (myBd3 * gcon33 + Bu1 * gcon03 * gcov01 + Bu2 * gcon03 * gcov02 + Bu1 * gcon13 * gcov11 +
+                  Bu2 * gcon13 * gcov12 + Bu1 * gcon23 * gcov21 + Bu2 * gcon23 * gcov22) * igd;
+  }
+  if (up) {
+    // inflow_check_rel4vel (fixup.c:3255) for the outer radial boundary, then limit_gamma
+    double ucon[4], gamma, qsq2;
+    ucon_of<double>(p, gi, ucon, gamma, qsq2);
+    if (ucon[1] < 0.) {
+      p[HARM_U1] /= gamma; p[HARM_U2] /= gamma; p[HARM_U3] /= gamma;
+      double alpha = 1. / sqrt(-gi.gcon[0]);
+      double betacon = gi.gcon[1] * alpha * alpha;
+      p[HARM_U1] = betacon / alpha;
+      double vsq = 0.;
+#pragma unroll
+      for (int a = 1; a < 4; a++)
+#pragma unroll
+        for (int b = 1; b < 4; b++) vsq += gi.gcov[sym(a, b)] * p[HARM_U1 + a - 1] * p[HARM_U1 + b - 1];
+      if (vsq < 0.0 && vsq > -2.220446049250313e-16 * 100.0) vsq = 0.0;
+      if (vsq >= 1.0) vsq = 1.0 - 1.0 / (ph.gammamax * ph.gammamax);
+      gamma = 1. / sqrt(1. - vsq);
+      p[HARM_U1] *= gamma; p[HARM_U2] *= gamma; p[HARM_U3] *= gamma;
     }
+    limit_gamma<double>(ph.gammamax, p, gi);
+  }
+}
+
+// poledeath and POLEGAMMADEATH of the pole row j (active-relative: the ghost row or the first
+// active row of a pole) in column ii: p holds the row's own state and r the second active
+// row's; p takes rho, u, U1, U3 (and B3 in 2-D) of r; U2 is r's extrapolated linearly to zero
+// at the pole, or zero where it flows into the pole; then the Lorentz factor is limited (1.1,
+// growing as r/10 beyond r = 10, where u^r > 0; GAMMAMAX otherwise)
+__device__ __forceinline__ void pole_row(const Dims& d, const Phys& ph, double startx2, const double* __restrict__ geom,
+                                         const double* __restrict__ aux, int up, int j, int ii, const double* r,
+                                         double* p) {
+  const int rj = up ? d.n2 - 2 : 1, poleloc = up ? d.n2 : 0, jj = j + d.ng;
+  const double Xr2 = startx2 + (rj + 0 + 0.5) * ph.dx2, X02 = startx2 + (poleloc + 0) * ph.dx2;
+  const double X2 = startx2 + (j + 0 + 0.5) * ph.dx2;
+  p[HARM_RHO] = r[HARM_RHO];
+  p[HARM_UU] = r[HARM_UU];
+  p[HARM_U1] = r[HARM_U1];
+  p[HARM_U3] = r[HARM_U3];
+  double ftemp = r[HARM_U2];
+  if ((!up && ftemp > 0.0) || (up && ftemp < 0.0)) ftemp = 0.0;
+  p[HARM_U2] = ftemp + (X2 - Xr2) * (ftemp - 0.0) / (Xr2 - X02);
+  if (d.n3 == 1) p[HARM_B3] = r[HARM_B3];
+  Geo<double> gi;
+  cent_geo(d, geom, ii, jj, gi);
+  double ucon[4], gamma, qsq;
+  ucon_of<double>(p, gi, ucon, gamma, qsq);
+  if (ucon[1] > 0.0) {
+    const double rr = aux[(size_t)HARM_AUX_R * d.plane + (size_t)jj * d.n1e + ii];
+    const double lim = (rr <= 10.0) ? 1.1 : 1.1 * pow(rr / 10.0, 1.0);
+    limit_gamma<double>(lim, p, gi);
+  } else {
+    limit_gamma<double>(ph.gammamax, p, gi);
+  }
+}
+
+__device__ __forceinline__ void load_cell(const Dims& d, const double* P, size_t c, double* p) {
 #pragma unroll
-    for (int pl = HARM_U1; pl <= HARM_U3; pl++) p[pl] = p1[pl] + dq[pl] * di;
-#pragma unroll
-    for (int pl = HARM_B1; pl <= HARM_B2; pl++) {
-      const double igd = copysign(1.0, gi.gdet) / (fabs(gi.gdet) + 1.e-300);
-      p[pl] = (p1[pl] * fabs(gr.gdet + dqgd[pl] * di)) * igd;
+  for (int pl = 0; pl < NPR; pl++) p[pl] = P[(size_t)pl * d.cells + c];
+}
+
+// the sections of one k_bound launch, in blocks of 128 threads: x1 ghost cells over the whole
+// j, k extent; x2 ghost rows and the first active row of each pole over active i and the whole
+// k extent; the other x3 ghost cells; with flags, their x3 ghost planes
+struct BoundBlocks {
+  unsigned int x1, x2, x3, fl;
+};
+
+// only_if (optional): nothing is done where *only_if is 0 (the second bound of a substep, whose
+// input is the first one's output where post_fixup recorded no fix: every boundary value is
+// then what it already is)
+__global__ void __launch_bounds__(128) k_bound(Dims d, Phys ph, double startx2, double* P, const double* __restrict__ geom,
+                                               const double* __restrict__ aux, int8_t* flag, BoundBlocks nb,
+                                               const unsigned int* __restrict__ only_if) {
+  if (only_if && *only_if == 0u) return;
+  unsigned int blk = blockIdx.x;
+  auto active_k = [&](int kk) { return (kk < d.ng3) ? kk + d.n3 : (kk >= d.ng3 + d.n3) ? kk - d.n3 : kk; };
+  if (blk < nb.x1 + nb.x2) {
+    const bool ghost1 = blk < nb.x1;
+    if (!ghost1) blk -= nb.x1;
+    // x1 ghosts: (2 ng) x n2e x n3e cells; x2 rows: n1 x (2 ng + 2) x n3e cells
+    const int w = ghost1 ? 2 * d.ng : d.n1, h = ghost1 ? d.n2e : 2 * d.ng + 2;
+    const long long t = (long long)blk * 128 + threadIdx.x;
+    if (t >= (long long)w * h * d.n3e) return;
+    const int x = (int)(t % w);
+    const long long r = t / w;
+    const int y = (int)(r % h), kk = (int)(r / h);
+    const int ii = ghost1 ? ((x < d.ng) ? x : x + d.n1) : x + d.ng;
+    const int jj = ghost1 ? y : ((y <= d.ng) ? y : y + d.n2 - 2);
+    const int j = jj - d.ng, ks = active_k(kk);
+    const int js = (j < 0) ? -j - 1 : (j >= d.n2) ? 2 * d.n2 - 1 - j : j;  // the mirrored row
+    const int up = j >= d.n2 - 1;
+    const bool pole = (j >= -1 && j <= 0) || (j >= d.n2 - 1 && j <= d.n2);
+    double p[NPR], q[NPR];
+    if (ghost1) x1_ghost(d, ph, P, geom, ii, js + d.ng, ks, p);
+    else load_cell(d, P, cidx(d, ii, js + d.ng, ks), p);
+    if (js != j) {
+      p[HARM_U2] *= -1.;
+      p[HARM_B2] *= -1.;
     }
-    {
-      const double Bu1 = p[HARM_B1], Bu2 = p[HARM_B2];
-      const double gcon03 = gi.gcon[sym(0, 3)], gcon13 = gi.gcon[sym(1, 3)], gcon23 = gi.gcon[sym(2, 3)],
-                   gcon33 = gi.gcon[sym(3, 3)];
-      const double gcov01 = gi.gcov[sym(0, 1)], gcov02 = gi.gcov[sym(0, 2)], gcov11 = gi.gcov[sym(1, 1)],
-                   gcov12 = gi.gcov[sym(1, 2)], gcov21 = gcov12, gcov22 = gi.gcov[sym(2, 2)],
-                   gcov03 = gi.gcov[sym(0, 3)], gcov13 = gi.gcov[sym(1, 3)], gcov23 = gi.gcov[sym(2, 3)];
-      const double myBd3 = Bd3 + dqBd3 * di;
-      const double ftemp = (1.0 - gcon03 * gcov03 - gcon13 * gcov13 - gcon23 * gcov23);
-      const double igd = copysign(1.0, ftemp) / (fabs(ftemp) + 1.e-300);
-      p[HARM_B3] = (myBd3 * gcon33 + Bu1 * gcon03 * gcov01 + Bu2 * gcon03 * gcov02 + Bu1 * gcon13 * gcov11 +
-                    Bu2 * gcon13 * gcov12 + Bu1 * gcon23 * gcov21 + Bu2 * gcon23 * gcov22) * igd;
-    }
-    if (up) {
-      // inflow_check_rel4vel (fixup.c:3255) for the outer radial boundary, then limit_gamma
-      double ucon[4], gamma, qsq2;
-      ucon_of<double>(p, gi, ucon, gamma, qsq2);
-      if (ucon[1] < 0.) {
-        p[HARM_U1] /= gamma; p[HARM_U2] /= gamma; p[HARM_U3] /= gamma;
-        double alpha = 1. / sqrt(-gi.gcon[0]);
-        double betacon = gi.gcon[1] * alpha * alpha;
-        p[HARM_U1] = betacon / alpha;
-        double vsq = 0.;
-        for (int a = 1; a < 4; a++)
-          for (int b = 1; b < 4; b++) vsq += gi.gcov[sym(a, b)] * p[HARM_U1 + a - 1] * p[HARM_U1 + b - 1];
-        if (vsq < 0.0 && vsq > -2.220446049250313e-16 * 100.0) vsq = 0.0;
-        if (vsq >= 1.0) vsq = 1.0 - 1.0 / (ph.gammamax * ph.gammamax);
-        gamma = 1. / sqrt(1. - vsq);
-        p[HARM_U1] *= gamma; p[HARM_U2] *= gamma; p[HARM_U3] *= gamma;
-      }
-      limit_gamma<double>(ph.gammamax, p, gi);
+    if (pole) {
+      const int rj = (up ? d.n2 - 2 : 1) + d.ng;
+      if (ghost1) x1_ghost(d, ph, P, geom, ii, rj, ks, q);
+      else load_cell(d, P, cidx(d, ii, rj, ks), q);
+      pole_row(d, ph, startx2, geom, aux, up, j, ii, q, p);
     }
     const size_t c = cidx(d, ii, jj, kk);
+    // an active cell's field is its own (other cells of this launch read it), but for B3 in 2-D
+    const bool active = !ghost1 && js == j && ks == kk;
 #pragma unroll
-    for (int pl = 0; pl < NPR; pl++) P[(size_t)pl * d.cells + c] = p[pl];
+    for (int pl = 0; pl < NPR; pl++)
+      if (!active || pl < HARM_B1 || (pl == HARM_B3 && d.n3 == 1)) P[(size_t)pl * d.cells + c] = p[pl];
+    return;
   }
+  blk -= nb.x1 + nb.x2;
+  if (blk < nb.x3) {  // the x3 ghosts of the rows that neither pole rewrites
+    const long long t = (long long)blk * 128 + threadIdx.x;
+    const int h = d.n2 - 2;
+    if (t >= (long long)d.n1 * h * 2 * d.ng3) return;
+    const int ii = (int)(t % d.n1) + d.ng;
+    const long long r = t / d.n1;
+    const int jj = (int)(r % h) + 1 + d.ng, z = (int)(r / h);
+    const int kk = (z < d.ng3) ? z : z + d.n3;
+    const size_t dst = cidx(d, ii, jj, kk);
+    double p[NPR];
+    load_cell(d, P, cidx(d, ii, jj, active_k(kk)), p);
+#pragma unroll
+    for (int pl = 0; pl < NPR; pl++) P[(size_t)pl * d.cells + dst] = p[pl];
+    return;
+  }
+  blk -= nb.x3;
+  {
+    const long long t = (long long)blk * 128 + threadIdx.x;
+    if (t >= (long long)d.plane * 2 * d.ng3) return;
+    const int z = (int)(t / (long long)d.plane);
+    const size_t c = (size_t)(t % (long long)d.plane);
+    const int kk = (z < d.ng3) ? z : z + d.n3;
+    flag[(size_t)kk * d.plane + c] = flag[(size_t)active_k(kk) * d.plane + c];
+  }
+}
+
+// The directions one after the other, for grids whose mirrored or periodic sources are
+// themselves ghost cells or pole rows (k_bound's comment).
+__global__ void k_bound_x1(Dims d, Phys ph, double* __restrict__ P, const double* __restrict__ geom) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 2LL * d.ng * d.n2 * d.n3) return;
+  const int x = (int)(t % (2 * d.ng));
+  const long long r = t / (2 * d.ng);
+  const int ii = (x < d.ng) ? x : x + d.n1, jj = (int)(r % d.n2) + d.ng, kk = (int)(r / d.n2) + d.ng3;
+  double p[NPR];
+  x1_ghost(d, ph, P, geom, ii, jj, kk, p);
+  const size_t c = cidx(d, ii, jj, kk);
+#pragma unroll
+  for (int pl = 0; pl < NPR; pl++) P[(size_t)pl * d.cells + c] = p[pl];
 }
 
 // polar reflection of the ghost rows of column (ii,kk) at both poles
@@ -202,11 +344,7 @@ __global__ void k_bound_x2_reflect(Dims d, double* __restrict__ P) {
   }
 }
 
-// poledeath and POLEGAMMADEATH of column (ii,kk) at one pole: the ghost cell and the first
-// active cell take rho, u, U1, U3 (and B3 in 2-D) of the second active cell; U2 there is the
-// second cell's extrapolated linearly to zero at the pole, or zero where it flows into the
-// pole; then the Lorentz factor is limited (1.1, growing as r/10 beyond r = 10, where u^r > 0;
-// GAMMAMAX otherwise)
+// the pole rows of column (ii,kk) at one pole
 __global__ void k_bound_x2_pole(Dims d, Phys ph, double startx2, double* __restrict__ P,
                                 const double* __restrict__ geom, const double* __restrict__ aux) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -214,38 +352,13 @@ __global__ void k_bound_x2_pole(Dims d, Phys ph, double startx2, double* __restr
   const int up = (int)(t & 1);
   long long r = t >> 1;
   const int ii = (int)(r % d.n1e), kk = (int)(r / d.n1e) + d.ng3;
-  const int rj = up ? d.n2 - 2 : 1, js = up ? d.n2 - 1 : -1, poleloc = up ? d.n2 : 0;
-  const double Xr2 = startx2 + (rj + 0 + 0.5) * ph.dx2, X02 = startx2 + (poleloc + 0) * ph.dx2;
-  const size_t cr = cidx(d, ii, rj + d.ng, kk);
+  const int rj = up ? d.n2 - 2 : 1, js = up ? d.n2 - 1 : -1;
+  double ref[NPR], p[NPR];
+  load_cell(d, P, cidx(d, ii, rj + d.ng, kk), ref);
   for (int j = js; j <= js + 1; j++) {
     const size_t c = cidx(d, ii, j + d.ng, kk);
-#pragma unroll
-    for (int pl = HARM_RHO; pl <= HARM_U3; pl++) {
-      if (pl == HARM_U2) continue;
-      P[(size_t)pl * d.cells + c] = P[(size_t)pl * d.cells + cr];
-    }
-    double ftemp = P[(size_t)HARM_U2 * d.cells + cr];
-    const double X2 = startx2 + (j + 0 + 0.5) * ph.dx2;
-    if ((!up && ftemp > 0.0) || (up && ftemp < 0.0)) ftemp = 0.0;
-    P[(size_t)HARM_U2 * d.cells + c] = ftemp + (X2 - Xr2) * (ftemp - 0.0) / (Xr2 - X02);
-    if (d.n3 == 1) P[(size_t)HARM_B3 * d.cells + c] = P[(size_t)HARM_B3 * d.cells + cr];
-  }
-  for (int j = js; j <= js + 1; j++) {
-    const int jj = j + d.ng;
-    const size_t c = cidx(d, ii, jj, kk);
-    Geo<double> gi;
-    cent_geo(d, geom, ii, jj, gi);
-    double p[NPR], ucon[4], gamma, qsq;
-#pragma unroll
-    for (int pl = 0; pl < NPR; pl++) p[pl] = P[(size_t)pl * d.cells + c];
-    ucon_of<double>(p, gi, ucon, gamma, qsq);
-    if (ucon[1] > 0.0) {
-      const double rr = aux[(size_t)HARM_AUX_R * d.plane + (size_t)jj * d.n1e + ii];
-      const double lim = (rr <= 10.0) ? 1.1 : 1.1 * pow(rr / 10.0, 1.0);
-      limit_gamma<double>(lim, p, gi);
-    } else {
-      limit_gamma<double>(ph.gammamax, p, gi);
-    }
+    load_cell(d, P, c, p);
+    pole_row(d, ph, startx2, geom, aux, up, j, ii, ref, p);
 #pragma unroll
     for (int pl = 0; pl < NPR; pl++) P[(size_t)pl * d.cells + c] = p[pl];
   }
@@ -268,12 +381,13 @@ __global__ void k_bound_x3(Dims d, double* P, int8_t* flag) {
 }
 
 // Ghost flags for post_fixup's neighbour test, as bound_pflag_user (boundsint.c:18) sets
-// them for the torus, in its order: x3 periodic first over the full i, j extent (k_bound_x3;
-// ghost cells in x1 or x2 of the x3 ghost planes so take the values their periodic partners
-// hold from the previous call), then the x1 outer OUTFLOW copy of the last active cell over
-// the active j, k (k_bound_flags_x1; the inner x1 boundary is FREEOUTFLOW, which leaves its
-// ghost flags alone), then the x2 POLARAXIS mirror within the same k plane over the full i
-// extent and the active k (k_bound_flags_x2).
+// them for the torus, in its order: x3 periodic first over the full i, j extent (k_bound or
+// k_bound_x3; ghost cells in x1 or x2 of the x3 ghost planes so take the values their periodic
+// partners hold from the previous call), then the x1 outer OUTFLOW copy of the last active cell
+// over the active j, k (the inner x1 boundary is FREEOUTFLOW, which leaves its ghost flags
+// alone), then the x2 POLARAXIS mirror within the same k plane over the full i extent and the
+// active k.  The last two are written by k_fixup_compute as it scans the active cells; grids
+// too small for k_bound take k_bound_flags_x1 and k_bound_flags_x2 before it.
 __global__ void k_bound_flags_x1(Dims d, int8_t* flag) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long n = (long long)d.ng * d.n2 * d.n3;
@@ -298,6 +412,17 @@ __global__ void k_bound_flags_x2(Dims d, int8_t* flag) {
   flag[cidx(d, ii, jj, kk)] = flag[cidx(d, ii, js, kk)];
 }
 
+// the flag that the boundary order above gives cell (ii, jj, kk) within one cell of the active
+// ones, from the active cells' flags, the inner x1 ghost flags and the x3 ghost planes alone
+__device__ __forceinline__ int8_t flag_at(const Dims& d, const int8_t* flag, int ii, int jj, int kk) {
+  if (kk >= d.ng3 && kk < d.ng3 + d.n3) {
+    if (jj < d.ng) jj = 2 * d.ng - 1 - jj;
+    else if (jj >= d.ng + d.n2) jj = 2 * (d.ng + d.n2) - 1 - jj;
+    if (ii >= d.ng + d.n1) ii = d.ng + d.n1 - 1;
+  }
+  return flag[cidx(d, ii, jj, kk)];
+}
+
 // ------------------------------------------------------------------ post_fixup
 
 
@@ -312,18 +437,26 @@ __global__ void k_bound_flags_x2(Dims d, int8_t* flag) {
 // GAMMAMAX), and the flag of fixuputoprim_accounting (fixup.c:1592): -1, for the negative
 // density/energy and U2AVG codes only on the final substep.  Each fixed cell is recorded and
 // written by k_fixup_apply, so that every cell's fix reads the unfixed neighbours.
+// One thread per cell of the extended i, j range and the active k: the ghost flags of x1 and
+// x2 (ghosts set) are written by their own threads, and the active cells read their neighbours'
+// flags through flag_at, which reads none of those.
 __global__ void __launch_bounds__(256) k_fixup_compute(Dims d, Phys ph, const double* __restrict__ P,
-                                                       const int8_t* __restrict__ flag, const double* __restrict__ geom,
+                                                       int8_t* flag, const double* __restrict__ geom,
                                                        FixRec* __restrict__ recs, unsigned int* __restrict__ nrec,
-                                                       unsigned int cap, int finalstep) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)d.n1 * d.n2 * d.n3) return;
-  int i = (int)(t % d.n1);
-  long long r = t / d.n1;
-  int j = (int)(r % d.n2), k = (int)(r / d.n2);
-  int ii = i + d.ng, jj = j + d.ng, kk = k + d.ng3;
-  size_t id = cidx(d, ii, jj, kk);
-  int8_t f = flag[id];
+                                                       unsigned int cap, int finalstep, int ghosts) {
+  const unsigned int c2 = blockIdx.x * 256u + threadIdx.x;
+  if (c2 >= (unsigned int)d.plane) return;
+  const int ii = (int)(c2 % (unsigned int)d.n1e), jj = (int)(c2 / (unsigned int)d.n1e), kk = (int)blockIdx.y + d.ng3;
+  const int i = ii - d.ng, j = jj - d.ng;
+  const size_t id = (size_t)kk * d.plane + c2;
+  if (i < 0 || i >= d.n1 || j < 0 || j >= d.n2) {
+    if (ghosts && (j < 0 || j >= d.n2 || i >= d.n1)) {
+      const int js = (j < 0) ? 2 * d.ng - 1 - jj : (j >= d.n2) ? 2 * (d.ng + d.n2) - 1 - jj : jj;
+      flag[id] = flag[cidx(d, (i >= d.n1) ? d.ng + d.n1 - 1 : ii, js, kk)];
+    }
+    return;
+  }
+  const int8_t f = flag[id];
   if (f <= 0) return;
   int startpl, endpl;
   const bool u2 = (f == HARM_UTOPRIMFAILU2AVG1 || f == HARM_UTOPRIMFAILU2AVG2);
@@ -339,7 +472,7 @@ __global__ void __launch_bounds__(256) k_fixup_compute(Dims d, Phys ph, const do
   for (int qq = 0; qq < npairs; qq++) {
     int di = (qq % rnx) - s1, dj = ((qq % (rnx * rny)) / rnx) - s2, dk = (qq / (rnx * rny)) - s3;
     size_t a = cidx(d, ii + di, jj + dj, kk + dk), b = cidx(d, ii - di, jj - dj, kk - dk);
-    int thisok = flag[a] <= 0, thatok = flag[b] <= 0;
+    int thisok = flag_at(d, flag, ii + di, jj + dj, kk + dk) <= 0, thatok = flag_at(d, flag, ii - di, jj - dj, kk - dk) <= 0;
     numavg0 += thisok + thatok;
     for (int p = startpl; p <= endpl; p++) {
       double fa = P[(size_t)p * d.cells + a], fb = P[(size_t)p * d.cells + b];
@@ -595,11 +728,29 @@ int hp_emf_to_flux_fp64(harm_ctx* c, const double* emf, double* F1, double* F2, 
   return 0;
 }
 
-int hp_bound(harm_ctx* c, double* P, int8_t* flag) {
+// whether the grid's mirrored and periodic boundary sources are active cells off the pole rows
+static bool bound_one_launch(const Dims& d) { return d.n2 > d.ng && (d.n3 == 1 || d.n3 >= d.ng3); }
+
+int hp_bound(harm_ctx* c, double* P, int8_t* flag, const unsigned int* only_if) {
   Dims d = dims_of(c->g);
   Phys ph = phys_of(c->g);
+  if (bound_one_launch(d)) {
+    BoundBlocks nb{};
+    if (P) {
+      nb.x1 = nblk(2LL * d.ng * d.n2e * d.n3e, 128);
+      nb.x2 = nblk((long long)d.n1 * (2 * d.ng + 2) * d.n3e, 128);
+      nb.x3 = nblk((long long)d.n1 * (d.n2 - 2) * 2 * d.ng3, 128);
+    }
+    if (flag) nb.fl = nblk((long long)d.plane * 2 * d.ng3, 128);
+    const unsigned int blocks = nb.x1 + nb.x2 + nb.x3 + nb.fl;
+    if (blocks == 0) return 0;
+    k_bound<<<blocks, 128, 0, c->stream>>>(d, ph, c->g.startx[2], P, c->d_geom, c->d_aux, flag, nb, only_if);
+    c->launches++;
+    CK(cudaGetLastError());
+    return 0;
+  }
   if (P) {
-    k_bound_x1_extrap<<<nblk(2LL * d.n2 * d.n3, 128), 128, 0, c->stream>>>(d, ph, P, c->d_geom);
+    k_bound_x1<<<nblk(2LL * d.ng * d.n2 * d.n3, 128), 128, 0, c->stream>>>(d, ph, P, c->d_geom);
     k_bound_x2_reflect<<<nblk(2LL * d.n1e * d.n3, 128), 128, 0, c->stream>>>(d, P);
     k_bound_x2_pole<<<nblk(2LL * d.n1e * d.n3, 128), 128, 0, c->stream>>>(d, ph, c->g.startx[2], P, c->d_geom, c->d_aux);
     c->launches += 3;
@@ -634,9 +785,8 @@ int hp_fixup(harm_ctx* c, double* pf, int8_t* pflag, int finalstep, bool bound_f
   Phys ph = phys_of(c->g);
   if (bound_flags && hp_bound(c, nullptr, pflag)) return 1;
   CK(cudaMemsetAsync(c->d_nrec, 0, sizeof(unsigned int), c->stream));
-  long long ncell = (long long)d.n1 * d.n2 * d.n3;
-  k_fixup_compute<<<nblk(ncell), 256, 0, c->stream>>>(d, ph, pf, pflag, c->d_geom, (FixRec*)c->d_fixrec, c->d_nrec,
-                                                       c->fix_cap, finalstep);
+  k_fixup_compute<<<dim3(nblk((long long)d.plane), d.n3), 256, 0, c->stream>>>(
+      d, ph, pf, pflag, c->d_geom, (FixRec*)c->d_fixrec, c->d_nrec, c->fix_cap, finalstep, bound_one_launch(d) ? 1 : 0);
   k_fixup_apply<<<4 * c->num_sms, 256, 0, c->stream>>>(d, pf, pflag, (const FixRec*)c->d_fixrec, c->d_nrec, c->fix_cap);
   c->launches += 2;
   CK(cudaGetLastError());

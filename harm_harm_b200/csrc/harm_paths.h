@@ -21,7 +21,9 @@ int hp_update_fp64fma(harm_ctx* c, const StepCoef& sc, const double* pi, const d
 int hp_update_mixed(harm_ctx* c, const StepCoef& sc, const double* pi, const double* pb, double* pf, int8_t* pflag,
                     double* stats);
 int hp_emf_to_flux_fp64(harm_ctx* c, const double* emf, double* F1, double* F2, double* F3);
-int hp_bound(harm_ctx* c, double* P, int8_t* flag);
+// bound_prim of P and, with flag, the boundary flags that post_fixup starts from (the x3 ghost
+// planes where post_fixup fills the rest itself); only_if: a device count, 0 for nothing to do
+int hp_bound(harm_ctx* c, double* P, int8_t* flag, const unsigned int* only_if = nullptr);
 int hp_copy_ghosts(harm_ctx* c, const double* pb, double* pf);
 // post_fixup of the final substep (finalstep 1) or an earlier one (0); bound_flags = false when
 // the caller has already filled the flags' ghost zones
