@@ -60,13 +60,25 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   CK(cudaMalloc(&c->d_geomf, gsz * sizeof(float)));
   CK(cudaMalloc(&c->d_conn, 64 * d.plane * sizeof(double)));
   CK(cudaMalloc(&c->d_aux, HARM_NAUX * d.plane * sizeof(double)));
+  // fluxes of the three directions and one direction's edge values, in FP64 or in FP32: a substep
+  // runs in one arithmetic and leaves nothing in them, so the two share their memory
+  const size_t nf = NPR * d.cells;
+  CK(cudaMalloc(&c->d_flux, 5 * nf * sizeof(double)));
   for (int q = 0; q < 3; q++) {
-    CK(cudaMalloc(&c->d_F[q], NPR * d.cells * sizeof(double)));
-    CK(cudaMalloc(&c->d_Ff[q], NPR * d.cells * sizeof(float)));
+    c->d_F[q] = (double*)c->d_flux + q * nf;
+    c->d_Ff[q] = (float*)c->d_flux + q * nf;
   }
+  c->d_edge = (double*)c->d_flux + 3 * nf;
+  c->d_edgef = (float*)c->d_flux + 3 * nf;
   CK(cudaMalloc(&c->d_emf, 3 * d.cells * sizeof(double)));
-  CK(cudaMalloc(&c->d_emff, 3 * d.cells * sizeof(float)));
-  if (g->lim == HARM_LIM_WENO5) CK(cudaMalloc(&c->d_line, 9 * d.cells * sizeof(double)));
+  c->d_emff = (float*)c->d_emf;
+  if (g->lim == HARM_LIM_WENO5 || g->lim == HARM_LIM_PARALINE) {
+    const size_t nl = (g->lim == HARM_LIM_WENO5 ? 9 : 4) * d.cells;
+    CK(cudaMalloc(&c->d_line, (nl + d.cells) * sizeof(double)));
+    c->d_coef = (double*)c->d_line + nl;
+    // read (and not used) at ghost cells that no pass writes
+    CK(cudaMemset(c->d_coef, 0, d.cells * sizeof(double)));
+  }
   CK(cudaMalloc(&c->d_pk, NPR * d.cells * sizeof(double)));
   CK(cudaMalloc(&c->d_U, NPR * d.cells * sizeof(double)));
   CK(cudaMalloc(&c->d_rare, (size_t)d.n1 * d.n2 * d.n3 * sizeof(unsigned int)));
@@ -144,8 +156,8 @@ extern "C" int harm_b200_destroy(harm_ctx* c) {
   if (!c) return 0;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  void* ptrs[] = {c->d_geom, c->d_geomf, c->d_conn, c->d_aux, c->d_F[0], c->d_F[1], c->d_F[2], c->d_Ff[0], c->d_Ff[1],
-                  c->d_Ff[2], c->d_emf, c->d_emff, c->d_line, c->d_Paos, c->d_pk, c->d_U, c->d_rare, c->d_pflag, c->d_fixrec, c->d_scal, c->d_Pdev, c->d_mlp, c->d_wpg,
+  void* ptrs[] = {c->d_geom, c->d_geomf, c->d_conn, c->d_aux, c->d_flux, c->d_emf, c->d_line, c->d_Paos,
+                  c->d_pk, c->d_U, c->d_rare, c->d_pflag, c->d_fixrec, c->d_scal, c->d_Pdev, c->d_mlp, c->d_wpg,
                   c->d_mlp_master, c->d_mlp_adam, c->d_mlp_work};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -294,6 +294,7 @@ __device__ __forceinline__ void weno_tile_edges(const T* s_y, T* s_w, T* s_el, T
                                                 SX sx, EX ex, WX wx, SPLIT split) {
   if constexpr (sizeof(T) == 4) {
     // FP32: two cells per thread on the packed FP32 pipe (harm_weno_f32x2.cuh)
+    const WenoK K = weno_consts();
     constexpr int NU = NV * (NL - 4) * NT, NU2 = (NU + 1) / 2;
     for (int idx = tid; idx < NU2; idx += 256) {
       const int ib = idx + NU2;
@@ -307,8 +308,9 @@ __device__ __forceinline__ void weno_tile_edges(const T* s_y, T* s_w, T* s_el, T
 #pragma unroll
       for (int q = 0; q < 5; q++) u5[q] = f2((float)ya[sx(ca - 2 + q, ta)], (float)yb[sx(cb - 2 + q, tb)]);
       F2 w[3];
-      const F2 m = smono_indicator_f2(u5 + 2);
-      weno5_cell_weights_f2(u5 + 2, m, w);
+      const Sten st = stencil_of(K, u5 + 2);
+      const F2 m = smono_indicator_f2(K, st, u5 + 2);
+      weno5_cell_weights_f2(K, st, u5 + 2, m, w);
       T* wsa = s_w + (va * PW + wx(ca, ta)) * 4;
       T* wsb = s_w + (vb * PW + wx(cb, tb)) * 4;
       float a, b;
@@ -345,7 +347,7 @@ __device__ __forceinline__ void weno_tile_edges(const T* s_y, T* s_w, T* s_el, T
         wp[k] = f2((float)wa[wx(ca + 2, ta) * 4 + k], (float)wb[wx(cb + 2, tb) * 4 + k]);
       }
       const F2 m = f2((float)wa[wx(ca, ta) * 4 + 3], (float)wb[wx(cb, tb) * 4 + 3]);
-      F2 f = weno_frac_f2(w, wm, wp);
+      F2 f = weno_frac_f2(K, w[0], w[2], wm[0], wp[2]);
       const float ssa = weno_dp_strength<float>((float)s_dP[ex(ca, ta)]);
       const float ssb = weno_dp_strength<float>((float)s_dP[ex(cb, tb)]);
       if (ssa > 0.0f || ssb > 0.0f) {  // rare: a momentum-flux jump above 0.25
@@ -358,7 +360,7 @@ __device__ __forceinline__ void weno_tile_edges(const T* s_y, T* s_w, T* s_el, T
         f = f2(fa, fb);
       }
       F2 yl, yr;
-      weno5_edges_f2(u5 + 2, w, f, m, yl, yr);
+      weno5_edges_f2(K, stencil_of(K, u5 + 2), u5 + 2, w, f, m, yl, yr);
       float la, lb, ra, rb;
       f2split(yl, la, lb);
       f2split(yr, ra, rb);
@@ -405,9 +407,9 @@ __device__ __forceinline__ void weno_tile_edges(const T* s_y, T* s_w, T* s_el, T
 
 // The face physics of k_fluxt: B^DIR continuity, limit_gamma, states, fluxes, wave speeds and
 // the HLL flux of one face (flux.c:852, vchar.c:34; LAXF where both speeds vanish or where
-// fluxmethod is LAXF, fluxcompute.c:243) into F at `id`; returns cour*dx/ctop.
+// fluxmethod is LAXF, fluxcompute.c:243) into F at `id`; returns ctop.
 template <int DIR, typename T, typename GT>
-__device__ __forceinline__ double face_hll(const Dims& d, const Phys& ph, const GT* __restrict__ geom,
+__device__ __forceinline__ T face_hll(const Dims& d, const Phys& ph, const GT* __restrict__ geom,
                                            T* __restrict__ F, size_t id, int ii, int jj, T* pl, T* pr) {
   constexpr int loc = (DIR == 1) ? HARM_LOC_FACE1 : (DIR == 2) ? HARM_LOC_FACE2 : HARM_LOC_CENT;
   Geo<T> g;
@@ -433,17 +435,22 @@ __device__ __forceinline__ double face_hll(const Dims& d, const Phys& ph, const 
   lmax = fabs(fmax(T(0), lmax));
   const T cmin = lmin, cmax = lmax, ctop = fmax(lmax, lmin);
   if (!ph.laxf && cmax + cmin != T(0)) {
-    const T inv = cmax + cmin;
+    const WScale<T> n(cmax + cmin);
 #pragma unroll
-    for (int p = 0; p < NPR; p++) F[(size_t)p * d.cells + id] = ((cmax * Fl[p] + cmin * Fr[p]) - (cmax * cmin) * (Ur[p] - Ul[p])) / inv;
+    for (int p = 0; p < NPR; p++) F[(size_t)p * d.cells + id] = n((cmax * Fl[p] + cmin * Fr[p]) - (cmax * cmin) * (Ur[p] - Ul[p]));
   } else {
 #pragma unroll
     for (int p = 0; p < NPR; p++) F[(size_t)p * d.cells + id] = T(0.5) * ((Fl[p] + Fr[p]) - ctop * (Ur[p] - Ul[p]));
   }
+  return ctop;
+}
+
+// a face's time-step limit cour*dx/ctop
+template <int DIR>
+__device__ __forceinline__ double face_dt(const Phys& ph, double ctop) {
   const double dxd = (DIR == 1) ? ph.dx1 : (DIR == 2) ? ph.dx2 : ph.dx3;
-  double dtij = ph.cour * dxd / (double)ctop;
-  if (!(dtij > 0.0)) dtij = 1.e300;
-  return dtij;
+  const double dtij = ph.cour * dxd / ctop;
+  return (dtij > 0.0) ? dtij : 1.e300;
 }
 
 // HARM_FLUXT_MINB: resident blocks per SM the tiled flux kernel is compiled for (the mixed
@@ -463,13 +470,10 @@ __host__ __device__ __forceinline__ int fluxt_tshift(const FaceBox& fb, int ng) 
   return (fb.lo[0] + ng) & (NT - 1);
 }
 
-// L (WENO5, optional): the dP line quantities of every extended cell from k_cellprep,
-// [3 (DIR-1) + q][cells] for q = par, veff, upar; where null, the kernel computes them.
 template <int DIR, int LIM, typename T, typename GT, int TU = HARM_TU>
 __global__ void HARM_FLUXT_LB k_fluxt(Dims d, Phys ph, FaceBox fb, const double* __restrict__ P,
                                                const GT* __restrict__ geom, T* __restrict__ F,
-                                               unsigned long long* __restrict__ dtslot,
-                                               const T* __restrict__ L = nullptr) {
+                                               unsigned long long* __restrict__ dtslot) {
   using TL = FluxTile<LIM, T>;
   constexpr int A = TL::A, AF = TL::AF, NT = TL::NT, H = TL::H, NL = TL::NL, VB = TL::VB, PL = TL::PLANE, PE = TL::PE, PW = TL::PW;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -569,50 +573,24 @@ __global__ void HARM_FLUXT_LB k_fluxt(Dims d, Phys ph, FaceBox fb, const double*
   // WENO5: the line quantities of dP (compute_df_line_new interpline.c:3557) of the staged
   // cells H-2 .. H+A (the edge cells and their neighbours along DIR), from all the cell's
   // primitives and the cell-centre metric, into the edge planes, then dP of each edge cell.
-  // From L where the cell pass computed them; otherwise here: with all primitives staged at
-  // once (FP32) from the staged tile below, else (FP64, two groups) loaded here.
-  constexpr int DPC = AF + 3;  // cells with line quantities per line
-  auto weno_line = [&](int cl, int ct, const T* pc) {
-    const int lext = min(max(l0 - H + cl + ngL, 0), nLe - 1);
-    const int text = min(max(t0 + ct + d.ng, 0), nTe - 1);
-    const int ii = (DIR == 1) ? lext : text, jj = (DIR == 1) ? text : (DIR == 2) ? lext : o + d.ng;
-    Geo<T> g;
-    load_geo<T, GT>(geom + (size_t)HARM_LOC_CENT * HARM_NGF * d.plane, d.plane, (size_t)jj * d.n1e + ii, g);
-    weno_line_cell<DIR, PL, T>(s_el, sx(cl, ct), pc, g, (T)ph.gam);
-  };
-  const bool dp_from_L = (LIM == HARM_LIM_WENO5) && (L != nullptr);
   if constexpr (LIM == HARM_LIM_WENO5) {
-    if (dp_from_L) {
-      const T* Lq = L + (size_t)3 * (DIR - 1) * d.cells;
-      for (int idx = tid; idx < DPC * NT; idx += 256) {
-        int v, cl, ct;
-        split(idx, H - 2, DPC, v, cl, ct);
-        const int lext = min(max(l0 - H + cl + ngL, 0), nLe - 1);
-        const int text = min(max(t0 + ct + d.ng, 0), nTe - 1);
-        const size_t cid = cell_index(lext, text);
-        const int si = sx(cl, ct);
-        s_el[si] = (T)__ldg(P + (size_t)HARM_RHO * d.cells + cid);
-        s_el[PL + si] = __ldg(Lq + cid);
-        s_el[2 * PL + si] = __ldg(Lq + d.cells + cid);
-        s_el[3 * PL + si] = __ldg(Lq + 2 * d.cells + cid);
-      }
-      __syncthreads();
-      weno_dp_edges<AF, NT, H, PL, T>(s_el, s_dP, tid, sx, ex, split);
-    } else if constexpr (VB < NPR) {
-      for (int idx = tid; idx < DPC * NT; idx += 256) {
-        int v, cl, ct;
-        split(idx, H - 2, DPC, v, cl, ct);
-        const int lext = min(max(l0 - H + cl + ngL, 0), nLe - 1);
-        const int text = min(max(t0 + ct + d.ng, 0), nTe - 1);
-        const size_t cid = cell_index(lext, text);
-        T pc[NPR];
+    constexpr int DPC = AF + 3;  // cells with line quantities per line
+    for (int idx = tid; idx < DPC * NT; idx += 256) {
+      int v, cl, ct;
+      split(idx, H - 2, DPC, v, cl, ct);
+      const int lext = min(max(l0 - H + cl + ngL, 0), nLe - 1);
+      const int text = min(max(t0 + ct + d.ng, 0), nTe - 1);
+      const size_t cid = cell_index(lext, text);
+      T pc[NPR];
 #pragma unroll
-        for (int p = 0; p < NPR; p++) pc[p] = (T)__ldg(P + (size_t)p * d.cells + cid);
-        weno_line(cl, ct, pc);
-      }
-      __syncthreads();
-      weno_dp_edges<AF, NT, H, PL, T>(s_el, s_dP, tid, sx, ex, split);
+      for (int p = 0; p < NPR; p++) pc[p] = (T)__ldg(P + (size_t)p * d.cells + cid);
+      const int ii = (DIR == 1) ? lext : text, jj = (DIR == 1) ? text : (DIR == 2) ? lext : o + d.ng;
+      Geo<T> g;
+      load_geo<T, GT>(geom + (size_t)HARM_LOC_CENT * HARM_NGF * d.plane, d.plane, (size_t)jj * d.n1e + ii, g);
+      weno_line_cell<DIR, PL, T>(s_el, sx(cl, ct), pc, g, (T)ph.gam);
     }
+    __syncthreads();
+    weno_dp_edges<AF, NT, H, PL, T>(s_el, s_dP, tid, sx, ex, split);
   }
   T pl[NPR], pr[NPR];
   __shared__ T s_xl[NPR * NT], s_xr[NPR * NT];  // edge values of the tile's face A
@@ -632,20 +610,6 @@ __global__ void HARM_FLUXT_LB k_fluxt(Dims d, Phys ph, FaceBox fb, const double*
     }
     __syncthreads();
     if constexpr (LIM == HARM_LIM_WENO5) {
-      if constexpr (VB == NPR) {
-        if (!dp_from_L) {
-          for (int idx = tid; idx < DPC * NT; idx += 256) {
-            int v, cl, ct;
-            split(idx, H - 2, DPC, v, cl, ct);
-            T pc[NPR];
-#pragma unroll
-            for (int p = 0; p < NPR; p++) pc[p] = s_y[p * PL + sx(cl, ct)];
-            weno_line(cl, ct, pc);
-          }
-          __syncthreads();
-          weno_dp_edges<AF, NT, H, PL, T>(s_el, s_dP, tid, sx, ex, split);
-        }
-      }
       weno_tile_edges<VB, AF, NT, H, NL, PL, PE, PW, T>(s_y, s_w, s_el, s_er, s_dP, tid, sx, ex, wx, split);
     } else if (LIM == HARM_LIM_PARA) {
       for (int idx = tid; idx < VB * (AF + 1) * NT; idx += 256) {
@@ -702,7 +666,7 @@ __global__ void HARM_FLUXT_LB k_fluxt(Dims d, Phys ph, FaceBox fb, const double*
     if (DIR == 1) { ii = lext; jj = text; }
     else if (DIR == 2) { ii = text; jj = lext; }
     else { ii = text; jj = o + d.ng; }
-    dtij = face_hll<DIR, T, GT>(d, ph, geom, F, id, ii, jj, pl, pr);
+    dtij = face_dt<DIR>(ph, (double)face_hll<DIR, T, GT>(d, ph, geom, F, id, ii, jj, pl, pr));
   }
   {
     // the tile's face A (the sweep's last face), on line tid, by the threads tid < NT, from
@@ -719,7 +683,7 @@ __global__ void HARM_FLUXT_LB k_fluxt(Dims d, Phys ph, FaceBox fb, const double*
       if (DIR == 1) { ii = lext; jj = text; }
       else if (DIR == 2) { ii = text; jj = lext; }
       else { ii = text; jj = o + d.ng; }
-      dtij = fmin(dtij, face_hll<DIR, T, GT>(d, ph, geom, F, id, ii, jj, pl, pr));
+      dtij = fmin(dtij, face_dt<DIR>(ph, (double)face_hll<DIR, T, GT>(d, ph, geom, F, id, ii, jj, pl, pr)));
     }
   }
   // block minimum and one atomic per block
@@ -768,12 +732,12 @@ static inline bool face_box_k(FaceBox b, int klo, int khi, FaceBox* out) {
   return true;
 }
 
-// The cell pass of a WENO5 flux stage: the dP line quantities (par, veff, upar of
-// compute_df_line_new interpline.c:3557) of every extended cell of planes [k0, k1), for the
-// three directions, from one evaluation of the cell's state (get_state) in the arithmetic
-// type T of the flux tiles; L[3 (dir-1) + q][cells].  The tiles of the three directions
-// read them instead of evaluating the state of each staged cell once per direction.
-template <typename T, typename GT, int TU = HARM_TU>
+// The cell pass of a flux stage, from one evaluation of each extended cell's state (get_state) of
+// planes [k0, k1) in the arithmetic type T of the reconstruction.  WENO5: the line quantities of
+// dP (par, veff, upar of compute_df_line_new interpline.c:3557) of the three directions,
+// L[3 (dir-1) + q][cells].  PARALINE: total pressure and sqrt(-g) rho u^dir of get_V_and_P
+// (interpline.c:2964), L[0] and L[dir].
+template <int LIM, typename T, typename GT, int TU = HARM_TU>
 __global__ void __launch_bounds__(256) k_cellprep(Dims d, Phys ph, const double* __restrict__ P,
                                                   const GT* __restrict__ geom, T* __restrict__ L, int k0, int k1) {
   const long long n = (long long)(k1 - k0) * d.plane;
@@ -788,22 +752,30 @@ __global__ void __launch_bounds__(256) k_cellprep(Dims d, Phys ph, const double*
   load_geo<T, GT>(geom + (size_t)HARM_LOC_CENT * HARM_NGF * d.plane, d.plane, c2, g);
   State<T> q;
   get_state<T>(pc, g, (T)ph.gam, q);
+  if constexpr (LIM == HARM_LIM_PARALINE) {
+    T pt = q.pressure;
+    pt += T(0.5) * q.bsq;
+    L[id] = pt;
 #pragma unroll
-  for (int dir = 1; dir <= 3; dir++) {
-    T par, veff, upar;
-    weno_dp_of_state<T>(pc, g, q, dir, par, veff, upar);
-    L[(size_t)(3 * (dir - 1) + 0) * d.cells + id] = par;
-    L[(size_t)(3 * (dir - 1) + 1) * d.cells + id] = veff;
-    L[(size_t)(3 * (dir - 1) + 2) * d.cells + id] = upar;
+    for (int dir = 1; dir <= 3; dir++) L[(size_t)dir * d.cells + id] = g.gdet * pc[HARM_RHO] * q.ucon[dir];
+  } else {
+#pragma unroll
+    for (int dir = 1; dir <= 3; dir++) {
+      T par, veff, upar;
+      weno_dp_of_state<T>(pc, g, q, dir, par, veff, upar);
+      L[(size_t)(3 * (dir - 1) + 0) * d.cells + id] = par;
+      L[(size_t)(3 * (dir - 1) + 1) * d.cells + id] = veff;
+      L[(size_t)(3 * (dir - 1) + 2) * d.cells + id] = upar;
+    }
   }
 }
 
-template <typename T, typename GT>
+template <int LIM, typename T, typename GT>
 static inline cudaError_t launch_cellprep(const Dims& d, const Phys& ph, const double* P, const GT* geom, T* L, int k0,
                                           int k1, cudaStream_t st) {
   const long long n = (long long)(k1 - k0) * d.plane;
   if (n <= 0) return cudaSuccess;
-  k_cellprep<T, GT><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, ph, P, geom, L, k0, k1);
+  k_cellprep<LIM, T, GT><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, ph, P, geom, L, k0, k1);
   return cudaGetLastError();
 }
 
@@ -811,69 +783,15 @@ static inline cudaError_t launch_cellprep(const Dims& d, const Phys& ph, const d
 // its dynamic shared-memory limit where the tile needs more than 48 KB (FP32 WENO5: 63 KB)
 template <int DIR, int LIM, typename T, typename GT>
 static inline cudaError_t launch_fluxt(const Dims& d, const Phys& ph, const FaceBox& fb, const double* P,
-                                       const GT* geom, T* F, unsigned long long* dtslot, cudaStream_t st,
-                                       const T* L = nullptr) {
+                                       const GT* geom, T* F, unsigned long long* dtslot, cudaStream_t st) {
   constexpr size_t smem = FluxTile<LIM, T>::smem;
   if (smem > 48 * 1024) {
     static std::atomic<unsigned long long> raised{0};  // per instantiation
     cudaError_t e = raise_smem_limit_once(raised, (const void*)k_fluxt<DIR, LIM, T, GT>, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_fluxt<DIR, LIM, T, GT><<<fluxt_grid<DIR, LIM, T>(fb, d.ng), 256, smem, st>>>(d, ph, fb, P, geom, F, dtslot, L);
+  k_fluxt<DIR, LIM, T, GT><<<fluxt_grid<DIR, LIM, T>(fb, d.ng), 256, smem, st>>>(d, ph, fb, P, geom, F, dtslot);
   return cudaGetLastError();
-}
-
-// The three flux directions of one substep while the state is still arriving in k-slabs
-// (SlabWait): after each slab's copy, the x1 and x2 faces of its planes (their stencils stay in
-// the plane) and every row of x3 tiles (A faces along k) whose staged planes have all arrived.
-// Same kernels and results as the whole-grid launches.
-// L (WENO5, optional): the cell pass's output buffer; each slab's cell pass runs once the
-// slab has arrived, before the tiles that stage its planes.
-template <int LIM, typename T, typename GT>
-static inline cudaError_t launch_flux_slabs(const Dims& d, const Phys& ph, const double* pb, const GT* geom, T* F1,
-                                            T* F2, T* F3, unsigned long long* slots, cudaStream_t st,
-                                            const SlabWait& sw, unsigned long long& launches, T* L = nullptr) {
-  constexpr int A = FluxTile<LIM, T>::A, X = ReconGeom<LIM>::X;
-  const FaceBox b1 = face_box(d, 1), b2 = face_box(d, 2), b3 = face_box(d, 3);
-  int f3 = b3.lo[2];  // first x3 face not launched yet
-  cudaError_t e;
-  for (int s = 0; s < sw.nslab; s++) {
-    if ((e = cudaStreamWaitEvent(st, sw.ev[s], 0)) != cudaSuccess) return e;
-    const int resident = (s + 1) * sw.planes;  // planes [0, resident) are on the device
-    const int klo = s * sw.planes - d.ng3, khi = resident - 1 - d.ng3;
-    if (sw.aos && hp_harm_to_soa(sw.ctx, sw.aos, sw.soa, s * sw.planes, resident < d.n3e ? resident : d.n3e))
-      return cudaErrorLaunchFailure;
-    if (L) {
-      const int k1 = resident < d.n3e ? resident : d.n3e;
-      if ((e = launch_cellprep<T, GT>(d, ph, pb, geom, L, s * sw.planes, k1, st)) != cudaSuccess) return e;
-      launches++;
-    }
-    FaceBox sb;
-    if (face_box_k(b1, klo, khi, &sb)) {
-      if ((e = launch_fluxt<1, LIM, T, GT>(d, ph, sb, pb, geom, F1, slots + 0, st, L)) != cudaSuccess) return e;
-      launches++;
-    }
-    if (face_box_k(b2, klo, khi, &sb)) {
-      if ((e = launch_fluxt<2, LIM, T, GT>(d, ph, sb, pb, geom, F2, slots + 1, st, L)) != cudaSuccess) return e;
-      launches++;
-    }
-    // x3 tile rows: a row of faces f0 .. last stages planes up to last + ng3 + X (clamped);
-    // a row of tiles with room for one more face takes the sweep's last face when it is the
-    // only one left after it
-    while (d.n3 > 1 && f3 <= b3.hi[2]) {
-      int last = f3 + A - 1;
-      if (b3.hi[2] - last == 1) last = b3.hi[2];
-      int top = last + d.ng3 + X;
-      if (top > d.n3e - 1) top = d.n3e - 1;
-      if (top >= resident && s + 1 < sw.nslab) break;
-      if (face_box_k(b3, f3, last, &sb)) {
-        if ((e = launch_fluxt<3, LIM, T, GT>(d, ph, sb, pb, geom, F3, slots + 2, st, L)) != cudaSuccess) return e;
-        launches++;
-      }
-      f3 = last + 1;
-    }
-  }
-  return cudaSuccess;
 }
 
 // ------------------------------------------------------------------ EMF kernel

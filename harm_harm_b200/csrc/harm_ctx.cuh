@@ -38,12 +38,16 @@ struct harm_ctx {
   double* d_conn;
   double* d_aux;
   // scratch of one substep
+  void* d_flux;     // the arrays of the flux stage: d_F and d_edge, or d_Ff and d_edgef
   double* d_F[3];
   float* d_Ff[3];
   double* d_emf;
   float* d_emff;
-  void* d_line;     // WENO5: dP line quantities of the flux stage's cell pass, [9][cells] (FP64
-                    // path: double, mixed path: float)
+  void* d_line;     // the flux stage's cell pass: WENO5 [9][cells], PARALINE [4][cells] (FP64 path:
+                    // double, mixed path: float)
+  void* d_coef;     // its per-cell coefficient of one direction, [cells]
+  double* d_edge;   // left and right edge values of one direction, [2][8][cells]
+  float* d_edgef;
   double* d_pk;     // midpoint primitives of the RK2 step
   double* d_U;      // conserved variables to invert (UEVOLVE)
   unsigned int* d_rare;   // cells finished by the rare inversion path

@@ -55,6 +55,37 @@ __device__ __forceinline__ void load_geo(const S* __restrict__ tab, size_t plane
   g.igdet = (T)tab_ld<LDG>(tab + (size_t)HARM_G_IGDET * plane + c);
 }
 
+// a/b from b's correctly rounded reciprocal y (P. Markstein, IBM J. Res. Dev. 34, 1990): the
+// quotient estimate q = a y corrected by its exact remainder, q + (a - b q) y.  The corrected
+// value is a/b to within 2^-52 ulp before its rounding, so it is the IEEE quotient unless a/b
+// lies that close to the middle of two doubles (b normal, no overflow or underflow; a = 0
+// gives 0).  Three operations against the dozen of a division: the WENO sums divide several
+// values by one denominator, and several by constants.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+
+// Several values over one denominator: one reciprocal, FP64 with the quotients corrected.
+template <typename T>
+struct WScale {
+  T d, y;
+  __device__ __forceinline__ explicit WScale(T den) : d(den), y(T(1) / den) {}
+  __device__ __forceinline__ T operator()(T a) const { return div_by(a, d, y); }
+};
+template <>
+struct WScale<float> {
+  float r;
+  __device__ __forceinline__ explicit WScale(float den) {
+#ifdef __CUDA_ARCH__
+    r = __fdividef(1.0f, den);
+#else
+    r = 1.0f / den;  // host pass only parses this; the kernels use the line above
+#endif
+  }
+  __device__ __forceinline__ float operator()(float a) const { return a * r; }
+};
+
 template <typename T>
 struct State {
   T ucon[4], ucov[4], bsq, pressure, plus1ud0, gamma, qsq;
@@ -143,9 +174,10 @@ __device__ __forceinline__ void primtoflux(const T* pr, const State<T>& q, int d
 #pragma unroll
   for (int mu = 0; mu < 4; mu++) F[HARM_UU + mu] = (ma[mu] + em[mu] * ig2) * gd;
   if (dir > 0) {
-    F[HARM_B1] = ((pr[HARM_B1] * ud - Bd * q.ucon[1]) / q.ucon[0]) * gd;
-    F[HARM_B2] = ((pr[HARM_B2] * ud - Bd * q.ucon[2]) / q.ucon[0]) * gd;
-    F[HARM_B3] = ((pr[HARM_B3] * ud - Bd * q.ucon[3]) / q.ucon[0]) * gd;
+    const WScale<T> n(q.ucon[0]);
+    F[HARM_B1] = n(pr[HARM_B1] * ud - Bd * q.ucon[1]) * gd;
+    F[HARM_B2] = n(pr[HARM_B2] * ud - Bd * q.ucon[2]) * gd;
+    F[HARM_B3] = n(pr[HARM_B3] * ud - Bd * q.ucon[3]) * gd;
   } else {
     F[HARM_B1] = pr[HARM_B1] * gd;
     F[HARM_B2] = pr[HARM_B2] * gd;
@@ -403,36 +435,16 @@ __device__ __forceinline__ float wdiv<float>(float a, float b) {
   return __fdividef(a, b);
 }
 
-// Division by a compile-time constant: FP64 divides; FP32 multiplies by the folded reciprocal.
+// Division by a compile-time constant: FP64 the quotient from the folded reciprocal; FP32
+// multiplies by it.
 template <typename T>
 __device__ __forceinline__ T wdivk(T a, T b) {
-  return a / b;
+  return div_by(a, b, T(1) / b);
 }
 template <>
 __device__ __forceinline__ float wdivk<float>(float a, float b) {
   return a * (1.0f / b);
 }
-
-// Several values over one denominator: FP64 divides each (the oracle's operations); FP32
-// multiplies by one fast reciprocal.
-template <typename T>
-struct WScale {
-  T d;
-  __device__ __forceinline__ explicit WScale(T den) : d(den) {}
-  __device__ __forceinline__ T operator()(T a) const { return a / d; }
-};
-template <>
-struct WScale<float> {
-  float r;
-  __device__ __forceinline__ explicit WScale(float den) {
-#ifdef __CUDA_ARCH__
-    r = __fdividef(1.0f, den);
-#else
-    r = 1.0f / den;  // host pass only parses this; the kernels use the line above
-#endif
-  }
-  __device__ __forceinline__ float operator()(float a) const { return a * r; }
-};
 
 template <typename T>
 __device__ __forceinline__ T limit_weight(int order, T w) {
@@ -535,13 +547,13 @@ __device__ __forceinline__ void weno3_unopt(const T* u, T* w) {
 // gives 0 .. 1 (SMONO_DO_SMOOTH_TRANSITION)
 template <typename T>
 __device__ __forceinline__ T smono_indicator(const T* y) {
-  const T k12 = T(12), k2 = T(2);
+  const T k12 = T(12);
   T ld1 = wdivk<T>(((T(-3) * y[-2] + y[2]) + (T(-10) * y[-1] - T(6) * y[1])) + T(18) * y[0], k12);
   T ld2 = wdivk<T>(((T(11) * y[-2] - y[2]) + (T(-20) * y[-1] + T(4) * y[1])) + T(6) * y[0], k12);
-  T ld3 = wdivk<T>(((T(-3) * y[-2] - y[2]) + (T(10) * y[-1] + T(6) * y[1])) - T(12) * y[0], k2);
+  T ld3 = (((T(-3) * y[-2] - y[2]) + (T(10) * y[-1] + T(6) * y[1])) - T(12) * y[0]) * T(0.5);
   T rd1 = wdivk<T>(((-y[-2] + T(3) * y[2]) + (T(6) * y[-1] + T(10) * y[1])) - T(18) * y[0], k12);
   T rd2 = wdivk<T>(((-y[-2] + T(11) * y[2]) + (T(4) * y[-1] - T(20) * y[1])) + T(6) * y[0], k12);
-  T rd3 = wdivk<T>(((y[-2] + T(3) * y[2]) - (T(6) * y[-1] + T(10) * y[1])) + T(12) * y[0], k2);
+  T rd3 = (((y[-2] + T(3) * y[2]) - (T(6) * y[-1] + T(10) * y[1])) + T(12) * y[0]) * T(0.5);
   auto mm = [](T a, T b) -> T { return (a * b <= T(0)) ? T(0) : ((fabs(a) < fabs(b)) ? a : b); };
   ld1 = mm(ld1, y[-1] - y[-2]);
   rd1 = mm(rd1, y[2] - y[1]);

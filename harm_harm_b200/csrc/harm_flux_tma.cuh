@@ -223,8 +223,15 @@ __global__ void __launch_bounds__(256, TmaOcc<LIM>::blocks) k_fluxt_tma(Dims d, 
       if (DIR == 1) { ii = lext; jj = text; kk = o + d.ng3; }
       else if (DIR == 2) { ii = text; jj = lext; kk = o + d.ng3; }
       else { ii = text; jj = o + d.ng; kk = lext; }
-      const double dt = face_hll<DIR, T, GT>(d, ph, geom, F, cidx(d, ii, jj, kk), ii, jj, pl, pr);
-      dtmin = fmin(dtmin, dt);
+      constexpr int loc = (DIR == 1) ? HARM_LOC_FACE1 : (DIR == 2) ? HARM_LOC_FACE2 : HARM_LOC_CENT;
+      FaceGeo g;
+      load_face_geo<DIR>(geom + (size_t)loc * HARM_NGF * d.plane, d.plane, (size_t)jj * d.n1e + ii, g);
+      T Fo[NPR];
+      const float ctop = face_flux_f2<DIR>(g, pl, pr, (float)ph.gam, (float)ph.gammamax, ph.laxf, Fo);
+      dtmin = fmin(dtmin, face_dt<DIR>(ph, (double)ctop));
+      const size_t id = cidx(d, ii, jj, kk);
+#pragma unroll
+      for (int v = 0; v < NPR; v++) F[(size_t)v * d.cells + id] = Fo[v];
     }
     __syncthreads();  // the tile buffers are rewritten by the next iteration
   }

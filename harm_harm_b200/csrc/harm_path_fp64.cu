@@ -6,14 +6,9 @@
 // FMA contraction and the inversion's shared reciprocals (HARM_FP64_FMA_TU): the FP64 path as
 // fast as the compiler makes it, for comparisons of speed (HARM_PREC_FP64_FMA); this build
 // (HARM_PREC_FP64) performs the CPU restatement's IEEE operations in its order.
-// FP64 flux tiles at 2 resident blocks per SM (128 registers; harm_common.cuh): left to
-// itself the compiler can take ~160 registers and 1 block per SM, which halves the resident
-// warps (40.1 ms of flux per substep at 384x192x128 instead of 24.6)
-#ifndef HARM_FLUXT_MINB
-#define HARM_FLUXT_MINB 2
-#endif
 #include <algorithm>
 #include "harm_common.cuh"
+#include "harm_recon.cuh"
 #include "harm_mlp_tc.cuh"
 #include "harm_paths.h"
 
@@ -639,24 +634,16 @@ __global__ void __launch_bounds__(256, 2) k_utoprim_points_mlp(size_t n, Phys ph
 template <int LIM>
 static int flux_dirs_double(harm_ctx* c, const Dims& d, const Phys& ph, const double* pb, double* F1, double* F2, double* F3,
                          unsigned long long* slots, const SlabWait* sw) {
-  // WENO5: the cell pass computes the dP line quantities once per cell for the three directions
-  double* L = (LIM == HARM_LIM_WENO5) ? reinterpret_cast<double*>(c->d_line) : nullptr;
-  if (sw) {
-    CK((launch_flux_slabs<LIM, double, double>(d, ph, pb, c->d_geom, F1, F2, F3, slots, c->stream, *sw, c->launches, L)));
+  double* L = reinterpret_cast<double*>(c->d_line);
+  double* S = reinterpret_cast<double*>(c->d_coef);
+  double* E = c->d_edge;
+  if (sw) {  // state arriving in slabs
+    CK((launch_flux_slabs<LIM, double, double>(d, ph, pb, c->d_geom, F1, F2, F3, slots, c->stream, *sw, c->num_sms,
+                                               c->launches, L, S, E)));
     return 0;
   }
-  if (L) {
-    CK((launch_cellprep<double, double>(d, ph, pb, c->d_geom, L, 0, d.n3e, c->stream)));
-    c->launches++;
-  }
-  FaceBox b1 = face_box(d, 1), b2 = face_box(d, 2), b3 = face_box(d, 3);
-  CK((launch_fluxt<1, LIM, double, double>(d, ph, b1, pb, c->d_geom, F1, slots + 0, c->stream, L)));
-  CK((launch_fluxt<2, LIM, double, double>(d, ph, b2, pb, c->d_geom, F2, slots + 1, c->stream, L)));
-  c->launches += 2;
-  if (d.n3 > 1) {
-    CK((launch_fluxt<3, LIM, double, double>(d, ph, b3, pb, c->d_geom, F3, slots + 2, c->stream, L)));
-    c->launches++;
-  }
+  CK((launch_flux_dirs<LIM, double, double>(d, ph, pb, c->d_geom, F1, F2, F3, slots, c->stream, c->num_sms, c->launches,
+                                            L, S, E)));
   return 0;
 }
 

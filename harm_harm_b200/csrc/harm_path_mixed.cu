@@ -2,15 +2,12 @@
 // flux-CT; FP64 conserved update, sources and inversion (compiled with FMA contraction).
 // the inversion of this path shares reciprocals between its FP64 divisions (harm_invert.cuh)
 #define HARM_INVERT_FAST_DIV 1
-// FP32 flux tiles at 3 resident blocks per SM (harm_common.cuh)
-#ifndef HARM_FLUXT_MINB
-#define HARM_FLUXT_MINB 3
-#endif
 #include <algorithm>
 #include <cudaTypedefs.h>
 #include <mutex>
 #include "harm_common.cuh"
 #include "harm_mlp_tc.cuh"
+#include "harm_recon.cuh"
 #include "harm_flux_tma.cuh"
 #include "harm_paths.h"
 
@@ -69,17 +66,18 @@ static int launch_fluxt_tma(harm_ctx* c, const Dims& d, const Phys& ph, const Fa
 template <int LIM>
 static int flux_dirs_float(harm_ctx* c, const Dims& d, const Phys& ph, const double* pb, float* F1, float* F2, float* F3,
                          unsigned long long* slots, const SlabWait* sw) {
-  // WENO5: the cell pass computes the dP line quantities once per cell for the three
-  // directions (the plain-load tiles read them; the TMA-staged tiles compute their own)
-  float* L = (LIM == HARM_LIM_WENO5) ? reinterpret_cast<float*>(c->d_line) : nullptr;
-  if (sw) {  // state arriving in slabs: plain-load tiles, launched slab by slab
-    CK((launch_flux_slabs<LIM, float, float>(d, ph, pb, c->d_geomf, F1, F2, F3, slots, c->stream, *sw, c->launches, L)));
+  float* L = reinterpret_cast<float*>(c->d_line);
+  float* S = reinterpret_cast<float*>(c->d_coef);
+  float* E = c->d_edgef;
+  if (sw) {  // state arriving in slabs
+    CK((launch_flux_slabs<LIM, float, float>(d, ph, pb, c->d_geomf, F1, F2, F3, slots, c->stream, *sw, c->num_sms,
+                                             c->launches, L, S, E)));
     return 0;
   }
-  FaceBox b1 = face_box(d, 1), b2 = face_box(d, 2), b3 = face_box(d, 3);
-  // the TMA-staged variant covers MC, PARA and WENO5; PARALINE always takes k_fluxt
+  // the TMA-staged variant covers MC, PARA and WENO5
   if constexpr (LIM != HARM_LIM_PARALINE) {
     if (tma_usable(c, pb)) {
+      const FaceBox b1 = face_box(d, 1), b2 = face_box(d, 2), b3 = face_box(d, 3);
       if (int rc = launch_fluxt_tma<1, LIM>(c, d, ph, b1, pb, F1, slots + 0)) return rc;
       if (int rc = launch_fluxt_tma<2, LIM>(c, d, ph, b2, pb, F2, slots + 1)) return rc;
       c->launches += 2;
@@ -90,17 +88,8 @@ static int flux_dirs_float(harm_ctx* c, const Dims& d, const Phys& ph, const dou
       return 0;
     }
   }
-  if (L) {
-    CK((launch_cellprep<float, float>(d, ph, pb, c->d_geomf, L, 0, d.n3e, c->stream)));
-    c->launches++;
-  }
-  CK((launch_fluxt<1, LIM, float, float>(d, ph, b1, pb, c->d_geomf, F1, slots + 0, c->stream, L)));
-  CK((launch_fluxt<2, LIM, float, float>(d, ph, b2, pb, c->d_geomf, F2, slots + 1, c->stream, L)));
-  c->launches += 2;
-  if (d.n3 > 1) {
-    CK((launch_fluxt<3, LIM, float, float>(d, ph, b3, pb, c->d_geomf, F3, slots + 2, c->stream, L)));
-    c->launches++;
-  }
+  CK((launch_flux_dirs<LIM, float, float>(d, ph, pb, c->d_geomf, F1, F2, F3, slots, c->stream, c->num_sms, c->launches, L,
+                                          S, E)));
   return 0;
 }
 

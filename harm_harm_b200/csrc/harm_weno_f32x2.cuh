@@ -1,13 +1,21 @@
 // harm_weno_f32x2.cuh -- the FP32 WENO5 weights and edge values of two cells at once on
 // Blackwell's packed FP32 pipe (add/mul/fma on float2: one instruction, two lanes).
 //
-// The arithmetic is that of smono_indicator / weno5_cell_weights / weno3_unopt / weno_frac /
-// weno5_edges for T = float (harm_device.cuh), lane by lane; operations without a packed form (reciprocals, compares,
-// selects, min/max) run on each lane.  Where the scalar code branches on f > 0 (the WENO3
-// blend of the stencil reduction), the packed code evaluates the blend for both lanes when
-// either needs it: with f = 0 it multiplies by 1 and adds zeros, so a lane's value is the
-// one its scalar branch gives (the WENO3 weights are finite: every epsilon keeps its square
-// a normal FP32 number).
+// The algorithm is that of smono_indicator / weno5_cell_weights / weno3_unopt / weno_frac /
+// weno5_edges (harm_device.cuh) for T = float, lane by lane, in the differences of the stencil
+// to its centre (exact for neighbouring values within a factor of two, so a constant line
+// gives its value exactly); operations without a packed form (reciprocals, compares, selects,
+// min/max) run on each lane.  Where the scalar code branches on a lane's value (monotone
+// cells, the WENO3 blend of the stencil reduction), the packed code evaluates both sides when
+// either lane needs them and blends with exact zeros and ones, so that a lane's value never
+// depends on its partner.
+//
+// What bounds it is the FMA pipe (a packed operation takes two of its cycles), then the ALU
+// (compares and min/max at half rate) and the special-function unit (a reciprocal takes eight
+// cycles of a warp's quarter of the SM).  So the derivatives come from the sums and
+// differences of opposite neighbours (19 packed operations instead of 54), min-mods of
+// magnitudes are sign tests and minima, the three 1/beta^2 share their denominators, and the
+// weight ratios are divided out only where one exceeds the threshold.
 #pragma once
 #include "harm_device.cuh"
 
@@ -20,12 +28,20 @@ using F2 = float2;
 
 __device__ __forceinline__ F2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ F2 f2(float a) { return make_float2(a, a); }
+// 1/x for x and 1/x normal (the hardware approximation, 1 ulp; every operand here is a sum with
+// the smallest normal number or larger)
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ void f2split(F2 x, float& a, float& b) {
   a = x.x;
   b = x.y;
 }
 __device__ __forceinline__ F2 operator+(F2 a, F2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+// a - b as fma(b, -1, a): one packed instruction, where negating a pair takes two more
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ F2 ffma2(F2 a, F2 b, F2 c) { return __ffma2_rn(a, b, c); }
 // lane-wise helpers
@@ -42,204 +58,221 @@ __device__ __forceinline__ F2 lanes(F2 x, F2 y, Fn fn) {
   f2split(y, c, d);
   return f2(fn(a, c), fn(b, d));
 }
-__device__ __forceinline__ F2 rcp2(F2 x) {
-  return lanes(x, [](float a) { return __fdividef(1.0f, a); });
-}
+__device__ __forceinline__ F2 rcp2(F2 x) { return f2(rcp_ftz(x.x), rcp_ftz(x.y)); }
 
 __device__ __forceinline__ F2 symsum3(F2 a0, F2 a1, F2 a2) { return (a0 + a2) + a1; }
-__device__ __forceinline__ F2 symsum2(F2 a0, F2 a1) { return a0 + a1; }
 
-// limit_weight<float> of two weights: the two ramps in the scalar code's operations on the
-// packed pipe, the clamps per lane
+// The constants of the packed arithmetic, as pairs.  A packed operation takes its operands from
+// register pairs only, and the compiler rebuilds a literal pair with two moves at a use, so a
+// kernel makes the constants that are used often once, by an assembly statement that it cannot
+// repeat, and carries them in registers; a constant used once scales each lane by an immediate.
+struct WenoK {
+  F2 m1, m2, m4, c3, c6, k133, eps4, tiny, weps, m13, m10, p10, p5;
+};
+__device__ __forceinline__ F2 kept(float c) {
+  unsigned long long r;
+  asm volatile("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(c));
+  return make_float2(__uint_as_float((unsigned)r), __uint_as_float((unsigned)(r >> 32)));
+}
+// both lanes times a literal, as scalar products with an immediate operand
+__device__ __forceinline__ F2 scaled(F2 a, float k) { return f2(a.x * k, a.y * k); }
+__device__ __forceinline__ WenoK weno_consts() {
+  WenoK k;
+  k.m1 = kept(-1.0f); k.m2 = kept(-2.0f); k.m4 = kept(-4.0f);
+  k.c3 = kept(3.0f); k.c6 = kept(6.0f); k.k133 = kept((float)(13. / 3.)); k.eps4 = kept(4.0f * WenoEps<float>::eps);
+  k.tiny = kept(WenoEps<float>::tiny); k.weps = kept(WenoEps<float>::weps);
+  k.m13 = kept(-1.3f); k.m10 = kept(-10.0f); k.p10 = kept(10.0f); k.p5 = kept(5.0f);
+  return k;
+}
+
+// the five-point stencil of two cells: its centre u0, the differences m2 .. p2 of the others to
+// it, and the sums s and differences a of opposite ones
+struct Sten {
+  F2 u0, m2, m1, p1, p2, s1, a1, s2, a2;
+};
+// u points at the cells' centre values (u[-2..2])
+__device__ __forceinline__ Sten stencil_of(const WenoK& K, const F2* u) {
+  Sten s;
+  s.u0 = u[0];
+  s.m2 = ffma2(u[0], K.m1, u[-2]);
+  s.m1 = ffma2(u[0], K.m1, u[-1]);
+  s.p1 = ffma2(u[0], K.m1, u[1]);
+  s.p2 = ffma2(u[0], K.m1, u[2]);
+  s.s1 = s.p1 + s.m1;
+  s.a1 = ffma2(s.m1, K.m1, s.p1);
+  s.s2 = s.p2 + s.m2;
+  s.a2 = ffma2(s.m2, K.m1, s.p2);
+  return s;
+}
+
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// limit_weight<float> (0 | ramp to avg | avg | ramp to 1) of ORDER weights w[k] * r at most 1, in
+// units of avg: the lower ramp saturated to [0, 1] plus (1 - avg)/avg times the upper one; the
+// saturation is part of the multiply-add, where min/max would load the half-rate ALU
 template <int ORDER>
-__device__ __forceinline__ F2 limit_weight_f2(F2 w) {
+__device__ __forceinline__ void limit_weights_f2(F2* w, F2 r) {
   constexpr float avg = 1.0f / (float)ORDER, w1 = 0.2f * avg, w2 = (1.0f - 0.2f) * avg, w3 = (1.0f + 0.2f) * avg,
-                  w4 = 1.0f;
-  const F2 lo = (f2(avg) * (w - f2(w1))) * f2(1.0f / (w2 - w1));
-  const F2 up = ((w - f2(w3)) * f2(w4 - avg)) * f2(1.0f / (w4 - w3));
-  return f2(fmaxf(fminf(lo.x, avg), 0.0f), fmaxf(fminf(lo.y, avg), 0.0f)) + f2(fmaxf(up.x, 0.0f), fmaxf(up.y, 0.0f));
-}
-__device__ __forceinline__ F2 limit_weight3_f2(F2 w) { return limit_weight_f2<3>(w); }
-__device__ __forceinline__ F2 limit_weight2_f2(F2 w) { return limit_weight_f2<2>(w); }
-
-// weno5_unopt of two cells: u points at the cells' centre values (u[-2..2])
-__device__ __forceinline__ void weno5_unopt_f2(const F2* u, F2* w) {
-  const F2 c3 = f2(3.0f), c4 = f2(4.0f), c2 = f2(2.0f), k13 = f2((float)(13. / 12.)), k14 = f2(0.25f);
-  const F2 fd0 = (c4 * u[1]) - ffma2(c3, u[0], u[2]);
-  const F2 fd1 = u[1] - u[-1];
-  const F2 fd2 = ffma2(c3, u[0], u[-2]) - (c4 * u[-1]);
-  const F2 sd0 = (u[0] + u[2]) - (c2 * u[1]);
-  const F2 sd1 = (u[-1] + u[1]) - (c2 * u[0]);
-  const F2 sd2 = (u[0] + u[-2]) - (c2 * u[-1]);
-  F2 b[3];
-  b[0] = ffma2(k13 * sd0, sd0, k14 * fd0 * fd0);
-  b[1] = ffma2(k13 * sd1, sd1, k14 * fd1 * fd1);
-  b[2] = ffma2(k13 * sd2, sd2, k14 * fd2 * fd2);
-  const F2 normu = ffma2(u[0], u[0], ffma2(u[-1], u[-1], u[1] * u[1]) + ffma2(u[-2], u[-2], u[2] * u[2]));
-  const F2 ee = normu * f2(WenoEps<float>::eps);
+                  w4 = 1.0f, kl = 1.0f / (w2 - w1), ku = 1.0f / (w4 - w3);
+  const float lx = r.x * kl, ly = r.y * kl, ux = r.x * ku, uy = r.y * ku;
 #pragma unroll
-  for (int s = 0; s < 3; s++) b[s] = b[s] + ee;
-  const F2 rb = rcp2(symsum3(b[0], b[1], b[2]) + f2(WenoEps<float>::tiny));
-#pragma unroll
-  for (int s = 0; s < 3; s++) {
-    const F2 t = ffma2(b[s], rb, f2(WenoEps<float>::weps));  // contracted, as the scalar FP32 code
-    w[s] = rcp2(t * t);
+  for (int k = 0; k < ORDER; k++) {
+    const F2 lo = f2(fma_sat(w[k].x, lx, -kl * w1), fma_sat(w[k].y, ly, -kl * w1));
+    const F2 up = f2(fma_sat(w[k].x, ux, -ku * w3), fma_sat(w[k].y, uy, -ku * w3));
+    w[k] = lo + up;
+    if (ORDER == 3) w[k] = w[k] + up;
   }
-  const F2 r1 = rcp2(symsum3(w[0], w[1], w[2]));
-#pragma unroll
-  for (int s = 0; s < 3; s++) w[s] = limit_weight3_f2(w[s] * r1);
-  const F2 r2 = rcp2(symsum3(w[0], w[1], w[2]));
-#pragma unroll
-  for (int s = 0; s < 3; s++) w[s] = w[s] * r2;
 }
 
-__device__ __forceinline__ void weno3_unopt_f2(const F2* u, F2* w) {
-  const F2 fd0 = u[1] - u[0], fd1 = u[0] - u[-1];
-  F2 b[2] = {fd0 * fd0, fd1 * fd1};
-  const F2 normu = ffma2(u[0], u[0], ffma2(u[-1], u[-1], u[1] * u[1]));
-  const F2 ee = normu * f2(WenoEps<float>::eps);
-  b[0] = b[0] + ee;
-  b[1] = b[1] + ee;
-  const F2 rb = rcp2(symsum2(b[0], b[1]) + f2(WenoEps<float>::tiny));
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const F2 t = ffma2(b[s], rb, f2(WenoEps<float>::weps));  // contracted, as the scalar FP32 code
-    w[s] = rcp2(t * t);
-  }
-  const F2 r1 = rcp2(symsum2(w[0], w[1]));
-  w[0] = limit_weight2_f2(w[0] * r1);
-  w[1] = limit_weight2_f2(w[1] * r1);
-  const F2 r2 = rcp2(symsum2(w[0], w[1]));
-  w[0] = w[0] * r2;
-  w[1] = w[1] * r2;
+// the smoothness weights 1/t^2 of three stencils up to the common factor (t0 t1 t2)^2, limited,
+// in units of avg; b: the regularised measures.  The t sum to one and none is below weps, so the
+// largest of the three is at least (weps/3)^2, a normal FP32 number, and a product that
+// underflows belongs to a weight below 1e-18 of it, which the limiter sets to zero.
+__device__ __forceinline__ void smooth3_f2(const WenoK& K, const F2* b, F2* w) {
+  const F2 rb = rcp2(symsum3(b[0], b[1], b[2]));
+  const F2 t0 = ffma2(b[0], rb, K.weps), t1 = ffma2(b[1], rb, K.weps), t2 = ffma2(b[2], rb, K.weps);
+  const F2 q0 = t1 * t2, q1 = t0 * t2, q2 = t0 * t1;
+  w[0] = q0 * q0;
+  w[1] = q1 * q1;
+  w[2] = q2 * q2;
+  limit_weights_f2<3>(w, rcp2(symsum3(w[0], w[1], w[2])));
 }
 
-// Weights times stencil values: eno_cvt skips zero weights; for the finite stencil values of
-// finite data the product of a zero weight is a zero anyway (at most of the other sign, which
-// no later sum can tell apart), so the packed path multiplies (and fuses the sums).
-__device__ __forceinline__ F2 nz_mul(F2 wgt, F2 x) { return wgt * x; }
+__device__ __forceinline__ float min_abs3(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
-// smono_indicator<float> of two cells: the derivative combinations on the packed pipe, the
-// min-mods and clamps per lane
-__device__ __forceinline__ F2 smono_indicator_f2(const F2* y) {
-  const F2 r12 = f2(1.0f / 12.0f), h = f2(0.5f);
-  const F2 ld1 = (((f2(-3.f) * y[-2] + y[2]) + (f2(-10.f) * y[-1] - f2(6.f) * y[1])) + f2(18.f) * y[0]) * r12;
-  const F2 ld2 = (((f2(11.f) * y[-2] - y[2]) + (f2(-20.f) * y[-1] + f2(4.f) * y[1])) + f2(6.f) * y[0]) * r12;
-  const F2 ld3 = (((f2(-3.f) * y[-2] - y[2]) + (f2(10.f) * y[-1] + f2(6.f) * y[1])) - f2(12.f) * y[0]) * h;
-  const F2 rd1 = (((y[2] * f2(3.f) - y[-2]) + (f2(6.f) * y[-1] + f2(10.f) * y[1])) - f2(18.f) * y[0]) * r12;
-  const F2 rd2 = (((y[2] * f2(11.f) - y[-2]) + (f2(4.f) * y[-1] - f2(20.f) * y[1])) + f2(6.f) * y[0]) * r12;
-  const F2 rd3 = (((y[-2] + f2(3.f) * y[2]) - (f2(6.f) * y[-1] + f2(10.f) * y[1])) + f2(12.f) * y[0]) * h;
-  const F2 d1l = y[-1] - y[-2], d1r = y[2] - y[1];
-  auto one = [](float y0, float ym1, float yp1, float ym2, float yp2, float l1, float l2, float l3, float r1, float r2,
-                float r3, float dl, float dr) {
-    auto mm = [](float a, float b) { return (a * b <= 0.0f) ? 0.0f : ((fabsf(a) < fabsf(b)) ? a : b); };
-    l1 = mm(l1, dl);
-    r1 = mm(r1, dr);
-    const float minabs = fminf(fminf(fabsf(mm(l1, r1)), fabsf(mm(l2, r2))), fabsf(mm(l3, r3)));
-    const float norm = fabsf(y0) + ((fabsf(ym1) + fabsf(yp1)) + (fabsf(ym2) + fabsf(yp2)));
-    const float v = __fdividef(minabs, norm * WenoEps<float>::smono + WenoEps<float>::tiny);
-    return fmaxf(fminf(v, 1.0f), 0.0f);
+// smono_indicator<float> of two cells.  Six times the left and right edge derivatives of orders
+// 1..3 of the 5-point polynomial, each pair a sum and a difference of the same two terms built
+// from the third and fourth differences h, e; the smallest magnitude of a min-mod chain is the
+// smallest of all where the signs agree and zero where any differs.
+__device__ __forceinline__ F2 smono_indicator_f2(const WenoK& K, const Sten& s, const F2* u) {
+  const F2 e = ffma2(K.m4, s.s1, s.s2), h = ffma2(K.m2, s.a1, s.a2), g = scaled(s.s2, 1.5f);
+  const F2 z = g + e, y = ffma2(e, K.m1, g), x = s.a1 + s.a2;
+  const F2 l1 = ffma2(y, K.m1, x), r1 = x + y;
+  const F2 h3 = K.c3 * h;
+  const F2 l2 = ffma2(h3, K.m1, z), r2 = z + h3;
+  const F2 l3 = K.c3 * ffma2(K.m2, e, h), r3 = ffma2(K.c6, e, h3);
+  const F2 dl = K.c6 * ffma2(s.m2, K.m1, s.m1), dr = K.c6 * ffma2(s.p1, K.m1, s.p2);
+  auto one = [](float l1, float r1, float l2, float r2, float l3, float r3, float dl, float dr, float cut, bool& part) {
+    const unsigned a = __float_as_uint(l1);
+    const unsigned differ = (a ^ __float_as_uint(r1)) | (a ^ __float_as_uint(dl)) | (a ^ __float_as_uint(dr)) |
+                            (__float_as_uint(l2) ^ __float_as_uint(r2)) | (__float_as_uint(l3) ^ __float_as_uint(r3));
+    float v = min_abs3(min_abs3(l1, r1, dl), min_abs3(dr, l2, r2), min_abs3(l3, r3, l3));
+    v = ((int)differ < 0) ? 0.0f : v;
+    part = part || (v > 0.0f && v < cut);
+    return v;
   };
-  return f2(one(y[0].x, y[-1].x, y[1].x, y[-2].x, y[2].x, ld1.x, ld2.x, ld3.x, rd1.x, rd2.x, rd3.x, d1l.x, d1r.x),
-            one(y[0].y, y[-1].y, y[1].y, y[-2].y, y[2].y, ld1.y, ld2.y, ld3.y, rd1.y, rd2.y, rd3.y, d1l.y, d1r.y));
+  auto cutoff = [](float u0, float um1, float up1, float um2, float up2) {
+    const float norm = fabsf(u0) + ((fabsf(um1) + fabsf(up1)) + (fabsf(um2) + fabsf(up2)));
+    return fmaf(norm, 6.0f * WenoEps<float>::smono, 6.0f * WenoEps<float>::tiny);
+  };
+  const float ca = cutoff(u[0].x, u[-1].x, u[1].x, u[-2].x, u[2].x), cb = cutoff(u[0].y, u[-1].y, u[1].y, u[-2].y, u[2].y);
+  bool part = false;
+  const float va = one(l1.x, r1.x, l2.x, r2.x, l3.x, r3.x, dl.x, dr.x, ca, part);
+  const float vb = one(l1.y, r1.y, l2.y, r2.y, l3.y, r3.y, dl.y, dr.y, cb, part);
+  if (part)  // rare: derivatives within 500 epsilons of the stencil's size
+    return f2(va < ca ? __fdividef(va, ca) : 1.0f, vb < cb ? __fdividef(vb, cb) : 1.0f);
+  return f2(va >= ca ? 1.0f : 0.0f, vb >= cb ? 1.0f : 0.0f);
 }
 
-// weno5_cell_weights<float> of two cells: (1 - m) w + m/3 is w itself for m = 0 and exactly
-// 1/3 for m = 1 (finite w), so both lanes take the blend; the unoptimised weights are skipped
-// when both cells are monotone
-__device__ __forceinline__ void weno5_cell_weights_f2(const F2* u, F2 m, F2* w) {
+// weno5_cell_weights<float> of two cells: the unoptimised weights blended towards 1/3 by m
+// ((1 - m) w + m/3 is w itself for m = 0 and exactly 1/3 for m = 1), skipped when both cells
+// are monotone.  The smoothness measures are 4 times the reference's (they are only ever
+// normalised by their sum), their regularisation with them; the smallest normal number is
+// added to each instead of to their sum, so that a zero line has equal weights.
+__device__ __forceinline__ void weno5_cell_weights_f2(const WenoK& K, const Sten& s, const F2* u, F2 m, F2* w) {
   if (m.x == 1.0f && m.y == 1.0f) {
     w[0] = w[1] = w[2] = f2(1.0f / 3.0f);
     return;
   }
-  weno5_unopt_f2(u, w);
-  const F2 omm = f2(1.0f) - m, mt = m * f2(1.0f / 3.0f);
+  const F2 fd0 = ffma2(K.m4, s.p1, s.p2), fd2 = ffma2(K.m4, s.m1, s.m2);
+  const F2 sd0 = ffma2(K.m2, s.p1, s.p2), sd2 = ffma2(K.m2, s.m1, s.m2);
+  const F2 normu = ffma2(u[0], u[0], ffma2(u[-1], u[-1], u[1] * u[1]) + ffma2(u[-2], u[-2], u[2] * u[2]));
+  const F2 ee = ffma2(normu, K.eps4, K.tiny);
+  F2 b[3];
+  b[0] = ffma2(K.k133 * sd0, sd0, ffma2(fd0, fd0, ee));
+  b[1] = ffma2(K.k133 * s.s1, s.s1, ffma2(s.a1, s.a1, ee));
+  b[2] = ffma2(K.k133 * sd2, sd2, ffma2(fd2, fd2, ee));
+  smooth3_f2(K, b, w);
+  const F2 r = rcp2(symsum3(w[0], w[1], w[2])) * f2(1.0f - m.x, 1.0f - m.y), mt = scaled(m, 1.0f / 3.0f);
 #pragma unroll
-  for (int s = 0; s < 3; s++) w[s] = ffma2(omm, w[s], mt);
+  for (int k = 0; k < 3; k++) w[k] = ffma2(w[k], r, mt);
 }
 
-// weno_frac<float> of two cells
-__device__ __forceinline__ F2 weno_frac_f2(const F2* w, const F2* wm, const F2* wp) {
-  const F2 E = f2(WenoEps<float>::eps);
-  const F2 rl = (w[2] + E) * rcp2(wm[0] + E);  // the weight ratios: a fast reciprocal per lane
-  const F2 rr = (w[0] + E) * rcp2(wp[2] + E);
-  const F2 ratio = lanes(rl, rr, [](float a, float b) { return fminf(a, b); });
-  return lanes((ratio - f2(1.3f)) * f2(1.0f / (1.6f - 1.3f)), [](float a) { return fmaxf(0.0f, fminf(a, 1.0f)); });
+// weno_frac<float> of two cells from their outer weights and their neighbours' (at distance 2)
+// inner ones: the smaller weight ratio on a ramp from 1.3 to 1.6
+__device__ __forceinline__ F2 weno_frac_f2(const WenoK& K, F2 w0, F2 w2, F2 wm0, F2 wp2) {
+  const F2 el = ffma2(K.m13, wm0, w2), er = ffma2(K.m13, wp2, w0);  // ratio above 1.3 where positive
+  const float ea = fminf(el.x, er.x), eb = fminf(el.y, er.y);
+  if (fmaxf(ea, eb) > 0.0f) {
+    constexpr float E = WenoEps<float>::eps, s = 1.0f / (1.6f - 1.3f);
+    const float xa = fminf(el.x * rcp_ftz(wm0.x + E), er.x * rcp_ftz(wp2.x + E));
+    const float xb = fminf(el.y * rcp_ftz(wm0.y + E), er.y * rcp_ftz(wp2.y + E));
+    return f2(__saturatef(xa * s), __saturatef(xb * s));
+  }
+  return f2(0.0f);
 }
 
 // weno5_edges<float> of two cells from their weights w, final lower-order fractions f and
 // SMONO indicators m.  (1 - m) out + m y5 is out for m = 0 and y5 for m = 1 (finite out), so
 // the packed code blends both lanes; it skips the WENO sums when both cells are monotone and
-// the 5-point values when neither is partly monotone.
-// Offset form: every candidate edge value is the cell's value plus a combination of the
-// differences d_k = u_k - u_0 (each stencil's coefficients sum to one), and the weighted
-// combination is u_0 + sum_k w_k (rec_k - u_0).  In exact arithmetic this is the scalar
-// code's sum_k w_k rec_k (the normalised weights sum to one); in FP32 the rounding of the
-// weights' normalisation then scales only the offsets, not the cell value, so a constant
-// line reconstructs to its value exactly and the reconstruction carries no bias of the
-// order of that rounding times the value, which a near-steady flow would accumulate step
-// after step.
-__device__ __forceinline__ void weno5_edges_f2(const F2* u, const F2* w, F2 f, F2 m, F2& yl, F2& yr) {
-  const F2 dm2 = u[-2] - u[0], dm1 = u[-1] - u[0], dp1 = u[1] - u[0], dp2 = u[2] - u[0];
+// the 5-point values when neither is partly monotone.  Every edge value is the cell's value
+// plus a weighted combination of the differences (each stencil's coefficients sum to one), so
+// the rounding of the weights' normalisation scales only the offsets: the reconstruction
+// carries no bias of that rounding times the value, which a near-steady flow would accumulate
+// step after step.  The combinations are 8 (WENO5), 2 (WENO3) and 128 (5-point) times their
+// values, the weights 16 and 4 times theirs.
+__device__ __forceinline__ void weno5_edges_f2(const WenoK& K, const Sten& s, const F2* u, const F2* w, F2 f, F2 m, F2& yl,
+                                               F2& yr) {
   F2 o5l = f2(0.0f), o5r = f2(0.0f);
-  if (m.x != 0.0f || m.y != 0.0f) {
-    const F2 c0 = f2(-5.f / 128.f), c1 = f2(15.f / 32.f), c3 = f2(-5.f / 32.f), c4 = f2(3.f / 128.f);
-    o5l = ffma2(c1, dm1, c3 * dp1) + ffma2(c0, dm2, c4 * dp2);
-    o5r = ffma2(c3, dm1, c1 * dp1) + ffma2(c4, dm2, c0 * dp2);
-    if (m.x >= 1.0f && m.y >= 1.0f) {
-      yl = u[0] + o5l;
-      yr = u[0] + o5r;
+  if (fmaxf(m.x, m.y) > 0.0f) {
+    const F2 a = ffma2(s.s2, K.m1, scaled(s.s1, 20.0f)), c = K.m4 * ffma2(K.m10, s.a1, s.a2);
+    constexpr float k = 1.0f / 128.0f;
+    const F2 mk = scaled(m, k);
+    o5l = ffma2(c, K.m1, a) * mk;  // 60 d-1 - 20 d1 - 5 d-2 + 3 d2, and mirrored
+    o5r = (a + c) * mk;
+    if (fminf(m.x, m.y) >= 1.0f) {
+      yl = s.u0 + o5l;
+      yr = s.u0 + o5r;
       return;
     }
   }
-  F2 wl[3] = {w[0] * f2(1.f / 16.f), w[1] * f2(5.f / 8.f), w[2] * f2(5.f / 16.f)};
-  F2 wr[3] = {w[0] * f2(5.f / 16.f), w[1] * f2(5.f / 8.f), w[2] * f2(1.f / 16.f)};
-  const F2 nl = rcp2(symsum3(wl[0], wl[1], wl[2]) + f2(WenoEps<float>::tiny));
-  const F2 nr = rcp2(symsum3(wr[0], wr[1], wr[2]) + f2(WenoEps<float>::tiny));
-  float fa, fb;
-  f2split(f, fa, fb);
-  const bool two = (0.0f < fa) || (0.0f < fb);
-  const F2 omf = f2(1.0f) - f;
-#pragma unroll
-  for (int s = 0; s < 3; s++) {
-    wl[s] = wl[s] * nl;
-    wr[s] = wr[s] * nr;
-    if (two) {
-      wl[s] = wl[s] * omf;
-      wr[s] = wr[s] * omf;
-    }
+  // optimal face weights (1, 10, 5)/16 and mirrored; the stencils' edge values less u_0 are
+  // (-10 d1 + 3 d2)/8, (3 d-1 - d1)/8, (-d-2 + 6 d-1)/8
+  const F2 w1 = K.p10 * w[1], wl2 = K.p5 * w[2], wr0 = K.p5 * w[0];
+  const F2 sl = rcp2((w[0] + w1) + wl2), sr = rcp2((w[2] + w1) + wr0);
+  const F2 l0 = ffma2(K.m10, s.p1, K.c3 * s.p2), l1 = ffma2(s.p1, K.m1, K.c3 * s.m1), l2 = ffma2(s.m2, K.m1, K.c6 * s.m1);
+  const F2 r0 = ffma2(s.p2, K.m1, K.c6 * s.p1), r1 = ffma2(s.m1, K.m1, K.c3 * s.p1), r2 = ffma2(K.m10, s.m1, K.c3 * s.m2);
+  const F2 nl = scaled(sl, 0.125f), nr = scaled(sr, 0.125f);
+  F2 outl = ffma2(w1, l1, ffma2(w[0], l0, wl2 * l2)) * nl;
+  F2 outr = ffma2(w1, r1, ffma2(w[2], r2, wr0 * r0)) * nr;
+  if (fmaxf(f.x, f.y) > 0.0f) {
+    // the WENO3 blend: unoptimised weights of the two 2-point stencils, optimal weights (1, 3)/4
+    const F2 normu = ffma2(u[0], u[0], ffma2(u[-1], u[-1], u[1] * u[1]));
+    const F2 ee = ffma2(normu, f2(WenoEps<float>::eps), K.tiny);
+    const F2 b0 = ffma2(s.p1, s.p1, ee), b1 = ffma2(s.m1, s.m1, ee);
+    const F2 rb = rcp2(b0 + b1);
+    const F2 t0 = ffma2(b0, rb, K.weps), t1 = ffma2(b1, rb, K.weps);
+    F2 v[2] = {t1 * t1, t0 * t0};
+    limit_weights_f2<2>(v, rcp2(v[0] + v[1]));
+    const F2 v0 = K.c3 * v[0], v1 = K.c3 * v[1];
+    const F2 nl3 = rcp2(v[0] + v1), nr3 = rcp2(v0 + v[1]);
+    // -d1 and d-1 of the left edge, d1 and -d-1 of the right one, each times 1/2
+    const F2 t3l = ffma2(v1, s.m1, (v[0] * K.m1) * s.p1) * scaled(nl3, 0.5f);
+    const F2 t3r = ffma2(v0, s.p1, (v[1] * K.m1) * s.m1) * scaled(nr3, 0.5f);
+    const F2 omf = f2(1.0f - f.x, 1.0f - f.y);
+    outl = ffma2(omf, outl, f * t3l);
+    outr = ffma2(omf, outr, f * t3r);
   }
-  const F2 k54 = f2(-5.f / 4.f), k38 = f2(3.f / 8.f), k34 = f2(3.f / 4.f), k18 = f2(-1.f / 8.f);
-  // the stencils' edge values less u_0: (15/8, -5/4, 3/8) -> -5/4 d1 + 3/8 d2, and so on
-  const F2 recl0 = ffma2(k54, dp1, k38 * dp2);
-  const F2 recl1 = ffma2(k38, dm1, k18 * dp1);
-  const F2 recl2 = ffma2(k18, dm2, k34 * dm1);
-  const F2 recr0 = ffma2(k34, dp1, k18 * dp2);
-  const F2 recr1 = ffma2(k18, dm1, k38 * dp1);
-  const F2 recr2 = ffma2(k38, dm2, k54 * dm1);
-  auto poly3 = [](F2 k0, F2 x0, F2 k1, F2 x1, F2 k2, F2 x2) { return ffma2(k1, x1, ffma2(k0, x0, k2 * x2)); };
-  F2 outl = poly3(wl[0], recl0, wl[1], recl1, wl[2], recl2);
-  F2 outr = poly3(wr[0], recr0, wr[1], recr1, wr[2], recr2);
-  if (two) {
-    F2 w3[2];
-    weno3_unopt_f2(u, w3);
-    F2 l3[2] = {w3[0] * f2(0.25f), w3[1] * f2(0.75f)};
-    F2 r3[2] = {w3[0] * f2(0.75f), w3[1] * f2(0.25f)};
-    const F2 nl3 = rcp2(symsum2(l3[0], l3[1]) + f2(WenoEps<float>::tiny));
-    const F2 nr3 = rcp2(symsum2(r3[0], r3[1]) + f2(WenoEps<float>::tiny));
-#pragma unroll
-    for (int s = 0; s < 2; s++) {
-      l3[s] = (l3[s] * nl3) * f;
-      r3[s] = (r3[s] * nr3) * f;
-    }
-    const F2 h = f2(0.5f), km12 = f2(-0.5f);
-    // (3/2, -1/2) -> -1/2 d1; (1/2, 1/2) -> 1/2 d-1; (1/2, 1/2) -> 1/2 d1; (-1/2, 3/2) -> -1/2 d-1
-    outl = outl + ffma2(l3[0], km12 * dp1, nz_mul(l3[1], h * dm1));
-    outr = outr + ffma2(r3[0], h * dp1, nz_mul(r3[1], km12 * dm1));
-  }
-  const F2 omm = f2(1.0f) - m;
-  yl = u[0] + ffma2(omm, outl, m * o5l);
-  yr = u[0] + ffma2(omm, outr, m * o5r);
+  const F2 omm = f2(1.0f - m.x, 1.0f - m.y);
+  yl = s.u0 + ffma2(omm, outl, o5l);
+  yr = s.u0 + ffma2(omm, outr, o5r);
 }
 
 }  // namespace hb

@@ -1,0 +1,73 @@
+"""The flux stage's two kernels at the edges of their ranges: lines shorter than a warp's 32 or 64,
+grids of a few cells, segments and chunks with a remainder, one plane and several, with the
+reduction of WENO5BND (a planted pressure jump) and the PARALINE flattener active.  FP64 against
+the oracle to 1e-12 of each field's largest face value; FP32 (mixed path) against the FP64 path:
+both reconstruct the same state, and a face flux carries the rounding of a few dozen FP32
+operations on the face's largest terms, of which a substep adds dt/dx < 1: 64 half-ulps of a
+field's largest value (of the state's, for the vectors, whose components share their terms), in
+all but the hundredth of the cells next to those that the jump leaves without a solution, where the
+inversion multiplies rounding without bound."""
+from fractions import Fraction
+
+import numpy as np
+import pytest
+
+from helpers import make_torus, plant_compression, rel_err
+from harm_harm_b200 import HARM_PREC_FP64, HARM_PREC_MIXED, Harm
+from oracle import oracle as O
+
+SHAPES = [(5, 7, 1), (59, 9, 1), (33, 21, 6), (64, 13, 7), (131, 8, 12), (17, 70, 9)]
+
+
+def _faces(g, d):
+    gg = g.g
+    return (slice(None), slice(gg.ng3, gg.ng3 + gg.n3 + (d == 3)), slice(gg.ng, gg.ng + gg.n2 + (d == 2)),
+            slice(gg.ng, gg.ng + gg.n1 + (d == 1)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lim", [0, 1, 2, 3])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_flux_edges(cuda, shape, lim):
+    g, geom, conn, aux, P = make_torus(*shape, lim=lim)
+    plant_compression(g, P)
+    orc = O.Oracle(g, geom, conn, aux)
+    orc.bound_prim(P)
+    Fo = [np.zeros_like(P) for _ in range(3)]
+    ndt = orc.fluxcalc(P, *Fo)
+    dev = Harm(g, geom, conn, aux)
+    Pd = cuda.from_numpy(P).cuda()
+    Fd = [cuda.zeros_like(Pd) for _ in range(3)]
+    got = dev.fluxcalc(Pd, *Fd)
+    for d in range(3 if shape[2] > 1 else 2):
+        a, b = Fd[d].cpu().numpy()[_faces(g, d + 1)], Fo[d][_faces(g, d + 1)]
+        for pl in range(8):
+            assert rel_err(a[pl], b[pl]) < 1e-12, (d + 1, pl)
+        assert abs(got[d] - ndt[d]) <= 1e-12 * ndt[d]
+    dt = 0.2 / sum(1.0 / x for x in ndt if x < 1e99)
+    out, ok = [], True
+    for prec in (HARM_PREC_FP64, HARM_PREC_MIXED):
+        pf, flag = cuda.zeros_like(Pd), cuda.zeros(P.shape[1:], dtype=cuda.int8, device="cuda")
+        dev.advance(0, Pd, Pd, pf, flag, dt, precision=prec)
+        out.append(pf.cpu().numpy()[(slice(None), *g.active)])
+        ok = ok & (flag.cpu().numpy()[g.active] == 0)  # the jump leaves a few cells without a solution
+    assert ok.mean() > 0.9
+    for pl in range(8):
+        own, most = np.abs(out[0][pl]).max(), np.abs(out[0]).max()
+        diff = np.sort(np.abs(out[1][pl] - out[0][pl])[ok])
+        assert diff[int(0.99 * (diff.size - 1))] < 64 * 2.0**-24 * (own + (pl >= 2) * most), pl
+
+
+def test_corrected_quotients_are_ieee():
+    """The WENO sums' division by a shared denominator (a y corrected by its exact remainder, y the
+    rounded reciprocal), in exact rational arithmetic with each operation rounded: the IEEE quotient
+    for random operands and for the constants it divides by."""
+    rng = np.random.default_rng(5)
+    dens = list(10.0 ** rng.uniform(-12, 12, 300)) + [12.0, 1.6 - 1.3, 0.8 * (1 / 3) - 0.2 * (1 / 3), 1 - 1.2 * (1 / 3), 2.2250738585072014e-308]
+    for b in dens:
+        y = 1.0 / b
+        for a in rng.uniform(-1, 1, 20) * b * 10.0 ** rng.uniform(-9, 3, 20):
+            q = float(a) * y
+            r = float(Fraction(float(a)) - Fraction(b) * Fraction(q))  # fma(-b, q, a): one rounding
+            got = float(Fraction(r) * Fraction(y) + Fraction(q))       # fma(r, y, q)
+            assert got == float(a) / b
