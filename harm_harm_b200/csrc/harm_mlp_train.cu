@@ -2,11 +2,11 @@
 //
 // Training runs in FP32 with hand-written kernels:
 //   k_mlp_grad   forward and backward pass of the 10-64-64-64-2 SiLU network over a
-//                minibatch; each block owns a slice of the samples, keeps the parameters,
-//                activations and its gradient accumulators in shared memory (208 KB) and
+//                minibatch; each block owns a slice of the samples, keeps the parameters and
+//                activations in shared memory (181 KB) and its gradients in registers, and
 //                writes one partial gradient, so the reduction order is fixed
 //                (deterministic gradients);
-//   k_mlp_adam   sums the partial gradients in block order and applies Adam;
+//   k_mlp_adam   sums the partial gradients in a fixed order and applies Adam;
 //   k_mlp_norm   feature/target means and standard deviations (one block, FP64 sums);
 //   k_mlp_init   Glorot-uniform weights, zero biases, from a counter-based hash.
 // Loss: L = 1/(2n) sum_samples sum_outputs (y - t~)^2 over the standardised targets t~.
@@ -24,10 +24,12 @@ int hb_setmsg(const char* msg, int code);
 namespace {
 
 constexpr int TS = 64;           // samples per chunk
-constexpr int NPP = 9156;        // parameters padded to a multiple of 4
-constexpr int TR_GRID = 128;     // blocks of one training step
-constexpr size_t TR_SMEM = (size_t)(2 * NPP + TS * MLP_IN + 6 * TS * MLP_H + TS * 2 + 2 * TS * MLP_H + TS * 2 + 8) * 4;
-static_assert(MLP_NPARAMS <= NPP, "padding");
+constexpr int TP = TS + 4;       // row pitch of the shared-memory matrices
+constexpr int TR_GRID = 148;     // blocks of one training step at most
+// parameters (W2, W3 with padded rows), then activations [feature][sample]: inputs, the three
+// layers' outputs, and their derivatives, which become the layers' deltas in place
+constexpr int TM = MLP_H * TP;   // floats of one 64 x 64 matrix
+constexpr size_t TR_SMEM = (size_t)(MLP_IN * MLP_H + 3 * MLP_H + MLP_H * MLP_OUT + 4 + 8 * TM + MLP_IN * TP + 4 * TS + 8) * 4;
 
 __device__ __forceinline__ uint64_t smix(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -36,89 +38,142 @@ __device__ __forceinline__ uint64_t smix(uint64_t x) {
   return x ^ (x >> 31);
 }
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float dsilu_f(float z) {
-  const float s = 1.0f / (1.0f + expf(-z));
-  return s * (1.0f + z * (1.0f - s));
-}
-
-// Z = Hin W + b over a chunk (64 samples x 64 outputs); Hout = silu(Z)
-__device__ __forceinline__ void dense64(const float* Hin, const float* W, const float* b, float* Z, float* Hout) {
-  for (int e = threadIdx.x; e < TS * MLP_H; e += blockDim.x) {
-    const int s = e >> 6, o = e & 63;
-    float z = b[o];
-    const float* h = Hin + s * MLP_H;
+// 4 x 4 register tiles of 64 x 64 products; thread (tx, ty) of 16 x 16.  All matrices have rows
+// of TP floats, activations [feature][sample].  Each 16-byte load feeds eight multiply-adds, and
+// the rows' padding keeps the loads of neighbouring lanes in different banks.
+//
+// acc[a][b] += sum_k W[k][4 tx + a] H[k][4 ty + b]
+template <int K>
+__device__ __forceinline__ void mm_rows(const float* W, int wp, const float* H, int tx, int ty, float (&acc)[4][4]) {
 #pragma unroll 8
-    for (int k = 0; k < MLP_H; k++) z += h[k] * W[k * MLP_H + o];
-    Z[e] = z;
-    Hout[e] = silu_f(z);
+  for (int k = 0; k < K; k++) {
+    const float4 w = *reinterpret_cast<const float4*>(W + k * wp + 4 * tx);
+    const float4 h = *reinterpret_cast<const float4*>(H + k * TP + 4 * ty);
+    const float wv[4] = {w.x, w.y, w.z, w.w}, hv[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) acc[a][b] = fmaf(wv[a], hv[b], acc[a][b]);
   }
 }
-
-// gW[i][o] += sum_s Hin[s][i] D[s][o];  gb[o] += sum_s D[s][o]
-__device__ __forceinline__ void wgrad64(const float* Hin, int nin, const float* D, float* gW, float* gb) {
-  for (int e = threadIdx.x; e < nin * MLP_H; e += blockDim.x) {
-    const int i = e >> 6, o = e & 63;
-    float a = 0.0f;
-#pragma unroll 8
-    for (int s = 0; s < TS; s++) a += Hin[s * nin + i] * D[s * MLP_H + o];
-    gW[e] += a;
-  }
-  for (int o = threadIdx.x; o < MLP_H; o += blockDim.x) {
-    float a = 0.0f;
-    for (int s = 0; s < TS; s++) a += D[s * MLP_H + o];
-    gb[o] += a;
-  }
-}
-
-// Dout[s][i] = silu'(Zprev[s][i]) * sum_o Din[s][o] W[i][o]  (o rotated by i: no bank conflicts)
-__device__ __forceinline__ void bwd64(const float* Din, const float* W, const float* Zprev, float* Dout) {
-  for (int e = threadIdx.x; e < TS * MLP_H; e += blockDim.x) {
-    const int s = e >> 6, i = e & 63;
-    const float* dz = Din + s * MLP_H;
-    const float* w = W + i * MLP_H;
-    float a = 0.0f;
-#pragma unroll 8
-    for (int oo = 0; oo < MLP_H; oo++) {
-      const int o = (oo + i) & 63;
-      a += dz[o] * w[o];
+// acc[a][b] += sum_o W[tx + 16 a][o] D[o][4 ty + b]
+__device__ __forceinline__ void mm_back(const float* W, const float* D, int tx, int ty, float (&acc)[4][4]) {
+#pragma unroll 2
+  for (int o = 0; o < MLP_H; o += 4) {
+    float4 w[4], d[4];
+#pragma unroll
+    for (int a = 0; a < 4; a++) w[a] = *reinterpret_cast<const float4*>(W + (tx + 16 * a) * TP + o);
+#pragma unroll
+    for (int q = 0; q < 4; q++) d[q] = *reinterpret_cast<const float4*>(D + (o + q) * TP + 4 * ty);
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      const float wv[4] = {w[a].x, w[a].y, w[a].z, w[a].w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float dv[4] = {d[q].x, d[q].y, d[q].z, d[q].w};
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = fmaf(wv[q], dv[b], acc[a][b]);
+      }
     }
-    Dout[e] = a * dsilu_f(Zprev[e]);
+  }
+}
+// acc[a][b] += sum_s H[ty + 16 a][s] D[tx + 16 b][s]: the weights' gradient of a chunk
+__device__ __forceinline__ void mm_grad(const float* H, const float* D, int tx, int ty, float (&acc)[4][4]) {
+#pragma unroll 2
+  for (int s = 0; s < TS; s += 4) {
+    float4 h[4], d[4];
+#pragma unroll
+    for (int a = 0; a < 4; a++) h[a] = *reinterpret_cast<const float4*>(H + (ty + 16 * a) * TP + s);
+#pragma unroll
+    for (int b = 0; b < 4; b++) d[b] = *reinterpret_cast<const float4*>(D + (tx + 16 * b) * TP + s);
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        acc[a][b] = fmaf(h[a].x, d[b].x, acc[a][b]);
+        acc[a][b] = fmaf(h[a].y, d[b].y, acc[a][b]);
+        acc[a][b] = fmaf(h[a].z, d[b].z, acc[a][b]);
+        acc[a][b] = fmaf(h[a].w, d[b].w, acc[a][b]);
+      }
   }
 }
 
+// the outputs o = 4 tx + a of a layer for samples 4 ty + b from their pre-activations: SiLU into
+// H, its derivative into S
+__device__ __forceinline__ void put_layer(float* H, float* S, int tx, int ty, const float (&z)[4][4]) {
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    float h[4], d[4];
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const float s = 1.0f / (1.0f + expf(-z[a][b]));
+      h[b] = z[a][b] * s;
+      d[b] = s * (1.0f + z[a][b] * (1.0f - s));
+    }
+    *reinterpret_cast<float4*>(H + (4 * tx + a) * TP + 4 * ty) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4*>(S + (4 * tx + a) * TP + 4 * ty) = make_float4(d[0], d[1], d[2], d[3]);
+  }
+}
+// the deltas of rows i = tx + 16 a: S (the derivatives) times acc, in place
+__device__ __forceinline__ void put_delta(float* S, int tx, int ty, const float (&acc)[4][4]) {
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    float4* p = reinterpret_cast<float4*>(S + (tx + 16 * a) * TP + 4 * ty);
+    const float4 d = *p;
+    *p = make_float4(acc[a][0] * d.x, acc[a][1] * d.y, acc[a][2] * d.z, acc[a][3] * d.w);
+  }
+}
+
+// Forward and backward of the network over a block's samples, 64 at a time, in FP32.  Bounded by
+// the FMA pipe and the shared-memory loads that feed it, about evenly: one block of 256 threads
+// fills an SM's shared memory, each thread a 4 x 4 tile of every 64 x 64 product; the gradients
+// stay in registers over the block's chunks.  (With two scalar loads per multiply-add, from
+// layouts of one product each, a step of 8192 samples took 98 us and a pass over 131,072 samples
+// 1332 us; now 36 and 318 us.  512 threads with tiles of 4 x 2 took 43 and 378 us.)
 __global__ void __launch_bounds__(256, 1) k_mlp_grad(size_t ndata, const float* __restrict__ feat,
                                                      const float* __restrict__ targ, const float* __restrict__ norm,
                                                      const float* __restrict__ params, long long nbatch,
                                                      uint64_t seed, long long step, float inv_n,
                                                      float* __restrict__ partial, double* __restrict__ partial_loss) {
   extern __shared__ __align__(16) float sm[];
-  float* P = sm;
-  float* G = P + NPP;
-  float* X = G + NPP;
-  float* Z1 = X + TS * MLP_IN;
-  float* Z2 = Z1 + TS * MLP_H;
-  float* Z3 = Z2 + TS * MLP_H;
-  float* H1 = Z3 + TS * MLP_H;
-  float* H2 = H1 + TS * MLP_H;
-  float* H3 = H2 + TS * MLP_H;
-  float* DY = H3 + TS * MLP_H;
-  float* DA = DY + TS * 2;
-  float* DB = DA + TS * MLP_H;
-  float* T = DB + TS * MLP_H;
-  float* red = T + TS * 2;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < NPP; i += blockDim.x) {
-    P[i] = (i < MLP_NPARAMS) ? params[i] : 0.0f;
-    G[i] = 0.0f;
+  float* W1 = sm;                       // [10][64]
+  float* Bs = W1 + MLP_IN * MLP_H;      // b1, b2, b3
+  float* W4 = Bs + 3 * MLP_H;           // [64][2]
+  float* B4 = W4 + MLP_H * MLP_OUT;
+  float* W2 = B4 + 4;
+  float* W3 = W2 + TM;
+  float* H1 = W3 + TM;
+  float* H2 = H1 + TM;
+  float* H3 = H2 + TM;
+  float* S1 = H3 + TM;
+  float* S2 = S1 + TM;
+  float* S3 = S2 + TM;
+  float* X = S3 + TM;                   // [10][TP]
+  float* T = X + MLP_IN * TP;           // targets [2][TS]
+  float* DY = T + 2 * TS;               // output errors [2][TS]
+  float* red = DY + 2 * TS;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int i = tid; i < MLP_IN * MLP_H; i += 256) W1[i] = params[MLP_OFF_W1 + i];
+  for (int i = tid; i < MLP_H; i += 256) {
+    Bs[i] = params[MLP_OFF_B1 + i];
+    Bs[MLP_H + i] = params[MLP_OFF_B2 + i];
+    Bs[2 * MLP_H + i] = params[MLP_OFF_B3 + i];
   }
+  for (int i = tid; i < MLP_H * MLP_OUT; i += 256) W4[i] = params[MLP_OFF_W4 + i];
+  if (tid < MLP_OUT) B4[tid] = params[MLP_OFF_B4 + tid];
+  for (int i = tid; i < MLP_H * MLP_H; i += 256) {
+    W2[(i >> 6) * TP + (i & 63)] = params[MLP_OFF_W2 + i];
+    W3[(i >> 6) * TP + (i & 63)] = params[MLP_OFF_W3 + i];
+  }
+  float g2[4][4] = {}, g3[4][4] = {};   // gradients of W[ty + 16 a][tx + 16 b]
+  float g1[3] = {}, gb = 0.0f, g4 = 0.0f;  // W1 entries tid + 256 q; a bias (tid < 192); W4 and b4 (tid < 130)
   const long long per = (nbatch + gridDim.x - 1) / gridDim.x;
   const long long s0 = (long long)blockIdx.x * per, s1 = min(nbatch, s0 + per);
   float lacc = 0.0f;
   for (long long c0 = s0; c0 < s1; c0 += TS) {
     const int nc = (int)min((long long)TS, s1 - c0);
     __syncthreads();
-    for (int e = tid; e < TS * 12; e += blockDim.x) {
+    for (int e = tid; e < TS * 12; e += 256) {
       const int s = e / 12, col = e % 12;
       float v = 0.0f;
       if (s < nc) {
@@ -127,87 +182,179 @@ __global__ void __launch_bounds__(256, 1) k_mlp_grad(size_t ndata, const float* 
         if (col < MLP_IN) v = (feat[idx * MLP_IN + col] - norm[col]) / norm[MLP_IN + col];
         else v = (targ[idx * MLP_OUT + col - MLP_IN] - norm[2 * MLP_IN + col - MLP_IN]) / norm[2 * MLP_IN + 2 + col - MLP_IN];
       }
-      if (col < MLP_IN) X[s * MLP_IN + col] = v;
-      else T[s * 2 + col - MLP_IN] = v;
+      if (col < MLP_IN) X[col * TP + s] = v;
+      else T[(col - MLP_IN) * TS + s] = v;
     }
     __syncthreads();
-    // layer 1
-    for (int e = tid; e < TS * MLP_H; e += blockDim.x) {
-      const int s = e >> 6, o = e & 63;
-      float z = P[MLP_OFF_B1 + o];
+    auto bias = [&](const float* b, float (&z)[4][4]) {
 #pragma unroll
-      for (int i = 0; i < MLP_IN; i++) z += X[s * MLP_IN + i] * P[MLP_OFF_W1 + i * MLP_H + o];
-      Z1[e] = z;
-      H1[e] = silu_f(z);
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) z[a][q] = b[4 * tx + a];
+    };
+    {
+      float z[4][4];
+      bias(Bs, z);
+      mm_rows<MLP_IN>(W1, MLP_H, X, tx, ty, z);
+      put_layer(H1, S1, tx, ty, z);
     }
     __syncthreads();
-    dense64(H1, P + MLP_OFF_W2, P + MLP_OFF_B2, Z2, H2);
+    {
+      float z[4][4];
+      bias(Bs + MLP_H, z);
+      mm_rows<MLP_H>(W2, TP, H1, tx, ty, z);
+      put_layer(H2, S2, tx, ty, z);
+    }
     __syncthreads();
-    dense64(H2, P + MLP_OFF_W3, P + MLP_OFF_B3, Z3, H3);
+    {
+      float z[4][4];
+      bias(Bs + 2 * MLP_H, z);
+      mm_rows<MLP_H>(W3, TP, H2, tx, ty, z);
+      put_layer(H3, S3, tx, ty, z);
+    }
     __syncthreads();
     // output and its error
     if (tid < TS * 2) {
-      const int s = tid >> 1, o = tid & 1;
-      float y = P[MLP_OFF_B4 + o];
-#pragma unroll 8
-      for (int k = 0; k < MLP_H; k++) y += H3[s * MLP_H + k] * P[MLP_OFF_W4 + k * 2 + o];
+      const int o = tid >> 6, s = tid & 63;
+      float y0 = B4[o], y1 = 0.0f, y2 = 0.0f, y3 = 0.0f;
+#pragma unroll 4
+      for (int k = 0; k < MLP_H; k += 4) {
+        y0 = fmaf(H3[k * TP + s], W4[k * 2 + o], y0);
+        y1 = fmaf(H3[(k + 1) * TP + s], W4[k * 2 + 2 + o], y1);
+        y2 = fmaf(H3[(k + 2) * TP + s], W4[k * 2 + 4 + o], y2);
+        y3 = fmaf(H3[(k + 3) * TP + s], W4[k * 2 + 6 + o], y3);
+      }
       float dy = 0.0f;
       if (s < nc) {
-        const float r = y - T[s * 2 + o];
+        const float r = ((y0 + y1) + (y2 + y3)) - T[tid];
         lacc += 0.5f * r * r;
         dy = r * inv_n;
       }
       DY[tid] = dy;
     }
     __syncthreads();
+    {  // delta of layer 3, in place of its derivatives
+      float acc[4][4];
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+          acc[a][b] = DY[4 * ty + b] * W4[(tx + 16 * a) * 2] + DY[TS + 4 * ty + b] * W4[(tx + 16 * a) * 2 + 1];
+      put_delta(S3, tx, ty, acc);
+    }
+    // W4[k][o] (threads 2k + o) and b4
     if (tid < MLP_H * 2) {
       const int k = tid >> 1, o = tid & 1;
+      float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll 8
+      for (int q = 0; q < TS; q += 2) {  // rotated by k: neighbouring rows in different banks
+        const int s = (q + 2 * k) & (TS - 1);
+        a0 = fmaf(H3[k * TP + s], DY[o * TS + s], a0);
+        a1 = fmaf(H3[k * TP + s + 1], DY[o * TS + s + 1], a1);
+      }
+      g4 += a0 + a1;
+    } else if (tid < MLP_H * 2 + 2) {
       float a = 0.0f;
-      for (int s = 0; s < TS; s++) a += H3[s * MLP_H + k] * DY[s * 2 + o];
-      G[MLP_OFF_W4 + tid] += a;
-    }
-    if (tid < 2) {
-      float a = 0.0f;
-      for (int s = 0; s < TS; s++) a += DY[s * 2 + tid];
-      G[MLP_OFF_B4 + tid] += a;
-    }
-    for (int e = tid; e < TS * MLP_H; e += blockDim.x) {
-      const int s = e >> 6, k = e & 63;
-      const float dh = DY[s * 2] * P[MLP_OFF_W4 + k * 2] + DY[s * 2 + 1] * P[MLP_OFF_W4 + k * 2 + 1];
-      DA[e] = dh * dsilu_f(Z3[e]);
+      for (int s = 0; s < TS; s++) a += DY[(tid - MLP_H * 2) * TS + s];
+      g4 += a;
     }
     __syncthreads();
-    wgrad64(H2, MLP_H, DA, G + MLP_OFF_W3, G + MLP_OFF_B3);
-    bwd64(DA, P + MLP_OFF_W3, Z2, DB);
+    mm_grad(H2, S3, tx, ty, g3);
+    {
+      float acc[4][4] = {};
+      mm_back(W3, S3, tx, ty, acc);
+      put_delta(S2, tx, ty, acc);
+    }
     __syncthreads();
-    wgrad64(H1, MLP_H, DB, G + MLP_OFF_W2, G + MLP_OFF_B2);
-    bwd64(DB, P + MLP_OFF_W2, Z1, DA);
+    mm_grad(H1, S2, tx, ty, g2);
+    {
+      float acc[4][4] = {};
+      mm_back(W2, S2, tx, ty, acc);
+      put_delta(S1, tx, ty, acc);
+    }
     __syncthreads();
-    wgrad64(X, MLP_IN, DA, G + MLP_OFF_W1, G + MLP_OFF_B1);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const int e = tid + 256 * q;
+      if (e < MLP_IN * MLP_H) {
+        const float* x = X + (e >> 6) * TP;
+        const float* d = S1 + (e & 63) * TP;
+        float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll 4
+        for (int s = 0; s < TS; s += 4) {
+          const float4 xv = *reinterpret_cast<const float4*>(x + s), dv = *reinterpret_cast<const float4*>(d + s);
+          a0 = fmaf(xv.x, dv.x, a0);
+          a1 = fmaf(xv.y, dv.y, a1);
+          a0 = fmaf(xv.z, dv.z, a0);
+          a1 = fmaf(xv.w, dv.w, a1);
+        }
+        g1[q] += a0 + a1;
+      }
+    }
+    if (tid < 3 * MLP_H) {  // the biases: sums of the deltas' rows
+      const float* d = (tid < MLP_H ? S1 : tid < 2 * MLP_H ? S2 : S3) + (tid & 63) * TP;
+      float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll 4
+      for (int s = 0; s < TS; s += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(d + s);
+        a0 += v.x + v.z;
+        a1 += v.y + v.w;
+      }
+      gb += a0 + a1;
+    }
   }
-  __syncthreads();
-  for (int i = tid; i < MLP_NPARAMS; i += blockDim.x) partial[(size_t)blockIdx.x * MLP_NPARAMS + i] = G[i];
+  float* out = partial + (size_t)blockIdx.x * MLP_NPARAMS;
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const int e = (ty + 16 * a) * MLP_H + tx + 16 * b;
+      out[MLP_OFF_W2 + e] = g2[a][b];
+      out[MLP_OFF_W3 + e] = g3[a][b];
+    }
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    if (tid + 256 * q < MLP_IN * MLP_H) out[MLP_OFF_W1 + tid + 256 * q] = g1[q];
+  if (tid < 3 * MLP_H) out[(tid < MLP_H ? MLP_OFF_B1 : tid < 2 * MLP_H ? MLP_OFF_B2 : MLP_OFF_B3) + (tid & 63)] = gb;
+  if (tid < MLP_H * 2) out[MLP_OFF_W4 + tid] = g4;
+  else if (tid < MLP_H * 2 + 2) out[MLP_OFF_B4 + tid - MLP_H * 2] = g4;
   // block loss in a fixed order
+  __syncthreads();
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lacc += __shfl_xor_sync(0xffffffffu, lacc, o);
   if ((tid & 31) == 0) red[tid >> 5] = lacc;
   __syncthreads();
   if (tid == 0) {
     double s = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
+    for (int w = 0; w < 8; w++) s += red[w];
     partial_loss[blockIdx.x] = s;
   }
 }
 
-// sum of the partial gradients (block order), then Adam when lr > 0
-__global__ void k_mlp_adam(int nb, const float* __restrict__ partial, const double* __restrict__ partial_loss,
-                           float* __restrict__ params, float* __restrict__ m, float* __restrict__ v, float lr,
-                           float b1, float b2, float eps, float bc1, float bc2, float inv_n,
-                           float* __restrict__ grad_out, double* __restrict__ loss_out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// sum of the partial gradients, then Adam when lr > 0.  A block sums 32 parameters, its eight
+// warps an eighth of the partials each, combined in their order (fixed, so the gradient stays
+// deterministic): 8 us; with one thread per parameter over all partials the 36 blocks' serial
+// loads took 15 us.
+__global__ void __launch_bounds__(256) k_mlp_adam(int nb, const float* __restrict__ partial,
+                                                  const double* __restrict__ partial_loss, float* __restrict__ params,
+                                                  float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2,
+                                                  float eps, float bc1, float bc2, float inv_n,
+                                                  float* __restrict__ grad_out, double* __restrict__ loss_out) {
+  __shared__ float part[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane;
+  float a = 0.0f;
   if (p < MLP_NPARAMS) {
+    const int per = (nb + 7) / 8, q1 = min(nb, (w + 1) * per);
+#pragma unroll 8
+    for (int q = w * per; q < q1; q++) a += partial[(size_t)q * MLP_NPARAMS + p];
+  }
+  part[w][lane] = a;
+  __syncthreads();
+  if (w == 0 && p < MLP_NPARAMS) {
     float g = 0.0f;
-    for (int b = 0; b < nb; b++) g += partial[(size_t)b * MLP_NPARAMS + p];
+#pragma unroll
+    for (int q = 0; q < 8; q++) g += part[q][lane];
     if (grad_out) grad_out[p] = g;
     if (lr > 0.0f) {
       const float mm = b1 * m[p] + (1.0f - b1) * g;
@@ -217,7 +364,7 @@ __global__ void k_mlp_adam(int nb, const float* __restrict__ partial, const doub
       params[p] -= lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
     }
   }
-  if (p == 0 && loss_out) {
+  if (blockIdx.x == 0 && threadIdx.x == 32 && loss_out) {
     double s = 0.0;
     for (int b = 0; b < nb; b++) s += partial_loss[b];
     *loss_out = s * (double)inv_n;
@@ -419,7 +566,7 @@ extern "C" int harm_b200_mlp_loss_grad(harm_ctx* c, size_t n, const float* d_fea
   const float inv_n = (float)(1.0 / (double)n);
   k_mlp_grad<<<nb, 256, TR_SMEM, c->stream>>>(n, d_feat, d_targ, d_norm, d_params, (long long)n, 0ull, 0ll, inv_n,
                                               partial, ploss);
-  k_mlp_adam<<<nblk(MLP_NPARAMS), 256, 0, c->stream>>>(nb, partial, ploss, nullptr, nullptr, nullptr, 0.0f, 0.f, 0.f,
+  k_mlp_adam<<<nblk(MLP_NPARAMS, 32), 256, 0, c->stream>>>(nb, partial, ploss, nullptr, nullptr, nullptr, 0.0f, 0.f, 0.f,
                                                        0.f, 1.f, 1.f, inv_n, d_grad, dloss);
   c->launches += 2;
   CK(cudaGetLastError());
@@ -460,7 +607,7 @@ extern "C" int harm_b200_mlp_train(harm_ctx* c, size_t n, const float* d_feat, c
     p2 *= b2;
     k_mlp_grad<<<nb, 256, TR_SMEM, c->stream>>>(n, d_feat, d_targ, d_norm, d_params, (long long)batch, seed,
                                                 (long long)s, inv_n, partial, ploss);
-    k_mlp_adam<<<nblk(MLP_NPARAMS), 256, 0, c->stream>>>(nb, partial, ploss, d_params, m, v, lr_s, b1, b2, eps,
+    k_mlp_adam<<<nblk(MLP_NPARAMS, 32), 256, 0, c->stream>>>(nb, partial, ploss, d_params, m, v, lr_s, b1, b2, eps,
                                                          (float)(1.0 - p1), (float)(1.0 - p2), inv_n, nullptr,
                                                          d_hist ? d_hist + s : dloss);
     c->launches += 2;
