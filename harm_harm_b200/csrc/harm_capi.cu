@@ -379,8 +379,8 @@ extern "C" int harm_b200_step(harm_ctx* c, int precision, int guess, double* d_P
   return harm_b200_step_n(c, precision, guess, d_P, 1, dt, stats);
 }
 
-// H2D of the state in at most HARM_H2D_SLABS slabs of k-planes (one cudaMemcpyAsync per
-// primitive and slab, each slab followed by an event) on the copy stream, after the context
+// H2D of the state in at most HARM_H2D_SLABS slabs of k-planes (one two-dimensional copy per
+// slab, followed by an event) on the copy stream, after the context
 // stream's earlier work
 // harm_layout: h_P is in HARM's [k][j][i][pl] layout (one copy per slab into d_Paos, converted
 // into d_Pdev on the context stream after the slab's event)
@@ -405,9 +405,9 @@ static int h2d_slabs(harm_ctx* c, const double* h_P, SlabWait* sw, bool harm_lay
     if (harm_layout) {
       CK(cudaMemcpyAsync(c->d_Paos + NPR * off, h_P + NPR * off, NPR * bytes, cudaMemcpyHostToDevice, c->copy_stream));
     } else {
-      for (int p = 0; p < NPR; p++)
-        CK(cudaMemcpyAsync(c->d_Pdev + (size_t)p * c->cells + off, h_P + (size_t)p * c->cells + off, bytes,
-                           cudaMemcpyHostToDevice, c->copy_stream));
+      // the slab of every primitive in one copy: eight rows of a primitive's pitch
+      const size_t pitch = c->cells * sizeof(double);
+      CK(cudaMemcpy2DAsync(c->d_Pdev + off, pitch, h_P + off, pitch, bytes, NPR, cudaMemcpyHostToDevice, c->copy_stream));
     }
     CK(cudaEventRecord(c->slab_ev[s], c->copy_stream));
   }
@@ -470,9 +470,8 @@ static int d2h_slabs(harm_ctx* c, double* h_P) {
   for (int s = 0; s < nslab; s++) {
     const int z0 = s * planes, z1 = (z0 + planes < n3e) ? z0 + planes : n3e;
     const size_t off = (size_t)z0 * c->plane, bytes = (size_t)(z1 - z0) * c->plane * sizeof(double);
-    for (int p = 0; p < NPR; p++)
-      CK(cudaMemcpyAsync(h_P + (size_t)p * c->cells + off, c->d_Pdev + (size_t)p * c->cells + off, bytes,
-                         cudaMemcpyDeviceToHost, c->d2h_stream));
+    const size_t pitch = c->cells * sizeof(double);
+    CK(cudaMemcpy2DAsync(h_P + off, pitch, c->d_Pdev + off, pitch, bytes, NPR, cudaMemcpyDeviceToHost, c->d2h_stream));
     CK(cudaEventRecord(c->d2h_ev[s], c->d2h_stream));
   }
   return 0;
