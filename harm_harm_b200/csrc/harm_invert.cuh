@@ -73,11 +73,17 @@ __device__ __forceinline__ bool coldgrhd(double Qtsq, double D, double& Wp) {
 // residual, derivative and Newton step of the hot (E') or cold (P^2) equation
 __device__ __forceinline__ void inv_func(double Wp, const InvC& c, double& resid, double& jac, double& dx, double& f) {
   if (kFastDiv && !c.cold) {
-    // the same residual and derivative with the divisors' reciprocals formed once
-    const double W = Wp + c.D, iW = frcp(W), X = c.Bsq + W + kSMALL, iX = frcp(X), iX2 = iX * iX, iX3 = iX2 * iX;
-    const double utsq = utsq_calc(W, c);
-    const double gammasq = 1.0 + utsq, gamma = sqrt(gammasq), igsq = frcp(gammasq);
-    const double wmrho0 = (Wp - c.D * utsq * frcp(1.0 + gamma)) * igsq;
+    // The same residual and derivative with four reciprocals instead of the twelve divisions:
+    // utsq with numerator and denominator times W^2 (no quotient inside the quotient), one
+    // reciprocal for W and X together and one for gamma^2 and 1 + gamma (k_invert<1> at
+    // 256x128x64: 248 -> 223 us; compiled for 2 or 4 blocks per SM instead of 3 it is the same).
+    const double W = Wp + c.D, X = c.Bsq + W + kSMALL, W2 = W * W, Y = fma(2.0, W, c.Bsq);
+    const double bq = c.QdotBsq * Y;
+    const double utsq = fma(c.Qtsq, W2, bq) * frcp(fma(fma(c.Bsq + X, W, fma(c.Bsq, c.Bsq, -c.Qtsq)), W2, -bq));
+    const double iWX = frcp(W * X), iX = iWX * W, iX2 = iX * iX, iX3 = iX2 * iX;
+    const double gammasq = 1.0 + utsq, gamma = sqrt(gammasq), gp1 = 1.0 + gamma;
+    const double ig = frcp(gammasq * gp1), igsq = ig * gp1;
+    const double wmrho0 = (Wp - c.D * utsq * (ig * gammasq)) * igsq;
     if (utsq < -0.9 * c.utsq_too_big || utsq != utsq) {
       resid = -kVERYBIG; jac = 0.0; dx = kVERYBIG; f = 0.5 * resid * resid;
       return;
@@ -87,14 +93,10 @@ __device__ __forceinline__ void inv_func(double Wp, const InvC& c, double& resid
     const double BQ = c.Bsq * c.Qtsq - c.QdotBsq;
     double Ep = c.Qdotnp + Wp - pofchi + 0.5 * c.Bsq + 0.5 * BQ * iX2;
     if (pofchi != pofchi || Ep != Ep) Ep = -kVERYBIG;
-    const double Xd = c.Bsq + W, iW3 = iW * iW * iW, iXd = frcp(Xd), iXd3 = iXd * iXd * iXd;
-    const double dvsq = -2.0 * iXd3 * (c.Qtsq + c.QdotBsq * (3.0 * W * Xd + c.Bsq * c.Bsq) * iW3);
-    const double dwmrho0dvsq = (c.D * (gamma * 0.5 - 1.0) - Wp), drho0dvsq = -c.D * gamma * 0.5;
-    const double dpdW = igsq * dpdchi;
-    const double dpdvsq = drho0dvsq * 0.0 + dwmrho0dvsq * dpdchi;
-    const double dpdWp = dpdW + dpdvsq * dvsq;
-    double dE = (1.0 - dpdWp) - BQ * iX3;
-    if (dvsq != dvsq || dpdW != dpdW || dpdvsq != dpdvsq || dpdWp != dpdWp || dE != dE) dE = 0.0;
+    const double dvsq = -2.0 * (iWX * iWX * iWX) * (c.Qtsq * (W2 * W) + c.QdotBsq * (3.0 * W * X + c.Bsq * c.Bsq));
+    const double dpdvsq = (c.D * (gamma * 0.5 - 1.0) - Wp) * dpdchi;
+    double dE = (1.0 - (igsq * dpdchi + dpdvsq * dvsq)) - BQ * iX3;
+    if (dE != dE) dE = 0.0;
     resid = Ep; jac = dE; dx = -Ep * frcp(dE); f = 0.5 * Ep * Ep;
     return;
   }
@@ -136,14 +138,26 @@ __device__ __forceinline__ void validate_Wp(double Wpold, double& Wpnew, const I
     coldgrhd(c.Qtsq, c.D, Wp);
     Wpnew = Wp * 10.0;
   }
-  Wpnew = (fabs(fdiv(Wpnew, c.w1)) > c.gsq_too_big) ? 0.5 * (Wpold + Wpnew) : Wpnew;
+  const bool big = kFastDiv ? fabs(Wpnew) > c.gsq_too_big * fabs(c.w1) : fabs(Wpnew / c.w1) > c.gsq_too_big;
+  Wpnew = big ? 0.5 * (Wpold + Wpnew) : Wpnew;
 }
 
 __device__ __forceinline__ bool ultrarel(double x0, const InvC& c) {
   return (fabs(c.w1) > c.w2) || (fabs(x0) > c.w2);
 }
-__device__ __forceinline__ bool errcheck(double errx, double x0, const InvC& c) {
-  return ultrarel(x0, c) ? (fabs(errx) <= kNEWT_TOL_UR) : (fabs(errx) <= kNEWT_TOL);
+// the error of a step, |step| / scale, against a tolerance (kFastDiv: the step against the
+// tolerance times the scale, without the division)
+struct NewtErr {
+  double step, scale;
+  __device__ __forceinline__ bool within(double tol) const {
+    return kFastDiv ? fabs(step) <= tol * scale : fabs(step / scale) <= tol;
+  }
+  __device__ __forceinline__ bool above(double tol) const {
+    return kFastDiv ? fabs(step) > tol * scale : fabs(step / scale) > tol;
+  }
+};
+__device__ __forceinline__ bool errcheck(const NewtErr& e, double x0, const InvC& c) {
+  return e.within(ultrarel(x0, c) ? kNEWT_TOL_UR : kNEWT_TOL);
 }
 __device__ __forceinline__ int extracheck(double x0, const InvC& c) { return ultrarel(x0, c) ? 4 : 2; }
 
@@ -151,10 +165,12 @@ __device__ __forceinline__ int extracheck(double x0, const InvC& c) { return ult
 // GATED: when the first Newton step from the start is larger than `gate` relative to
 // max(|w0|, |x|) (the scale of the convergence test), the start is judged poor and the
 // iteration stops there, returning 2 with xio unchanged (one iteration counted).
-template <bool GATED = false>
+// CAP: with CAP > 0 an iteration that has not ended after CAP steps stops there and returns 3.
+template <bool GATED = false, int CAP = 0>
 static __device__ int newton(int8_t& flag, double& xio, const InvC& c, int& lntries, int& nstroke, double gate = 0.0) {
   double x = xio, x_old = x, x_older = x;
-  double dx, dx_old = kVERYBIG, resid, jac, f = 1.0, errx = 1.0, damp = 1.0;
+  double dx, dx_old = kVERYBIG, resid, jac, f = 1.0, damp = 1.0;
+  NewtErr errx = {1.0, 1.0};
   int n_iter = 0, diddamp = 0, i_extra = 0, doing_extra = 0;
   bool keep = true;
   while (keep) {
@@ -183,7 +199,7 @@ static __device__ int newton(int8_t& flag, double& xio, const InvC& c, int& lntr
       }
     }
     x += damp * dx;
-    errx = (c.w0 == 0.) ? fabs(dx_old) : fabs(fdiv(dx_old, fmax(fabs(c.w0), fabs(x))));
+    errx = {dx_old, (c.w0 == 0.) ? 1.0 : fmax(fabs(c.w0), fabs(x))};
     validate_Wp(x_old, x, c);
     dx_old = dx;
     if (errcheck(errx, x, c) && doing_extra == 0 && extracheck(x, c) > 0) doing_extra = 1;
@@ -191,6 +207,7 @@ static __device__ int newton(int8_t& flag, double& xio, const InvC& c, int& lntr
     if ((errcheck(errx, x, c) && doing_extra == 0) || (i_extra > extracheck(x, c)) || (n_iter >= (kMAX_NEWT_ITER - 1)))
       keep = false;
     n_iter++;
+    if (CAP > 0 && keep && n_iter >= CAP) return 3;
   }
   if (!isfinite(x) || !isfinite(f) || !isfinite(-2.0 * f)) {
     flag = HARM_UTOPRIMFAILNANRESULT;
@@ -200,7 +217,7 @@ static __device__ int newton(int8_t& flag, double& xio, const InvC& c, int& lntr
   x = x_old;
   xio = x;
   if (errcheck(errx, x, c)) return 0;
-  if (fabs(errx) > kMIN_NEWT_TOL) { flag = HARM_UTOPRIMFAILCONVRET + 4; return 1; }
+  if (errx.above(kMIN_NEWT_TOL)) { flag = HARM_UTOPRIMFAILCONVRET + 4; return 1; }
   return 0;
 }
 
@@ -361,7 +378,8 @@ static __device__ __forceinline__ void jon_prepare(bool cold, const double* Ugf,
 // primitives on success; flag the outcome; wp_out (optional) the final W'.
 // GATED: returns true, with prim and flag untouched, where the first Newton step from Wp
 // exceeds `gate` (newton<true>); otherwise the same operations as without GATED.
-template <bool GATED = false>
+// CAP: the same where the iteration does not end within CAP steps.
+template <bool GATED = false, int CAP = 0>
 static __device__ __forceinline__ bool jon_solve(const JonSetup& s, double Wp, double* prim, int8_t& flag, int& nstroke,
                                                  double* wp_out = nullptr, double gate = 0.0) {
   int lntries = 0;
@@ -376,7 +394,12 @@ static __device__ __forceinline__ bool jon_solve(const JonSetup& s, double Wp, d
     }
     retval += r;
   } else {
-    retval += newton(flag, Wp, s.c, lntries, nstroke);
+    const int r = newton<false, CAP>(flag, Wp, s.c, lntries, nstroke);
+    if (CAP > 0 && r == 3) {
+      flag = flag_in;
+      return true;
+    }
+    retval += r;
   }
   if (wp_out) *wp_out = Wp;
   double pt[5];

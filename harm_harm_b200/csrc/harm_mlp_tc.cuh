@@ -507,7 +507,6 @@ template <int PATH>
 static int launch_invert_gated(harm_ctx* c, const Dims& d, const Phys& ph, const CellTile& ct, const double* pb,
                                double* pf, int8_t* pflag, double* stats) {
   unsigned int* hard = reinterpret_cast<unsigned int*>(c->d_wpg);  // n1*n2*n3 doubles: room for the list
-  CK(cudaMemsetAsync(c->d_nhard, 0, sizeof(unsigned int), c->stream));
   k_invert_gated<PATH><<<cell_grid(d.n1, d.n2, d.n3, ct), 256, 0, c->stream>>>(
       d, ph, c->d_U, pb, pf, pflag, c->d_geom, c->d_aux, c->d_rare, c->d_nrare, stats, ct, c->mlp_gate, hard, c->d_nhard);
   const long long ncell = (long long)d.n1 * d.n2 * d.n3;

@@ -106,7 +106,7 @@ extern "C" int harm_b200_fluxcalc_noalloc(const harm_grid* g, const double* d_ge
   else e = noalloc_dirs<HARM_LIM_MC>(d, ph, d_geom, d_pb, d_F1, d_F2, d_F3, dtmin, st);
   if (e != cudaSuccess) return noalloc_fail(cudaGetErrorString(e));
   long long nc = (long long)(d.n1 + 1) * (d.n2 + 1) * (d.n3 > 1 ? d.n3 + 1 : 1);
-  k_emf<double, double><<<nblk(nc), 256, 0, st>>>(d, d_F1, d_F2, d_F3, d_geom, emf);
+  k_emf<double, double><<<nblk(nc), 256, 0, st>>>(d, d_F1, d_F2, d_F3, d_geom, emf, StepCounters{});
   k_emf_to_flux<double><<<nblk(nc), 256, 0, st>>>(d, emf, d_F1, d_F2, d_F3);
   e = cudaGetLastError();
   if (e != cudaSuccess) return noalloc_fail(cudaGetErrorString(e));

@@ -566,19 +566,80 @@ __global__ void k_finalize_dt(Phys ph, unsigned long long* slots, double* dt, do
 
 // ------------------------------------------------------------------ points inversion
 
-__global__ void k_utoprim_points(size_t n, Phys ph, const double* __restrict__ U, const double* __restrict__ geom,
-                                 double* __restrict__ P, int8_t* __restrict__ pflag, int32_t* __restrict__ iters) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The hot inversion of every point.  A point that it cannot invert, or that has not converged
+// after kPointsCap steps, keeps its guess and a non-zero flag, and k_utoprim_points_rest inverts
+// it from the start, with the cold fallback.  Points of low u/rho and high B^2/rho, whose
+// residual is rounded more coarsely than the test asks, take all 200 steps: 0.2 % of the points
+// then held up 6.5 % of the warps for thirty times the others' length.  Bounded by the latency
+// of the divisions of the Newton chain, so also by the warps that the registers leave: without
+// the fallback four blocks of 128 threads fit an SM instead of one of 256.  300,007 points, two
+// per cent from their roots: 541 us in one kernel, 77 us here and 209 us for the rest (the chain
+// of one point's 200 steps).
+constexpr int kPointsCap = 12;
+__global__ void __launch_bounds__(128, 4) k_utoprim_points(size_t n, Phys ph, const double* __restrict__ U,
+                                                           const double* __restrict__ geom, double* __restrict__ P,
+                                                           int8_t* __restrict__ pflag, int32_t* __restrict__ iters) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   Geo<double> g;
   load_geo<double, double>(geom, n, t, g);
   double u[NPR], pr[NPR];
-  for (int p = 0; p < NPR; p++) { u[p] = U[(size_t)p * n + t]; pr[p] = P[(size_t)p * n + t]; }
+#pragma unroll
+  for (int p = 0; p < NPR; p++) { u[p] = U[(size_t)p * n + t] * g.igdet; pr[p] = P[(size_t)p * n + t]; }
   int8_t flag = 0;
-  int it = utoprimgen(u, g, g.igdet, pr, flag, ph.gam, ph.gammafail, false, 0.0, nullptr);
+  int it = 0;
+  JonSetup s;
+  jon_prepare(false, u, g, pr, ph.gam, ph.gammafail, s);
+  const bool slow = jon_solve<false, kPointsCap>(s, s.Wp_prev, pr, flag, it);
+  pflag[t] = slow ? (int8_t)HARM_UTOPRIMFAILCONVRET : flag;
+  if (slow || flag) return;
+#pragma unroll
   for (int p = 0; p < NPR; p++) P[(size_t)p * n + t] = pr[p];
-  pflag[t] = flag;
   if (iters) iters[t] = it;
+}
+// The flagged points, gathered per block into full warps: a block scans windows of 1024 flags
+// and works off its list whenever it holds a point for every thread, and at the end.
+__global__ void __launch_bounds__(128) k_utoprim_points_rest(size_t n, Phys ph, const double* __restrict__ U,
+                                                             const double* __restrict__ geom, double* __restrict__ P,
+                                                             int8_t* __restrict__ pflag, int32_t* __restrict__ iters) {
+  constexpr int kWin = 1024;
+  __shared__ unsigned int list[128 + kWin];  // offsets from the block's first window, in points
+  __shared__ unsigned int count;
+  const int tid = threadIdx.x;
+  auto work = [&](size_t t) {
+    Geo<double> g;
+    load_geo<double, double>(geom, n, t, g);
+    double u[NPR], pr[NPR];
+#pragma unroll
+    for (int p = 0; p < NPR; p++) { u[p] = U[(size_t)p * n + t]; pr[p] = P[(size_t)p * n + t]; }
+    int8_t flag = 0;
+    const int it = utoprimgen(u, g, g.igdet, pr, flag, ph.gam, ph.gammafail, false, 0.0, nullptr);
+#pragma unroll
+    for (int p = 0; p < NPR; p++) P[(size_t)p * n + t] = pr[p];
+    pflag[t] = flag;
+    if (iters) iters[t] = it;
+  };
+  if (tid == 0) count = 0;
+  __syncthreads();
+  // a window's number is blockIdx.x + k gridDim.x: the list holds k and the place in the window
+  for (unsigned int k = 0;; k++) {
+    const size_t w0 = ((size_t)blockIdx.x + (size_t)k * gridDim.x) * kWin;
+    const bool more = w0 < n;
+    if (more)
+      for (int q = tid; q < kWin; q += 128)
+        if (w0 + q < n && pflag[w0 + q] != 0) list[atomicAdd(&count, 1u)] = k * kWin + q;
+    __syncthreads();
+    while (count >= 128 || (!more && count > 0)) {
+      const unsigned int c = count, take = min(c, 128u);
+      unsigned int e = 0;
+      if (tid < (int)take) e = list[c - take + tid];
+      __syncthreads();
+      if (tid == 0) count = c - take;
+      if (tid < (int)take) work(((size_t)blockIdx.x + (size_t)(e / kWin) * gridDim.x) * kWin + e % kWin);
+      __syncthreads();
+    }
+    if (!more) break;
+  }
 }
 
 // the same with the learned start of the hot inversion (fallback to the plain start inside
@@ -656,7 +717,7 @@ int FP64_FN(hp_fluxes_fp64)(harm_ctx* c, const double* pb, double* F1, double* F
   else if (c->g.lim == HARM_LIM_PARALINE) { int rc = flux_dirs_double<HARM_LIM_PARALINE>(c, d, ph, pb, F1, F2, F3, slots, sw); if (rc) return rc; }
   else { int rc = flux_dirs_double<HARM_LIM_MC>(c, d, ph, pb, F1, F2, F3, slots, sw); if (rc) return rc; }
   long long nc = (long long)(d.n1 + 1) * (d.n2 + 1) * (d.n3 > 1 ? d.n3 + 1 : 1);
-  k_emf<double, double><<<nblk(nc), 256, 0, c->stream>>>(d, F1, F2, F3, c->d_geom, emf);
+  k_emf<double, double><<<nblk(nc), 256, 0, c->stream>>>(d, F1, F2, F3, c->d_geom, emf, {c->d_nrec, c->d_nrare, c->d_nhard});
   c->launches++;
   CK(cudaGetLastError());
   return 0;
@@ -675,7 +736,6 @@ int FP64_FN(hp_update_fp64)(harm_ctx* c, const StepCoef& sc, const double* pi, c
     k_conserved<double><<<cell_grid(d.n1, d.n2, d.n3, cct), 256, 0, c->stream>>>(d, ph, sc, c->d_dt, pi, pb, c->d_F[0], c->d_F[1],
                                                             c->d_F[2], c->d_emf, c->d_geom, c->d_conn, c->d_U, cct);
   }
-  CK(cudaMemsetAsync(c->d_nrare, 0, sizeof(unsigned int), c->stream));
   if (sc.guess == HARM_GUESS_MLP && c->mlp_tc == 4) {
     if (int rc = launch_invert_gated<FP64_PATH>(c, d, ph, ct, pb, pf, pflag, stats)) return rc;
   } else if (sc.guess == HARM_GUESS_MLP && c->mlp_tc == 2) {
@@ -771,7 +831,7 @@ int hp_fixup(harm_ctx* c, double* pf, int8_t* pflag, int finalstep, bool bound_f
   Dims d = dims_of(c->g);
   Phys ph = phys_of(c->g);
   if (bound_flags && hp_bound(c, nullptr, pflag)) return 1;
-  CK(cudaMemsetAsync(c->d_nrec, 0, sizeof(unsigned int), c->stream));
+  if (bound_flags) CK(cudaMemsetAsync(c->d_nrec, 0, sizeof(unsigned int), c->stream));  // else k_emf did
   k_fixup_compute<<<dim3(nblk((long long)d.plane), d.n3), 256, 0, c->stream>>>(
       d, ph, pf, pflag, c->d_geom, (FixRec*)c->d_fixrec, c->d_nrec, c->fix_cap, finalstep, bound_one_launch(d) ? 1 : 0);
   k_fixup_apply<<<4 * c->num_sms, 256, 0, c->stream>>>(d, pf, pflag, (const FixRec*)c->d_fixrec, c->d_nrec, c->fix_cap);
@@ -796,7 +856,10 @@ int hp_points(harm_ctx* c, size_t n, int guess, const double* U, const double* g
     k_utoprim_points_mlp<<<nb, 256, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters,
                                                    reinterpret_cast<const MlpPacked*>(c->d_mlp), c->d_stats);
   } else {
-    k_utoprim_points<<<nblk((long long)n), 256, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters);
+    k_utoprim_points<<<nblk((long long)n, 128), 128, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters);
+    const unsigned int nb = (unsigned int)std::min<size_t>((n + 1023) / 1024, (size_t)2 * c->num_sms);
+    k_utoprim_points_rest<<<nb, 128, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters);
+    c->launches++;
   }
   c->launches++;
   CK(cudaGetLastError());

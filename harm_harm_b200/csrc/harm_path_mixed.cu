@@ -102,7 +102,7 @@ int hp_fluxes_mixed(harm_ctx* c, const double* pb, float* F1, float* F2, float* 
   else if (c->g.lim == HARM_LIM_PARALINE) { int rc = flux_dirs_float<HARM_LIM_PARALINE>(c, d, ph, pb, F1, F2, F3, slots, sw); if (rc) return rc; }
   else { int rc = flux_dirs_float<HARM_LIM_MC>(c, d, ph, pb, F1, F2, F3, slots, sw); if (rc) return rc; }
   long long nc = (long long)(d.n1 + 1) * (d.n2 + 1) * (d.n3 > 1 ? d.n3 + 1 : 1);
-  k_emf<float, float><<<nblk(nc), 256, 0, c->stream>>>(d, F1, F2, F3, c->d_geomf, emf);
+  k_emf<float, float><<<nblk(nc), 256, 0, c->stream>>>(d, F1, F2, F3, c->d_geomf, emf, {c->d_nrec, c->d_nrare, c->d_nhard});
   c->launches++;
   CK(cudaGetLastError());
   return 0;
@@ -114,17 +114,17 @@ int hp_update_mixed(harm_ctx* c, const StepCoef& sc, const double* pi, const dou
   Phys ph = phys_of(c->g);
   const CellTile ct = cell_tile(d.n3, HARM_INVERT_LTK);
   const CellTile cct = (HARM_CONSERVED_LTK > 0 && d.n3 >= 8) ? cell_tile(d.n3, HARM_CONSERVED_LTK) : cell_linear();
+  const bool same = pi == pb;
   if (ct.lti == 4) {  // 16 i x 16 k tiles: the metric and connection staged per block
-    k_conserved_src<float, true><<<cell_grid(d.n1, d.n2, d.n3, ct), 256, 0, c->stream>>>(d, ph, sc, c->d_dt, pi, pb,
-                                                                                        c->d_geom, c->d_conn, c->d_U, ct);
+    const auto k = same ? k_conserved_src<float, true, true> : k_conserved_src<float, true, false>;
+    k<<<cell_grid(d.n1, d.n2, d.n3, ct), 256, 0, c->stream>>>(d, ph, sc, c->d_dt, pi, pb, c->d_geom, c->d_conn, c->d_U, ct);
   } else {
-    k_conserved_src<float, false><<<cell_grid(d.n1, d.n2, d.n3, cct), 256, 0, c->stream>>>(d, ph, sc, c->d_dt, pi, pb,
-                                                                                          c->d_geom, c->d_conn, c->d_U, cct);
+    const auto k = same ? k_conserved_src<float, false, true> : k_conserved_src<float, false, false>;
+    k<<<cell_grid(d.n1, d.n2, d.n3, cct), 256, 0, c->stream>>>(d, ph, sc, c->d_dt, pi, pb, c->d_geom, c->d_conn, c->d_U, cct);
   }
   k_conserved_div<float><<<cell_grid(d.n1, d.n2, d.n3, cct), 256, 0, c->stream>>>(d, ph, sc, c->d_dt, c->d_Ff[0], c->d_Ff[1],
                                                                                  c->d_Ff[2], c->d_emff, c->d_U, cct);
   c->launches++;
-  CK(cudaMemsetAsync(c->d_nrare, 0, sizeof(unsigned int), c->stream));
   if (sc.guess == HARM_GUESS_MLP && c->mlp_tc == 4) {
     if (int rc = launch_invert_gated<1>(c, d, ph, ct, pb, pf, pflag, stats)) return rc;
   } else if (sc.guess == HARM_GUESS_MLP && c->mlp_tc == 2) {

@@ -574,7 +574,7 @@ static inline ReconBox recon_box(const Dims& d, const FaceBox& fb) {
 // Chunks of a march: each costs its first cell's window again (10 loads and 4 cells' weights for
 // WENO5), so a line is cut only as far as the chip needs blocks: eight per SM (two waves; the
 // other limiters, lighter in registers and bound by the latency of their loads, 24), and at least
-// 12 cells.  x1: segments are independent, and a warp takes the next one's loads under its own.
+// 12 cells (the others 4: a march of a small grid is a chain of load latencies).  x1: segments are independent, and a warp takes the next one's loads under its own.
 template <int DIR, int LIM, typename T, typename GT>
 static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const FaceBox& fb, const double* P, const GT* geom,
                                           T* F, unsigned long long* slot, cudaStream_t st, const T* L, T* S, T* E,
@@ -601,7 +601,7 @@ static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const F
     const int groups = (rb.nlines + LN - 1) / LN;
     constexpr int per_sm = (LIM == HARM_LIM_WENO5) ? 8 : 24;
     int chunks = (per_sm * num_sms + groups * NPR - 1) / (groups * NPR);
-    chunks = std::max(1, std::min(chunks, nc / 12));
+    chunks = std::max(1, std::min(chunks, nc / ((LIM == HARM_LIM_WENO5) ? 12 : 4)));
     rb.chunk = (nc + chunks - 1) / chunks;
     chunks = (nc + rb.chunk - 1) / rb.chunk;
     k_recon<DIR, LIM, T><<<dim3(groups, chunks, NPR), 32 * kReconWarps, 0, st>>>(d, rb, P, S, EL, ER);
