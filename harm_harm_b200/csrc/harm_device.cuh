@@ -66,11 +66,36 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
   return fma(fma(-b, q, a), y, q);
 }
 
+// The reciprocals of several values from one division, each corrected by its own remainder (so,
+// as div_by's quotients, the IEEE value but for operands within 1e-15 of a midpoint): b's values
+// normal, and their product.
+__device__ __forceinline__ double recip_fix(double b, double y) { return fma(y, fma(-b, y, 1.0), y); }
+__device__ __forceinline__ void recips(double b0, double b1, double& y0, double& y1) {
+  const double r = 1.0 / (b0 * b1);
+  y0 = recip_fix(b0, r * b1);
+  y1 = recip_fix(b1, r * b0);
+}
+__device__ __forceinline__ void recips(double b0, double b1, double b2, double& y0, double& y1, double& y2) {
+  const double b01 = b0 * b1, r = 1.0 / (b01 * b2), r2 = r * b2;
+  y0 = recip_fix(b0, r2 * b1);
+  y1 = recip_fix(b1, r2 * b0);
+  y2 = recip_fix(b2, r * b01);
+}
+__device__ __forceinline__ void recips(float b0, float b1, float& y0, float& y1) {
+  y0 = __fdividef(1.0f, b0);
+  y1 = __fdividef(1.0f, b1);
+}
+__device__ __forceinline__ void recips(float b0, float b1, float b2, float& y0, float& y1, float& y2) {
+  recips(b0, b1, y0, y1);
+  y2 = __fdividef(1.0f, b2);
+}
+
 // Several values over one denominator: one reciprocal, FP64 with the quotients corrected.
 template <typename T>
 struct WScale {
   T d, y;
   __device__ __forceinline__ explicit WScale(T den) : d(den), y(T(1) / den) {}
+  __device__ __forceinline__ WScale(T den, T rec) : d(den), y(rec) {}
   __device__ __forceinline__ T operator()(T a) const { return div_by(a, d, y); }
 };
 template <>
@@ -83,6 +108,7 @@ struct WScale<float> {
     r = 1.0f / den;  // host pass only parses this; the kernels use the line above
 #endif
   }
+  __device__ __forceinline__ WScale(float, float rec) : r(rec) {}
   __device__ __forceinline__ float operator()(float a) const { return a * r; }
 };
 
@@ -490,11 +516,14 @@ __device__ __forceinline__ void weno5_unopt(const T* u, T* w) {
   const WScale<T> nb(sb + WenoEps<T>::tiny);
 #pragma unroll
   for (int s = 0; s < 3; s++) b[s] = nb(b[s]);
+  {
+    T t[3];
 #pragma unroll
-  for (int s = 0; s < 3; s++) {
-    T t = b[s] + WenoEps<T>::weps;
-    t *= t;
-    w[s] = wdiv<T>(T(1), t);
+    for (int s = 0; s < 3; s++) {
+      t[s] = b[s] + WenoEps<T>::weps;
+      t[s] *= t[s];
+    }
+    recips(t[0], t[1], t[2], w[0], w[1], w[2]);
   }
   T sw = symsum3(w[0], w[1], w[2]);
   const WScale<T> n1(sw + T(0));
@@ -523,11 +552,14 @@ __device__ __forceinline__ void weno3_unopt(const T* u, T* w) {
   const WScale<T> nb(sb + WenoEps<T>::tiny);
   b[0] = nb(b[0]);
   b[1] = nb(b[1]);
+  {
+    T t[2];
 #pragma unroll
-  for (int s = 0; s < 2; s++) {
-    T t = b[s] + WenoEps<T>::weps;
-    t *= t;
-    w[s] = wdiv<T>(T(1), t);
+    for (int s = 0; s < 2; s++) {
+      t[s] = b[s] + WenoEps<T>::weps;
+      t[s] *= t[s];
+    }
+    recips(t[0], t[1], w[0], w[1]);
   }
   T sw = symsum2(w[0], w[1]);
   const WScale<T> n1(sw + T(0));
@@ -564,9 +596,11 @@ __device__ __forceinline__ T smono_indicator(const T* y) {
   minabs = (minabs < m3) ? minabs : m3;
   const T norm = fabs(y[0]) + ((fabs(y[-1]) + fabs(y[1])) + (fabs(y[-2]) + fabs(y[2])));
   const T cutoff = norm * WenoEps<T>::smono + WenoEps<T>::tiny;
-  T v = wdiv<T>(minabs - T(0), cutoff - T(0));
-  v = (T(1) < v) ? T(1) : v;
-  return (T(0) > v) ? T(0) : v;
+  // min(minabs / cutoff, 1): divided out only between 0 and the cutoff
+  if (minabs >= cutoff) return T(1);
+  if (minabs == T(0)) return T(0);
+  const T v = wdiv<T>(minabs, cutoff);
+  return (T(1) < v) ? T(1) : v;
 }
 
 // the cell's WENO5 weights as the ratios and the edges use them: equal weights where the
@@ -589,8 +623,10 @@ __device__ __forceinline__ void weno5_cell_weights(const T* u, T m, T* w) {
 template <typename T>
 __device__ __forceinline__ T weno_frac(const T* w, const T* wm, const T* wp) {
   const T E = WenoEps<T>::eps;
-  T rl = wdiv<T>(w[2] + E, wm[0] + E);
-  T rr = wdiv<T>(w[0] + E, wp[2] + E);
+  const T nl = w[2] + E, dl = wm[0] + E, nr = w[0] + E, dr = wp[2] + E;
+  if (nl < T(1.29) * dl || nr < T(1.29) * dr) return T(0);  // a ratio below the ramp: no division
+  T rl = wdiv<T>(nl, dl);
+  T rr = wdiv<T>(nr, dr);
   T ratio = fmin(rl, rr);
   T f = wdivk<T>(ratio - T(1.3), T(1.6) - T(1.3));
   return fmax(T(0), fmin(f, T(1)));
@@ -674,7 +710,11 @@ __device__ __forceinline__ void weno5_edges(const T* u, const T* w, T f, T m, T&
   T wl[3] = {w[0] * T(1. / 16.), w[1] * T(5. / 8.), w[2] * T(5. / 16.)};
   T wr[3] = {w[0] * T(5. / 16.), w[1] * T(5. / 8.), w[2] * T(1. / 16.)};
   T sl = symsum3(wl[0], wl[1], wl[2]), sr = symsum3(wr[0], wr[1], wr[2]);
-  const WScale<T> nl(sl + WenoEps<T>::tiny), nr(sr + WenoEps<T>::tiny);
+  sl += WenoEps<T>::tiny;
+  sr += WenoEps<T>::tiny;
+  T rsl, rsr;
+  recips(sl, sr, rsl, rsr);
+  const WScale<T> nl(sl, rsl), nr(sr, rsr);
 #pragma unroll
   for (int s = 0; s < 3; s++) {
     wl[s] = nl(wl[s]);
@@ -709,8 +749,10 @@ __device__ __forceinline__ void weno5_edges(const T* u, const T* w, T f, T m, T&
     weno3_unopt<T>(u, w3);
     T l3[2] = {w3[0] * T(1. / 4.), w3[1] * T(3. / 4.)};
     T r3[2] = {w3[0] * T(3. / 4.), w3[1] * T(1. / 4.)};
-    T sl3 = symsum2(l3[0], l3[1]), sr3 = symsum2(r3[0], r3[1]);
-    const WScale<T> nl3(sl3 + WenoEps<T>::tiny), nr3(sr3 + WenoEps<T>::tiny);
+    const T sl3 = symsum2(l3[0], l3[1]) + WenoEps<T>::tiny, sr3 = symsum2(r3[0], r3[1]) + WenoEps<T>::tiny;
+    T yl3, yr3;
+    recips(sl3, sr3, yl3, yr3);
+    const WScale<T> nl3(sl3, yl3), nr3(sr3, yr3);
 #pragma unroll
     for (int s = 0; s < 2; s++) {
       l3[s] = nl3(l3[s]);

@@ -212,7 +212,10 @@ constexpr int kReconWarps = 4;
 #endif
 // steps unrolled: FP64's step is long, and an unrolled loop of it misses the instruction cache
 template <typename T>
-constexpr int kReconUnroll = sizeof(T) == 4 ? 4 : 1;
+#ifndef HARM_RECON_UNROLL
+#define HARM_RECON_UNROLL 4
+#endif
+constexpr int kReconUnroll = sizeof(T) == 4 ? HARM_RECON_UNROLL : 1;
 
 template <int DIR, int LIM, typename T, int TU = HARM_TU>
 __global__ void __launch_bounds__(32 * kReconWarps, HARM_RECON_MINB) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
