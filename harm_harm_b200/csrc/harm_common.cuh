@@ -1099,24 +1099,29 @@ __global__ void __launch_bounds__(256, HARM_CONSERVED_SRC_BLOCKS) k_conserved_sr
   __shared__ double s_tab[STAGE ? kStageF * kStageTI : 1];
   int i, j, k;
   const bool ok = tile_cell(d.n1, d.n2, d.n3, ct, blockIdx.x, blockIdx.y, blockIdx.z, i, j, k);
+  // the states' loads fly under the staging of the tables and its barrier
+  int ii = min(i, d.n1 - 1) + d.ng, jj = min(j, d.n2 - 1) + d.ng, kk = min(k, d.n3 - 1) + d.ng3;
+  const size_t id = cidx(d, ii, jj, kk), c2 = (size_t)jj * d.n1e + ii;
+  double pr[NPR], pn[SAME ? 1 : NPR];
+#pragma unroll
+  for (int p = 0; p < NPR; p++) pr[p] = pi[(size_t)p * d.cells + id];
+  if constexpr (!SAME) {
+#pragma unroll
+    for (int p = 0; p < NPR; p++) pn[p] = pb[(size_t)p * d.cells + id];
+  }
   stage_conn_geom<STAGE>(d, geom, conn, s_tab);
   if (!ok) return;
-  int ii = i + d.ng, jj = j + d.ng, kk = k + d.ng3;
-  const size_t id = cidx(d, ii, jj, kk), c2 = (size_t)jj * d.n1e + ii;
   const int il = i & (kStageTI - 1);
   Geo<double> g;
   if constexpr (STAGE) load_geo<double, double, false>(s_tab + 64 * kStageTI, kStageTI, il, g);
   else load_geo<double, double>(geom, d.plane, c2, g);
-  double pr[NPR];
-#pragma unroll
-  for (int p = 0; p < NPR; p++) pr[p] = pi[(size_t)p * d.cells + id];
   State<double> q;
   get_state<double>(pr, g, ph.gam, q);
   double Ui[NPR];
   primtoflux<double>(pr, q, 0, g, g.gdet, Ui);
   if constexpr (!SAME) {
 #pragma unroll
-    for (int p = 0; p < NPR; p++) pr[p] = pb[(size_t)p * d.cells + id];
+    for (int p = 0; p < NPR; p++) pr[p] = pn[p];
     get_state<double>(pr, g, ph.gam, q);
   }
   double dUg[NPR];

@@ -30,30 +30,8 @@ constexpr double kBIG = 1.e100;
 constexpr double kSQRTMIN = 1.4916681462400413e-154;
 constexpr double kSMALL = 1e-300;
 
-// Division inside the Newton iteration.  By default IEEE FP64 division (the operations of the
-// C restatement, so the FP64 path matches it to round-off).  A translation unit that defines
-// HARM_INVERT_FAST_DIV before including this header (the mixed-precision path) gets the
-// reciprocal from the hardware FP64 approximation refined by two Newton-Raphson steps
-// (r <- r + r (1 - b r), quadratic convergence from the approximation's relative error), a
-// multiply, and reciprocals shared between the divisions of one residual evaluation: within
-// an ulp or two of the IEEE quotients for normal operands, with fewer FP64 instructions.
-#ifdef HARM_INVERT_FAST_DIV
-constexpr bool kFastDiv = true;
-__device__ __forceinline__ double frcp(double b) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-  double e = fma(-b, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-b, r, 1.0);
-  return fma(r, e, r);
-}
-__device__ __forceinline__ double fdiv(double a, double b) { return a * frcp(b); }
-#else
-constexpr bool kFastDiv = false;
-__device__ __forceinline__ double frcp(double b) { return 1.0 / b; }
-__device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
-#endif
-
+// The divisions are fdiv and frcp (harm_device.cuh): IEEE, or on the mixed path the refined
+// hardware reciprocal, shared between the divisions of one residual evaluation.
 __device__ __forceinline__ double utsq_calc(double W, const InvC& c) {
   double SoW = fdiv(c.QdotB, W);
   double top = c.Qtsq + (c.Bsq + 2.0 * W) * SoW * SoW;
@@ -252,7 +230,7 @@ static __device__ __forceinline__ void inv_invariants(const double* U, const Geo
   c.QdotB = Qcov[1] * Bcon[1] + Qcov[2] * Bcon[2] + Qcov[3] * Bcon[3];
   c.QdotBsq = c.QdotB * c.QdotB;
   double alpha = g.alpha, alphasq = alpha * alpha;
-  double Dfactor = (-g.gcovpert_tt + alphasq * g.betasqoalphasq) / (alphasq + alpha);
+  double Dfactor = fdiv(-g.gcovpert_tt + alphasq * g.betasqoalphasq, alphasq + alpha);
   c.Qdotnp = Qconp[0] * ncov[0] + c.D * Dfactor;
 }
 
@@ -267,14 +245,14 @@ static __device__ int inv_setup(const double* U, const Geo<double>& g, const dou
     for (int j = 1; j < 4; j++) utsq += g.gcov[sym(i, j)] * prim[HARM_U1 + i - 1] * prim[HARM_U1 + j - 1];
   if ((utsq < 0.) && (fabs(utsq) < fabs(-0.9 * c.utsq_too_big))) utsq = 0.0;
   if (!(utsq >= 0. && utsq < c.utsq_too_big)) utsq = 0.0;
-  double gammasq = 1. + utsq, gamma = sqrt(gammasq), rho0 = c.D / gamma, u = prim[HARM_UU];
+  double gammasq = 1. + utsq, gamma = sqrt(gammasq), rho0 = fdiv(c.D, gamma), u = prim[HARM_UU];
   double p = (c.gam - 1.) * u;
   double bc[4] = {0.0, prim[HARM_B1], prim[HARM_B2], prim[HARM_B3]}, bcv[4];
   lower(bc, g, bcv);
   double bsq = bc[1] * bcv[1] + bc[2] * bcv[2] + bc[3] * bcv[3];
-  bsq *= (g.alpha * g.alpha) / gammasq;
-  Wp_last = c.D * utsq / (1.0 + gamma) + (u + p) * gammasq;
-  double Wpabs = fabs(c.D * utsq) / (1.0 + fabs(gamma)) + (fabs(u) + fabs(p)) * fabs(gammasq) + kSQRTMIN;
+  bsq *= fdiv(g.alpha * g.alpha, gammasq);
+  Wp_last = fdiv(c.D * utsq, 1.0 + gamma) + (u + p) * gammasq;
+  double Wpabs = fdiv(fabs(c.D * utsq), 1.0 + fabs(gamma)) + (fabs(u) + fabs(p)) * fabs(gammasq) + kSQRTMIN;
   double etaabs = fabs(rho0) + (fabs(u) + fabs(p) + fabs(bsq));
   c.w2 = 1e2 * fabs(rho0);
   if (gammasq * etaabs >= c.w2) {
@@ -314,11 +292,11 @@ static __device__ int inv_verify_guess(double& Wp_last, const InvC& c, int8_t& f
 static __device__ int inv_finish(double Wp, const InvC& c, const double* Qtcon, const double* Bcon, double* prim, int8_t& flag) {
   if (Wp == kBIG) flag = HARM_UTOPRIMFAILCONVRET + 1;
   else if (Wp <= -(c.D)) flag = HARM_UTOPRIMFAILCONVRET + 1;
-  else if (Wp / c.w1 > c.gsq_too_big) flag = HARM_UTOPRIMFAILCONVW;
+  else if (fdiv(Wp, c.w1) > c.gsq_too_big) flag = HARM_UTOPRIMFAILCONVW;
   double W = Wp + c.D;
   double utsq = utsq_calc(W, c), gammasq = 1.0 + utsq, gamma = sqrt(gammasq);
-  double wmrho0 = (Wp - c.D * utsq / (1.0 + gamma)) / gammasq;
-  double rho0 = c.D / gamma;
+  double wmrho0 = fdiv(Wp - fdiv(c.D * utsq, 1.0 + gamma), gammasq);
+  double rho0 = fdiv(c.D, gamma);
   double p = ((c.gam - 1.0) / c.gam) * wmrho0, u = wmrho0 - p;
   if ((rho0 <= 0.) || ((p < 0.) && !c.cold)) {
     if ((rho0 <= 0.) && (p >= 0.)) flag = HARM_UTOPRIMFAILRHONEG;
@@ -329,7 +307,7 @@ static __device__ int inv_finish(double Wp, const InvC& c, const double* Qtcon, 
   out[0] = rho0;
   out[1] = c.cold ? 0.0 : u;
 #pragma unroll
-  for (int i = 1; i < 4; i++) out[1 + i] = gamma / (W + c.Bsq) * (Qtcon[i] + c.QdotB * Bcon[i] / W);
+  for (int i = 1; i < 4; i++) out[1 + i] = fdiv(gamma, W + c.Bsq) * (Qtcon[i] + fdiv(c.QdotB * Bcon[i], W));
   bool nan = false;
 #pragma unroll
   for (int i = 0; i < 5; i++) nan |= !isfinite(out[i]);

@@ -207,18 +207,13 @@ struct ReconLine<HARM_LIM_WENO5, V> {
 // Warps per block and blocks per SM the marching kernel is compiled for: the window of FP32
 // WENO5 (56 registers beside its temporaries) and FP64's fit 128 registers without spills.
 constexpr int kReconWarps = 4;
-#ifndef HARM_RECON_MINB
-#define HARM_RECON_MINB 4
-#endif
-// steps unrolled: FP64's step is long, and an unrolled loop of it misses the instruction cache
+// steps unrolled: an unrolled loop saves moves and misses the instruction cache (FP32 WENO5 at
+// 256x128x64, full step: 1 step 2861 us, 2 2821, 4 2867, 8 3320; FP64's step is long)
 template <typename T>
-#ifndef HARM_RECON_UNROLL
-#define HARM_RECON_UNROLL 4
-#endif
-constexpr int kReconUnroll = sizeof(T) == 4 ? HARM_RECON_UNROLL : 1;
+constexpr int kReconUnroll = sizeof(T) == 4 ? 2 : 1;
 
 template <int DIR, int LIM, typename T, int TU = HARM_TU>
-__global__ void __launch_bounds__(32 * kReconWarps, HARM_RECON_MINB) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
+__global__ void __launch_bounds__(32 * kReconWarps, 4) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
                                                                              const T* __restrict__ S, T* __restrict__ EL,
                                                                              T* __restrict__ ER) {
   static_assert(DIR != 1, "x1: k_recon_x1");
