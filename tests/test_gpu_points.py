@@ -1,0 +1,50 @@
+"""Utoprimgen over points at the sizes where the split into a common kernel and one for the rest can
+go wrong: one point, the edges of a block of 128 and of a window of 1024 flags, and sets dense in
+points that do not converge within the common kernel's steps (low u/rho at high B^2/rho, whose
+residual rounds more coarsely than the test) or that the hot inversion cannot invert.  FP64 against
+the oracle point by point: the same flags, primitives to 1e-9 of each point's largest (W' of the
+slow points is only defined to 1e-12 of D, 1e-6 of itself and of u)."""
+import numpy as np
+import pytest
+
+from helpers import make_torus
+from harm_harm_b200 import Harm
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(g, geom, n, kind, seed):
+    rng = np.random.default_rng(seed)
+    cell = rng.integers(geom.shape[2] * geom.shape[3], size=n)
+    rec = np.ascontiguousarray(geom[0].reshape(28, -1)[:, cell])
+    P = np.zeros((8, n))
+    P[0] = 10.0 ** rng.uniform(-4, 0, n)
+    P[1] = P[0] * 10.0 ** (rng.uniform(-3, 0, n) if kind != "slow" else rng.uniform(-6, -5, n))
+    P[2:5] = rng.normal(0.0, 0.05, (3, n)) / np.sqrt(rec[[4, 7, 9]])
+    P[5:] = rng.normal(0.0, 1.0, (3, n)) * np.sqrt(P[0] * (10.0 if kind == "slow" else 0.01)) / np.sqrt(rec[[4, 7, 9]])
+    U = np.stack([O.primtoU_point(np.ascontiguousarray(rec[:, k]), P[:, k]) for k in range(n)], axis=1)
+    if kind == "failing":
+        bad = rng.random(n) < 0.5
+        U[1, bad] *= -3.0  # no root: the hot inversion fails, the cold one may take over
+    return U, rec, P * rng.uniform(0.99, 1.01, P.shape)
+
+
+@pytest.mark.parametrize("n,kind", [(1, "plain"), (127, "plain"), (129, "slow"), (1025, "slow"), (2300, "failing"), (1, "failing")])
+def test_points(cuda, n, kind):
+    g, geom, conn, aux, _ = make_torus(16, 16, 1)
+    U, rec, guess = _points(g, geom, n, kind, seed=n)
+    dev = Harm(g, geom, conn, aux)
+    Pd = cuda.from_numpy(guess.copy()).cuda()
+    flag = cuda.zeros(n, dtype=cuda.int8, device="cuda")
+    it = cuda.zeros(n, dtype=cuda.int32, device="cuda")
+    dev.Utoprimgen(cuda.from_numpy(U).cuda(), cuda.from_numpy(rec).cuda(), Pd, flag, it)
+    P, flag, it = Pd.cpu().numpy(), flag.cpu().numpy(), it.cpu().numpy()
+    for k in range(n):
+        pr, fl, _ = O.utoprimgen_point(g, np.ascontiguousarray(rec[:, k]), U[:, k], guess[:, k])
+        assert flag[k] == fl, (k, flag[k], fl)
+        assert np.abs(P[:, k] - pr).max() <= 1e-9 * np.abs(pr).max(), k
+    if kind == "slow":
+        assert (it > 12).any()
+    if kind == "failing" and n > 1:
+        assert (flag != 0).any()
