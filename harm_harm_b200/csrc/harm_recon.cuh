@@ -204,16 +204,20 @@ struct ReconLine<HARM_LIM_WENO5, V> {
   }
 };
 
-// Warps per block and blocks per SM the marching kernel is compiled for: the window of FP32
-// WENO5 (56 registers beside its temporaries) and FP64's fit 128 registers without spills.
+// Warps per block and blocks per SM the marching kernel is compiled for.  FP32: 4 (the window of
+// WENO5, 56 registers beside its temporaries, fits 128 without spills; 5 spill, and a full step at
+// 256x128x64 takes 3095 us instead of 2867; 3 are the same).  FP64: 5 (102 registers with a few
+// spills, 25 % more warps to hide the divisions: 330 us a direction at 192x96x64 against 350 at 4).
 constexpr int kReconWarps = 4;
+template <typename T>
+constexpr int kReconBlocks = sizeof(T) == 4 ? 4 : 5;
 // steps unrolled: an unrolled loop saves moves and misses the instruction cache (FP32 WENO5 at
 // 256x128x64, full step: 1 step 2861 us, 2 2821, 4 2867, 8 3320; FP64's step is long)
 template <typename T>
 constexpr int kReconUnroll = sizeof(T) == 4 ? 2 : 1;
 
 template <int DIR, int LIM, typename T, int TU = HARM_TU>
-__global__ void __launch_bounds__(32 * kReconWarps, 4) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
+__global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
                                                                              const T* __restrict__ S, T* __restrict__ EL,
                                                                              T* __restrict__ ER) {
   static_assert(DIR != 1, "x1: k_recon_x1");
@@ -314,6 +318,10 @@ struct ReconRow {
   static constexpr int E = 64 - 2 * M;                        // edge cells per segment
 };
 constexpr int kRowWarps = 8;
+// FP64: 3 blocks per SM (80 registers; left to itself 94 and 2 blocks, 330 us against 299 at
+// 192x96x64)
+template <typename T>
+constexpr int kRowBlocks = sizeof(T) == 4 ? 1 : 3;
 template <typename T>
 struct ReconRowSmem {
   T u[68];
@@ -321,7 +329,7 @@ struct ReconRowSmem {
 };
 
 template <int LIM, typename T, int TU = HARM_TU>
-__global__ void __launch_bounds__(32 * kRowWarps) k_recon_x1(Dims d, ReconBox rb, FastDiv dseg,
+__global__ void __launch_bounds__(32 * kRowWarps, kRowBlocks<T>) k_recon_x1(Dims d, ReconBox rb, FastDiv dseg,
                                                              const double* __restrict__ P,
                                                              const T* __restrict__ S, T* __restrict__ EL,
                                                              T* __restrict__ ER) {
@@ -483,8 +491,9 @@ __global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const d
 
 // One thread per (i, j) of the face box and kb consecutive k: the face's metric is loaded once
 // for them (FP32; x3-independent).  Bounded by the FMA pipe in FP32, by the FP64 pipe in FP64.
-// Registers: FP32 128 (4 blocks of 128 threads per SM: the next face's states are loaded under
-// this one's physics), FP64 168 (3 blocks; at 128 it spills).
+// Blocks of 128 threads per SM, in whose registers the next face's states are loaded under this
+// one's physics: FP32 4 (5, with spills, gain 2 us of 51 at 256x128x64 and lose as much on small
+// grids), FP64 3 (2: 160 us at 192x96x64, 3: 132, 4 with spills: 126, and slower on small grids).
 template <typename T>
 constexpr int kFaceBlocks = sizeof(T) == 4 ? 4 : 3;
 constexpr int kFaceThreads = 128;
