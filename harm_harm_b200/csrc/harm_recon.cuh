@@ -492,10 +492,10 @@ __global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const d
 // One thread per (i, j) of the face box and kb consecutive k: the face's metric is loaded once
 // for them (FP32; x3-independent).  Bounded by the FMA pipe in FP32, by the FP64 pipe in FP64.
 // Blocks of 128 threads per SM, in whose registers the next face's states are loaded under this
-// one's physics: FP32 4 (5, with spills, gain 2 us of 51 at 256x128x64 and lose as much on small
-// grids), FP64 3 (2: 160 us at 192x96x64, 3: 132, 4 with spills: 126, and slower on small grids).
+// one's physics: FP32 5 (49 us at 256x128x64; 4: 51, 3: 55), FP64 4 (126 us at 192x96x64, with
+// spills; 3: 132, 2: 160).
 template <typename T>
-constexpr int kFaceBlocks = sizeof(T) == 4 ? 4 : 3;
+constexpr int kFaceBlocks = sizeof(T) == 4 ? 5 : 4;
 constexpr int kFaceThreads = 128;
 template <int DIR, typename T, typename GT, int TU = HARM_TU>
 __global__ void __launch_bounds__(kFaceThreads, kFaceBlocks<T>) k_face(Dims d, Phys ph, FaceBox fb, const T* __restrict__ EL,
