@@ -78,10 +78,10 @@ def flux_bytes_per_cell(n3: int, precision: int, lim: str = "weno5") -> float:
     return b
 
 
-# DRAM traffic of the flux stage (k_cellprep and three k_fluxt launches; ncu dram__bytes_read.sum +
-# dram__bytes_write.sum) per active cell, measured on the 192x96x64 torus and scaled to a
-# workload by its cell count
-FLUX_TRAFFIC_PER_CELL = {("weno5", "mixed"): 449.0}
+# DRAM traffic of the flux stage (three reconstruction and three face launches; ncu
+# dram__bytes_read.sum + dram__bytes_write.sum: 1447 MB) per active cell, measured on the 256x128x64
+# torus and scaled to a workload by its cell count
+FLUX_TRAFFIC_PER_CELL = {("weno5", "mixed"): 689.8}
 
 
 def clock_sampler(stop: threading.Event, out: list, dev: int):
@@ -551,16 +551,18 @@ def run_ours(args, ws, rank, local):
             "mlp_gate": float(os.environ.get("HARM_B200_MLP_GATE", "0.02")),
             "learned_guess": mlp_info,
             "stage_ms": stages,
-            "roofline": {"bound": "hbm", "kernel": "k_fluxt (WENO5/PPM/MC reconstruction + HLL, 3 directions)",
+            "roofline": {"bound": "hbm", "kernel": "k_recon_x1 + k_recon (WENO5/PPM/MC reconstruction) + k_face (HLL), "
+                                                     "3 directions",
                          "achieved": ach_flux, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": ach_flux / peaks["hbm_gbs"], "peak_src": peaks["src"],
                          "traffic": (FLUX_TRAFFIC_PER_CELL[(LIMNAME[lim], args.precision)] * zones
                                      if (LIMNAME[lim], args.precision) in FLUX_TRAFFIC_PER_CELL else None),
-                         "unit_of_launch": "one flux stage (the WENO5 cell pass k_cellprep and three k_fluxt "
-                                           "launches, all directions)",
+                         "unit_of_launch": "one flux stage (the WENO5 cell pass k_cellprep and, in each "
+                                           "direction, one reconstruction and one face launch)",
                          "algorithmic_bytes_per_cell": flux_bytes_per_cell(n3, prec, LIMNAME[lim]),
-                         "limiter": "instruction issue, not HBM: 75 % of issue slots, ALU 56 %, FMA 52 %, "
-                                    "DRAM 6 % (ncu, WENO5 FP32 tile kernel, 192x96x64)"},
+                         "limiter": "instruction issue, not HBM, in the reconstruction (65-73 % of issue "
+                                    "slots, FMA 53-55 %, DRAM 22-23 %); loads and issue together in the faces "
+                                    "(56 %, FMA 48 %, DRAM 45 %) (ncu, FP32 WENO5, 256x128x64)"},
             "roofline_update_invert": {"bound": "hbm",
                                        "kernel": "conserved update + learned start + k_invert + k_invert_rare",
                                        "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
