@@ -629,16 +629,21 @@ __global__ void __launch_bounds__(128) k_utoprim_points_rest(size_t n, Phys ph, 
       for (int q = tid; q < kWin; q += 128)
         if (w0 + q < n && pflag[w0 + q] != 0) list[atomicAdd(&count, 1u)] = k * kWin + q;
     __syncthreads();
-    while (count >= 128 || (!more && count > 0)) {
-      const unsigned int c = count, take = min(c, 128u);
-      unsigned int e = 0;
-      if (tid < (int)take) e = list[c - take + tid];
-      __syncthreads();
-      if (tid == 0) count = c - take;
-      if (tid < (int)take) work(((size_t)blockIdx.x + (size_t)(e / kWin) * gridDim.x) * kWin + e % kWin);
-      __syncthreads();
+    // every thread's own copy of the length: a warp that is done here must not change what
+    // another one still decides by, so the next window's entries wait for the barrier below
+    unsigned int c = count;
+    while (c >= 128 || (!more && c > 0)) {
+      const unsigned int take = min(c, 128u);
+      c -= take;
+      if (tid < (int)take) {
+        const unsigned int e = list[c + tid];
+        work(((size_t)blockIdx.x + (size_t)(e / kWin) * gridDim.x) * kWin + e % kWin);
+      }
     }
+    __syncthreads();
     if (!more) break;
+    if (tid == 0) count = c;
+    __syncthreads();
   }
 }
 

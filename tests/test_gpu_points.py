@@ -1,6 +1,6 @@
 """Utoprimgen over points at the sizes where the split into a common kernel and one for the rest can
-go wrong: one point, the edges of a block of 128 and of a window of 1024 flags, and sets dense in
-points that do not converge within the common kernel's steps (low u/rho at high B^2/rho, whose
+go wrong: one point, the edges of a block of 128 and of a window of 1024 flags, several windows per
+block, and sets dense in points that do not converge within the common kernel's steps (low u/rho at high B^2/rho, whose
 residual rounds more coarsely than the test) or that the hot inversion cannot invert.  FP64 against
 the oracle point by point: the same flags, primitives to 1e-9 of each point's largest (W' of the
 slow points is only defined to 1e-12 of D, 1e-6 of itself and of u)."""
@@ -48,3 +48,32 @@ def test_points(cuda, n, kind):
         assert (it > 12).any()
     if kind == "failing" and n > 1:
         assert (flag != 0).any()
+
+
+@pytest.mark.parametrize("dense", [0.02, 0.7])
+def test_points_over_several_windows(cuda, dense):
+    """More points than two windows per block: what a block's list carries from one window into the
+    next, full passes with windows still to come (dense) and lists that fill over all of them
+    (sparse).  Slow, failing and plain points, checked against the oracle once, at random places: the
+    kernels' operations on a point do not depend on its place, so its copies are equal bit for bit."""
+    g, geom, conn, aux, _ = make_torus(16, 16, 1)
+    sets = [_points(g, geom, m, kind, seed=m) for m, kind in ((700, "plain"), (150, "slow"), (400, "failing"))]
+    U, rec, guess = (np.concatenate([s[q] for s in sets], axis=1) for q in range(3))
+    ref = [O.utoprimgen_point(g, np.ascontiguousarray(rec[:, k]), U[:, k], guess[:, k]) for k in range(U.shape[1])]
+    Pr, fr, ir = (np.array([r[q] for r in ref]) for q in range(3))
+    n = 2 * 2 * cuda.cuda.get_device_properties(0).multi_processor_count * 1024 + 517
+    rng = np.random.default_rng(11)
+    at = np.where(rng.random(n) < dense, rng.integers(700, U.shape[1], n), rng.integers(0, 700, n))
+    idx = cuda.from_numpy(at).cuda()
+    dev = Harm(g, geom, conn, aux)
+    Ud, recd, Pd = (cuda.from_numpy(a).cuda()[:, idx].contiguous() for a in (U, rec, guess))
+    flag = cuda.full((n,), 77, dtype=cuda.int8, device="cuda")
+    it = cuda.zeros(n, dtype=cuda.int32, device="cuda")
+    dev.Utoprimgen(Ud, recd, Pd, flag, it)
+    P, flag, it = Pd.cpu().numpy(), flag.cpu().numpy(), it.cpu().numpy()
+    assert (flag == fr[at]).all()
+    assert (np.abs(P - Pr[at].T).max(axis=0) <= 1e-9 * np.abs(Pr[at]).max(axis=1)).all()
+    first = np.zeros(U.shape[1], dtype=np.int64)
+    first[at[::-1]] = np.arange(n)[::-1]
+    assert np.array_equal(P, P[:, first[at]]) and np.array_equal(it, it[first[at]])
+    assert (it[flag == 0] > 12).any() and (fr != 0).any()
