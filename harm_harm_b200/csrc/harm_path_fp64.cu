@@ -464,10 +464,19 @@ __global__ void __launch_bounds__(256) k_fixup_compute(Dims d, Phys ph, const do
   for (int p = 0; p < 5; p++) lastmin[p] = 1E50;
   int numavg0 = 0, numavg1 = 0;
   const double ref = P[(size_t)HARM_UU * d.cells + id];
+  // cells with a neighbour whose flag this launch writes
+  const bool edge = ghosts && (i == d.n1 - 1 || j == 0 || j == d.n2 - 1);
   for (int qq = 0; qq < npairs; qq++) {
     int di = (qq % rnx) - s1, dj = ((qq % (rnx * rny)) / rnx) - s2, dk = (qq / (rnx * rny)) - s3;
     size_t a = cidx(d, ii + di, jj + dj, kk + dk), b = cidx(d, ii - di, jj - dj, kk - dk);
-    int thisok = flag_at(d, flag, ii + di, jj + dj, kk + dk) <= 0, thatok = flag_at(d, flag, ii - di, jj - dj, kk - dk) <= 0;
+    int thisok, thatok;
+    if (edge) {
+      thisok = flag_at(d, flag, ii + di, jj + dj, kk + dk) <= 0;
+      thatok = flag_at(d, flag, ii - di, jj - dj, kk - dk) <= 0;
+    } else {
+      thisok = flag[a] <= 0;
+      thatok = flag[b] <= 0;
+    }
     numavg0 += thisok + thatok;
     for (int p = startpl; p <= endpl; p++) {
       double fa = P[(size_t)p * d.cells + a], fb = P[(size_t)p * d.cells + b];
@@ -597,6 +606,22 @@ __global__ void __launch_bounds__(128, 4) k_utoprim_points(size_t n, Phys ph, co
   for (int p = 0; p < NPR; p++) P[(size_t)p * n + t] = pr[p];
   if (iters) iters[t] = it;
 }
+// Utoprimgen of point t, cold fallback included
+__device__ __forceinline__ void utoprim_point(size_t n, size_t t, const Phys& ph, const double* __restrict__ U,
+                                              const double* __restrict__ geom, double* __restrict__ P,
+                                              int8_t* __restrict__ pflag, int32_t* __restrict__ iters) {
+  Geo<double> g;
+  load_geo<double, double>(geom, n, t, g);
+  double u[NPR], pr[NPR];
+#pragma unroll
+  for (int p = 0; p < NPR; p++) { u[p] = U[(size_t)p * n + t]; pr[p] = P[(size_t)p * n + t]; }
+  int8_t flag = 0;
+  const int it = utoprimgen(u, g, g.igdet, pr, flag, ph.gam, ph.gammafail, false, 0.0, nullptr);
+#pragma unroll
+  for (int p = 0; p < NPR; p++) P[(size_t)p * n + t] = pr[p];
+  pflag[t] = flag;
+  if (iters) iters[t] = it;
+}
 // The flagged points, gathered per block into full warps: a block scans windows of 1024 flags
 // and works off its list whenever it holds a point for every thread, and at the end.
 __global__ void __launch_bounds__(128) k_utoprim_points_rest(size_t n, Phys ph, const double* __restrict__ U,
@@ -606,19 +631,6 @@ __global__ void __launch_bounds__(128) k_utoprim_points_rest(size_t n, Phys ph, 
   __shared__ unsigned int list[128 + kWin];  // offsets from the block's first window, in points
   __shared__ unsigned int count;
   const int tid = threadIdx.x;
-  auto work = [&](size_t t) {
-    Geo<double> g;
-    load_geo<double, double>(geom, n, t, g);
-    double u[NPR], pr[NPR];
-#pragma unroll
-    for (int p = 0; p < NPR; p++) { u[p] = U[(size_t)p * n + t]; pr[p] = P[(size_t)p * n + t]; }
-    int8_t flag = 0;
-    const int it = utoprimgen(u, g, g.igdet, pr, flag, ph.gam, ph.gammafail, false, 0.0, nullptr);
-#pragma unroll
-    for (int p = 0; p < NPR; p++) P[(size_t)p * n + t] = pr[p];
-    pflag[t] = flag;
-    if (iters) iters[t] = it;
-  };
   if (tid == 0) count = 0;
   __syncthreads();
   // a window's number is blockIdx.x + k gridDim.x: the list holds k and the place in the window
@@ -637,7 +649,7 @@ __global__ void __launch_bounds__(128) k_utoprim_points_rest(size_t n, Phys ph, 
       c -= take;
       if (tid < (int)take) {
         const unsigned int e = list[c + tid];
-        work(((size_t)blockIdx.x + (size_t)(e / kWin) * gridDim.x) * kWin + e % kWin);
+        utoprim_point(n, ((size_t)blockIdx.x + (size_t)(e / kWin) * gridDim.x) * kWin + e % kWin, ph, U, geom, P, pflag, iters);
       }
     }
     __syncthreads();
@@ -645,6 +657,18 @@ __global__ void __launch_bounds__(128) k_utoprim_points_rest(size_t n, Phys ph, 
     if (tid == 0) count = c;
     __syncthreads();
   }
+}
+
+// Few points, in one launch: as long as the chip holds about two rounds of them at 255 registers
+// (256 threads per SM), the longest point's chain is the call's length, and the split above only
+// adds its launch and the first kPointsCap steps to it (us per call, one kernel against two:
+// 1000 points 242 / 264, 25,000 246 / 272, 65,000 265 / 267, 75,000 268 / 268, 130,000 291 / 281).
+constexpr int kPointsOneLaunch = 512;  // points per SM up to which one launch is the faster
+__global__ void __launch_bounds__(128) k_utoprim_points_few(size_t n, Phys ph, const double* __restrict__ U,
+                                                            const double* __restrict__ geom, double* __restrict__ P,
+                                                            int8_t* __restrict__ pflag, int32_t* __restrict__ iters) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) utoprim_point(n, t, ph, U, geom, P, pflag, iters);
 }
 
 // the same with the learned start of the hot inversion (fallback to the plain start inside
@@ -860,6 +884,8 @@ int hp_points(harm_ctx* c, size_t n, int guess, const double* U, const double* g
     const unsigned int nb = (unsigned int)std::min<size_t>((n + 255) / 256, (size_t)2 * c->num_sms);
     k_utoprim_points_mlp<<<nb, 256, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters,
                                                    reinterpret_cast<const MlpPacked*>(c->d_mlp), c->d_stats);
+  } else if (n <= (size_t)kPointsOneLaunch * c->num_sms) {
+    k_utoprim_points_few<<<nblk((long long)n, 128), 128, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters);
   } else {
     k_utoprim_points<<<nblk((long long)n, 128), 128, 0, c->stream>>>(n, ph, U, geom, P, pflag, iters);
     const unsigned int nb = (unsigned int)std::min<size_t>((n + 1023) / 1024, (size_t)2 * c->num_sms);
