@@ -38,6 +38,8 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
     return seterr_msg("unknown reconstruction", 2);
   if (g->lim == HARM_LIM_WENO5 && g->ng < 6) return seterr_msg("WENO5 needs ng >= 6", 2);
   if (g->lim == HARM_LIM_PARALINE && g->ng < 4) return seterr_msg("PARALINE needs ng >= 4", 2);
+  // the fluxes of the transverse ghost layer that flux-CT reads
+  if (g->ng < 1 || (g->n3 > 1 && g->ng3 < 1)) return seterr_msg("at least one ghost zone is needed", 2);
   if (g->fluxmethod != HARM_FLUX_HLL && g->fluxmethod != HARM_FLUX_LAXF) return seterr_msg("unknown fluxmethod", 2);
   double mlp_gate = 0.02;  // the gated learned start's threshold (HARM_B200_MLP_GATE)
   if (const char* e = getenv("HARM_B200_MLP_GATE")) {

@@ -216,11 +216,13 @@ constexpr int kReconBlocks = sizeof(T) == 4 ? 4 : 5;
 template <typename T>
 constexpr int kReconUnroll = sizeof(T) == 4 ? 2 : 1;
 
-template <int DIR, int LIM, typename T, int TU = HARM_TU>
+// CLAMP: for fewer ghost zones than the stencil reaches (recon_narrow); cells beyond the grid are
+// the grid's last one in that direction.  It serves x1 too, whose rows have no ends to stop at.
+template <int DIR, int LIM, typename T, bool CLAMP = false, int TU = HARM_TU>
 __global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
                                                                              const T* __restrict__ S, T* __restrict__ EL,
                                                                              T* __restrict__ ER) {
-  static_assert(DIR != 1, "x1: k_recon_x1");
+  static_assert(DIR != 1 || CLAMP, "x1: k_recon_x1");
   using V = typename ReconLanes<T>::V;
   constexpr int N = ReconLanes<T>::N, D = ReconWin<LIM>::D;
   constexpr bool HAS_S = ReconWin<LIM>::S;
@@ -228,7 +230,8 @@ __global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dim
   const int line0 = ((int)blockIdx.x * kReconWarps + (int)(threadIdx.x >> 5)) * 32 * N;
   if (line0 >= rb.nlines) return;
   const int a = rb.c0 + (int)blockIdx.y * rb.chunk, b = min(a + rb.chunk - 1, rb.c1);
-  const unsigned stride = (DIR == 2) ? (unsigned)d.n1e : (unsigned)d.plane;
+  const unsigned stride = (DIR == 1) ? 1u : (DIR == 2) ? (unsigned)d.n1e : (unsigned)d.plane;
+  [[maybe_unused]] const int cells_along = (DIR == 1) ? d.n1e : (DIR == 2) ? d.n2e : d.n3e;
   const double* Pp = P + (size_t)blockIdx.z * d.cells;
   T* el = EL + (size_t)blockIdx.z * d.cells;
   T* er = ER + (size_t)blockIdx.z * d.cells;
@@ -238,8 +241,15 @@ __global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dim
   for (int q = 0; q < N; q++) {
     const int l = min(line0 + 32 * q + lane, rb.nlines - 1);
     const unsigned t = rb.t0 + l % rb.nt, o = rb.o0 + l / rb.nt;
-    at[q] = ((DIR == 2) ? o * (unsigned)d.plane + t : o * (unsigned)d.n1e + t) + (unsigned)(a - D) * stride;
+    const unsigned first = (DIR == 1) ? o * (unsigned)d.plane + t * (unsigned)d.n1e
+                         : (DIR == 2) ? o * (unsigned)d.plane + t : o * (unsigned)d.n1e + t;
+    at[q] = first + (unsigned)(a - D) * stride;
   }
+  // the value at cell c of line q, whose offset is at[q]
+  auto value = [&](int q, int c) -> double {
+    if constexpr (CLAMP) return __ldg(Pp + (at[q] + (unsigned)(min(max(c, 0), cells_along - 1) - c) * stride));
+    else return __ldg(Pp + at[q]);
+  };
   const bool ok0 = line0 + lane < rb.nlines, ok1 = N == 2 && line0 + 32 + lane < rb.nlines;
   const auto K = recon_consts<LIM, T>();
   ReconLine<LIM, V> ln;
@@ -250,9 +260,9 @@ __global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dim
   double nx[2][N];
 #pragma unroll
   for (int q = 0; q < N; q++) {
-    nx[0][q] = __ldg(Pp + at[q]);
+    nx[0][q] = value(q, cell);
     at[q] += stride;
-    nx[1][q] = __ldg(Pp + at[q]);
+    nx[1][q] = value(q, cell + 1);
   }
   cell++;
   // takes the next cell and loads the one two after it
@@ -266,7 +276,7 @@ __global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dim
     for (int q = 0; q < N; q++) {
       nx[0][q] = nx[1][q];
       at[q] += stride;
-      if (more) nx[1][q] = __ldg(Pp + at[q]);
+      if (more) nx[1][q] = value(q, cell);
     }
     return v;
   };
@@ -465,21 +475,24 @@ __global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const d
   else { l = (int)(t % rb.nlines); c = (int)(t / rb.nlines); }
   c += rb.c0;
   const int tt = rb.t0 + l % rb.nt, o = rb.o0 + l / rb.nt;
-  const size_t stride = (DIR == 1) ? 1 : (DIR == 2) ? (size_t)d.n1e : d.plane;
+  const long long stride = (DIR == 1) ? 1 : (DIR == 2) ? (long long)d.n1e : (long long)d.plane;
   const size_t id = (DIR == 1) ? cidx(d, c, tt, o) : (DIR == 2) ? cidx(d, tt, c, o) : cidx(d, tt, o, c);
+  // the cell q further along the direction, or the grid's last one
+  const int cells_along = (DIR == 1) ? d.n1e : (DIR == 2) ? d.n2e : d.n3e;
+  auto along = [&](int q) { return id + (min(max(c + q, 0), cells_along - 1) - c) * stride; };
   if constexpr (LIM == HARM_LIM_WENO5) {
     const T* Lq = L + (size_t)3 * (DIR - 1) * d.cells;
     const T* ve = Lq + d.cells;
     const T* up = Lq + 2 * d.cells;
     S[id] = weno_dp_strength<T>(weno_dp<T>((T)__ldg(P + (size_t)HARM_RHO * d.cells + id), __ldg(Lq + id), __ldg(up + id),
-                                           __ldg(ve + id - stride), __ldg(ve + id + stride), __ldg(up + id - stride),
-                                           __ldg(up + id + stride)));
+                                           __ldg(ve + along(-1)), __ldg(ve + along(1)), __ldg(up + along(-1)),
+                                           __ldg(up + along(1))));
   } else {
     const T* Vd = L + (size_t)DIR * d.cells;
     T v[7], pp[7];
 #pragma unroll
     for (int q = 0; q < 7; q++) {
-      const size_t at = id + (size_t)q * stride - 3 * stride;
+      const size_t at = along(q - 3);
       v[q] = (q >= 1 && q <= 5) ? __ldg(Vd + at) : T(0);
       pp[q] = __ldg(L + at);
     }
@@ -576,6 +589,16 @@ static inline ReconBox recon_box(const Dims& d, const FaceBox& fb) {
   return rb;
 }
 
+// Whether the stencils of a direction reach beyond its ghost zones (a caller's own grid:
+// harm_grid_setup gives as many as they need).  Grids of WENO5 and PARALINE are created with
+// enough of them in x1 and x2 only.
+template <int DIR, int LIM>
+constexpr bool recon_may_be_narrow = DIR == 3 || LIM == HARM_LIM_MC || LIM == HARM_LIM_PARA;
+template <int DIR, int LIM>
+static inline bool recon_narrow(const Dims& d) {
+  return recon_may_be_narrow<DIR, LIM> && (DIR == 3 ? d.ng3 : d.ng) <= ReconWin<LIM>::D;
+}
+
 // The two kernels of one direction on a face box; E: scratch of 2 x 8 x cells of T.  The cell
 // pass L has to be there for the box's stencils (WENO5, PARALINE).
 // Chunks of a march: each costs its first cell's window again (10 loads and 4 cells' weights for
@@ -597,7 +620,12 @@ static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const F
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     launches++;
   }
-  if constexpr (DIR == 1) {
+  if (recon_narrow<DIR, LIM>(d)) {
+    if constexpr (recon_may_be_narrow<DIR, LIM>) {
+      constexpr int LN = 32 * ReconLanes<T>::N * kReconWarps;
+      k_recon<DIR, LIM, T, true><<<dim3((rb.nlines + LN - 1) / LN, 1, NPR), 32 * kReconWarps, 0, st>>>(d, rb, P, S, EL, ER);
+    }
+  } else if constexpr (DIR == 1) {
     const long long range = (long long)rb.nt * d.n1e, nseg = (range + ReconRow<LIM>::E - 1) / ReconRow<LIM>::E;
     const long long items = nseg * (rb.nlines / rb.nt);
     if (items > 0x7FFFFFFF) return cudaErrorInvalidValue;

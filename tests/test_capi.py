@@ -56,3 +56,18 @@ def test_host_entry_points_reject_null_arguments():
     assert b"null" in dev.harm_b200_last_error()
     assert dev.harm_b200_mixed_reciprocal(None, None, None, 8) == 1
     assert dt.value == 1e-3
+
+
+def test_grids_without_ghost_zones_are_refused():
+    """Flux-CT reads the fluxes of one transverse ghost layer: a grid without one is an error (2)
+    before any CUDA call, in x3 only where the grid has that direction."""
+    import ctypes as C
+    from harm_harm_b200 import Grid
+    dev = N.device_lib()
+    ctx = C.c_void_p()
+    for n3, ng, ng3 in ((1, 0, 0), (8, 0, 0), (8, 4, 0)):
+        g = Grid.torus(16, 16, n3).g
+        g.ng, g.ng3 = ng, ng3
+        g.n1e, g.n2e, g.n3e = 16 + 2 * ng, 16 + 2 * ng, n3 + 2 * ng3
+        assert dev.harm_b200_create_grid(C.byref(g), 0, C.byref(ctx)) == 2
+        assert b"ghost zone" in dev.harm_b200_last_error() and not ctx

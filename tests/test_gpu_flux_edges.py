@@ -5,13 +5,14 @@ the oracle to 1e-12 of each field's largest face value; FP32 (mixed path) agains
 both reconstruct the same state, and a face flux carries the rounding of a few dozen FP32
 operations on the face's largest terms, of which a substep adds dt/dx < 1: 64 half-ulps of a
 field's largest value (of the state's, for the vectors, whose components share their terms)."""
+import ctypes as C
 from fractions import Fraction
 
 import numpy as np
 import pytest
 
 from helpers import make_torus, plant_compression, rel_err
-from harm_harm_b200 import HARM_PREC_FP64, HARM_PREC_MIXED, Harm
+from harm_harm_b200 import HARM_PREC_FP64, HARM_PREC_MIXED, Grid, Harm
 from oracle import oracle as O
 
 SHAPES = [(5, 7, 1), (59, 9, 1), (33, 21, 6), (64, 13, 7), (131, 8, 12), (17, 70, 9)]
@@ -73,3 +74,48 @@ def test_corrected_quotients_are_ieee():
             r = float(Fraction(float(a)) - Fraction(b) * Fraction(q))  # fma(-b, q, a): one rounding
             got = float(Fraction(r) * Fraction(y) + Fraction(q))       # fma(r, y, q)
             assert got == float(a) / b
+
+
+def _narrowed(g, geom, P, ng, ng3):
+    """the same active grid with ng (x3: ng3) ghost zones, its tables and its state; and the state of
+    the wide grid whose ghost zones beyond those repeat the last one of them"""
+    a, b = g.g, type(g.g)()
+    C.memmove(C.byref(b), C.byref(a), C.sizeof(a))
+    b.ng, b.ng3 = ng, ng3
+    b.n1e, b.n2e, b.n3e = a.n1 + 2 * ng, a.n2 + 2 * ng, a.n3 + 2 * ng3
+    cut, cut3 = a.ng - ng, a.ng3 - ng3
+    inner = slice(cut, -cut or None)
+    tables = [np.ascontiguousarray(t[..., inner, inner]) for t in geom]
+    Pn = np.ascontiguousarray(P[:, cut3:P.shape[1] - cut3, inner, inner])
+    k, j, i = (np.clip(np.arange(n) - c, 0, m - 1) for n, c, m in zip(P.shape[1:], (cut3, cut, cut), Pn.shape[1:]))
+    return Grid(b), tables, Pn, np.ascontiguousarray(Pn[:, k][:, :, j][:, :, :, i])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,lim,ng,ng3", [((40, 33, 1), 0, 1, 0), ((19, 70, 9), 0, 1, 1), ((70, 12, 7), 1, 1, 1), ((33, 21, 1), 1, 2, 0),
+                                              ((12, 9, 35), 1, 2, 2), ((37, 12, 9), 2, 6, 5), ((20, 9, 40), 2, 6, 1), ((33, 9, 8), 3, 4, 3),
+                                              ((70, 8, 9), 3, 4, 1)])
+def test_fewer_ghost_zones_than_the_stencil(cuda, shape, lim, ng, ng3):
+    """A caller's grid with fewer ghost zones than the reconstruction reads: a cell beyond the grid is
+    the grid's last one, so the fluxes are those of a wide grid whose outer ghost zones repeat it.
+    FP64 to the bit; the mixed path to a few FP32 roundings of the largest (as above)."""
+    g, geom, conn, aux, P = make_torus(*shape, lim=lim)
+    O.Oracle(g, geom, conn, aux).bound_prim(P)
+    gn, tables, Pn, Pw = _narrowed(g, (geom, conn, aux), P, ng, ng3)
+    got = []
+    for grid, tabs, p in ((g, (geom, conn, aux), Pw), (gn, tables, Pn)):
+        dev, Pd = Harm(grid, *tabs), cuda.from_numpy(p).cuda()
+        Fd = [cuda.zeros_like(Pd) for _ in range(3)]
+        ndt = dev.fluxcalc(Pd, *Fd)
+        pf, flag = cuda.zeros_like(Pd), cuda.zeros(p.shape[1:], dtype=cuda.int8, device="cuda")
+        dev.advance(0, Pd, Pd, pf, flag, 0.2 / sum(1.0 / x for x in ndt if x < 1e99), precision=HARM_PREC_MIXED)
+        ok = flag.cpu().numpy()[grid.active] == 0
+        got.append((ndt, [f.cpu().numpy()[_faces(grid, d + 1)] for d, f in enumerate(Fd)], pf.cpu().numpy()[(slice(None), *grid.active)], ok))
+    assert got[0][0] == got[1][0]
+    for d in range(3 if shape[2] > 1 else 2):
+        assert np.array_equal(got[0][1][d], got[1][1][d]), d + 1
+    ok = got[0][3] & got[1][3]
+    assert ok.mean() > 0.9
+    for pl in range(8):
+        own, most = np.abs(got[0][2][pl]).max(), np.abs(got[0][2]).max()
+        assert np.abs(got[1][2][pl] - got[0][2][pl])[ok].max() < 64 * 2.0**-24 * (own + (pl >= 2) * most), pl
