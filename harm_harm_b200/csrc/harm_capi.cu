@@ -62,10 +62,11 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   CK(cudaMalloc(&c->d_geomf, gsz * sizeof(float)));
   CK(cudaMalloc(&c->d_conn, 64 * d.plane * sizeof(double)));
   CK(cudaMalloc(&c->d_aux, HARM_NAUX * d.plane * sizeof(double)));
-  // fluxes of the three directions and one direction's edge values, in FP64 or in FP32: a substep
-  // runs in one arithmetic and leaves nothing in them, so the two share their memory
-  const size_t nf = NPR * d.cells;
-  CK(cudaMalloc(&c->d_flux, 5 * nf * sizeof(double)));
+  // fluxes of the three directions and one direction's edge values (a small grid's: each one's),
+  // in FP64 or in FP32: a substep runs in one arithmetic and leaves nothing in them, so the two
+  // share their memory
+  const size_t nf = NPR * d.cells, ndir = one_launch_fluxes(d, g->lim, false) ? 3 : 1;
+  CK(cudaMalloc(&c->d_flux, (3 + 2 * ndir) * nf * sizeof(double)));
   for (int q = 0; q < 3; q++) {
     c->d_F[q] = (double*)c->d_flux + q * nf;
     c->d_Ff[q] = (float*)c->d_flux + q * nf;
@@ -76,10 +77,10 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   c->d_emff = (float*)c->d_emf;
   if (g->lim == HARM_LIM_WENO5 || g->lim == HARM_LIM_PARALINE) {
     const size_t nl = (g->lim == HARM_LIM_WENO5 ? 9 : 4) * d.cells;
-    CK(cudaMalloc(&c->d_line, (nl + d.cells) * sizeof(double)));
+    CK(cudaMalloc(&c->d_line, (nl + ndir * d.cells) * sizeof(double)));
     c->d_coef = (double*)c->d_line + nl;
     // read (and not used) at ghost cells that no pass writes
-    CK(cudaMemset(c->d_coef, 0, d.cells * sizeof(double)));
+    CK(cudaMemset(c->d_coef, 0, ndir * d.cells * sizeof(double)));
   }
   CK(cudaMalloc(&c->d_pk, NPR * d.cells * sizeof(double)));
   CK(cudaMalloc(&c->d_U, NPR * d.cells * sizeof(double)));
@@ -381,6 +382,14 @@ extern "C" int harm_b200_step(harm_ctx* c, int precision, int guess, double* d_P
   return harm_b200_step_n(c, precision, guess, d_P, 1, dt, stats);
 }
 
+// planes of a slab of the host copies: at most HARM_H2D_SLABS slabs, of at least a megabyte (20 us
+// of PCIe, about what the flux launches of one slab take to start)
+static int slab_planes(const harm_ctx* c) {
+  const size_t bytes = NPR * c->plane * sizeof(double);
+  const int least = (int)std::min<size_t>(((size_t)1 << 20) / bytes + 1, (size_t)c->g.n3e);
+  return std::max((c->g.n3e + HARM_H2D_SLABS - 1) / HARM_H2D_SLABS, least);
+}
+
 // H2D of the state in at most HARM_H2D_SLABS slabs of k-planes (one two-dimensional copy per
 // slab, followed by an event) on the copy stream, after the context
 // stream's earlier work
@@ -396,7 +405,7 @@ static int h2d_slabs(harm_ctx* c, const double* h_P, SlabWait* sw, bool harm_lay
     for (int s = 0; s < HARM_H2D_SLABS; s++) CK(cudaEventCreateWithFlags(&c->slab_ev[s], cudaEventDisableTiming));
   }
   const int n3e = c->g.n3e;
-  const int planes = (n3e + HARM_H2D_SLABS - 1) / HARM_H2D_SLABS;
+  const int planes = slab_planes(c);
   const int nslab = (n3e + planes - 1) / planes;
   CK(cudaEventRecord(c->entry_ev, c->stream));
   CK(cudaStreamWaitEvent(c->copy_stream, c->entry_ev, 0));
@@ -465,7 +474,7 @@ static int d2h_slabs(harm_ctx* c, double* h_P) {
     for (int s = 0; s < HARM_H2D_SLABS; s++) CK(cudaEventCreateWithFlags(&c->d2h_ev[s], cudaEventDisableTiming));
   }
   const int n3e = c->g.n3e;
-  const int planes = (n3e + HARM_H2D_SLABS - 1) / HARM_H2D_SLABS;
+  const int planes = slab_planes(c);
   const int nslab = (n3e + planes - 1) / planes;
   CK(cudaEventRecord(c->done_ev, c->stream));
   CK(cudaStreamWaitEvent(c->d2h_stream, c->done_ev, 0));

@@ -177,6 +177,20 @@ struct FaceBox {
   long long n;
 };
 
+// Grids whose flux stage takes the three directions in one launch per kernel (harm_recon.cuh), with
+// edge values and coefficients of all three.  A launch that waits for the one before costs three to
+// four microseconds, and a small grid leaves most of the chip idle in each, so the line lies where
+// the joint kernels' larger code and registers cost more.  Full steps, one launch per direction
+// against joint, us, by extended cells:
+//   FP64 WENO5 27 k 550 / 409, 64 k 576 / 488, 112 k 587 / 572, but a 2-D one of 87 k 551 / 562 and
+//   200 k 727 / 813 (its x1 rows take three blocks per SM and 80 registers by themselves);
+//   the others gain up to the largest tried: mixed WENO5 200 k 422 / 380, 358 k 567 / 546, mixed MC
+//   161 k 303 / 278, 297 k 412 / 389, FP64 MC 161 k 384 / 372, 270 k 510 / 507, PARALINE 297 k
+//   mixed 492 / 452, FP64 677 / 646.
+static inline bool one_launch_fluxes(const Dims& d, int lim, bool fp64) {
+  return d.cells <= ((lim == HARM_LIM_WENO5 && fp64) ? 72000 : 360000);
+}
+
 static inline FaceBox face_box(const Dims& d, int dir) {
   FaceBox b;
   int n[3] = {d.n1, d.n2, d.n3};

@@ -45,8 +45,8 @@ struct harm_ctx {
   float* d_emff;
   void* d_line;     // the flux stage's cell pass: WENO5 [9][cells], PARALINE [4][cells] (FP64 path:
                     // double, mixed path: float)
-  void* d_coef;     // its per-cell coefficient of one direction, [cells]
-  double* d_edge;   // left and right edge values of one direction, [2][8][cells]
+  void* d_coef;     // its per-cell coefficient of one direction, [cells] (small grids: of each)
+  double* d_edge;   // left and right edge values of one direction, [2][8][cells] (small grids: of each)
   float* d_edgef;
   double* d_pk;     // midpoint primitives of the RK2 step
   double* d_U;      // conserved variables to invert (UEVOLVE)

@@ -415,7 +415,7 @@ __device__ __forceinline__ int8_t flag_at(const Dims& d, const int8_t* flag, int
     else if (jj >= d.ng + d.n2) jj = 2 * (d.ng + d.n2) - 1 - jj;
     if (ii >= d.ng + d.n1) ii = d.ng + d.n1 - 1;
   }
-  return flag[cidx(d, ii, jj, kk)];
+  return __ldg(flag + cidx(d, ii, jj, kk));
 }
 
 // ------------------------------------------------------------------ post_fixup
@@ -434,18 +434,19 @@ __device__ __forceinline__ int8_t flag_at(const Dims& d, const int8_t* flag, int
 // written by k_fixup_apply, so that every cell's fix reads the unfixed neighbours.
 // One thread per cell of the extended i, j range and the active k: the ghost flags of x1 and
 // x2 (ghosts set) are written by their own threads, and the active cells read their neighbours'
-// flags through flag_at, which reads none of those.
+// flags through flag_at, which reads none of those.  Without GHOSTS they are filled already.
+template <bool GHOSTS>
 __global__ void __launch_bounds__(256) k_fixup_compute(Dims d, Phys ph, const double* __restrict__ P,
                                                        int8_t* flag, const double* __restrict__ geom,
                                                        FixRec* __restrict__ recs, unsigned int* __restrict__ nrec,
-                                                       unsigned int cap, int finalstep, int ghosts) {
+                                                       unsigned int cap, int finalstep) {
   const unsigned int c2 = blockIdx.x * 256u + threadIdx.x;
   if (c2 >= (unsigned int)d.plane) return;
   const int ii = (int)(c2 % (unsigned int)d.n1e), jj = (int)(c2 / (unsigned int)d.n1e), kk = (int)blockIdx.y + d.ng3;
   const int i = ii - d.ng, j = jj - d.ng;
   const size_t id = (size_t)kk * d.plane + c2;
   if (i < 0 || i >= d.n1 || j < 0 || j >= d.n2) {
-    if (ghosts && (j < 0 || j >= d.n2 || i >= d.n1)) {
+    if (GHOSTS && (j < 0 || j >= d.n2 || i >= d.n1)) {
       const int js = (j < 0) ? 2 * d.ng - 1 - jj : (j >= d.n2) ? 2 * (d.ng + d.n2) - 1 - jj : jj;
       flag[id] = flag[cidx(d, (i >= d.n1) ? d.ng + d.n1 - 1 : ii, js, kk)];
     }
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(256) k_fixup_compute(Dims d, Phys ph, const do
   int numavg0 = 0, numavg1 = 0;
   const double ref = P[(size_t)HARM_UU * d.cells + id];
   // cells with a neighbour whose flag this launch writes
-  const bool edge = ghosts && (i == d.n1 - 1 || j == 0 || j == d.n2 - 1);
+  const bool edge = GHOSTS && (i == d.n1 - 1 || j == 0 || j == d.n2 - 1);
   for (int qq = 0; qq < npairs; qq++) {
     int di = (qq % rnx) - s1, dj = ((qq % (rnx * rny)) / rnx) - s2, dk = (qq / (rnx * rny)) - s3;
     size_t a = cidx(d, ii + di, jj + dj, kk + dk), b = cidx(d, ii - di, jj - dj, kk - dk);
@@ -474,8 +475,8 @@ __global__ void __launch_bounds__(256) k_fixup_compute(Dims d, Phys ph, const do
       thisok = flag_at(d, flag, ii + di, jj + dj, kk + dk) <= 0;
       thatok = flag_at(d, flag, ii - di, jj - dj, kk - dk) <= 0;
     } else {
-      thisok = flag[a] <= 0;
-      thatok = flag[b] <= 0;
+      thisok = __ldg(flag + a) <= 0;
+      thatok = __ldg(flag + b) <= 0;
     }
     numavg0 += thisok + thatok;
     for (int p = startpl; p <= endpl; p++) {
@@ -861,8 +862,9 @@ int hp_fixup(harm_ctx* c, double* pf, int8_t* pflag, int finalstep, bool bound_f
   Phys ph = phys_of(c->g);
   if (bound_flags && hp_bound(c, nullptr, pflag)) return 1;
   if (bound_flags) CK(cudaMemsetAsync(c->d_nrec, 0, sizeof(unsigned int), c->stream));  // else k_emf did
-  k_fixup_compute<<<dim3(nblk((long long)d.plane), d.n3), 256, 0, c->stream>>>(
-      d, ph, pf, pflag, c->d_geom, (FixRec*)c->d_fixrec, c->d_nrec, c->fix_cap, finalstep, bound_one_launch(d) ? 1 : 0);
+  const auto k = bound_one_launch(d) ? k_fixup_compute<true> : k_fixup_compute<false>;
+  k<<<dim3(nblk((long long)d.plane), d.n3), 256, 0, c->stream>>>(d, ph, pf, pflag, c->d_geom, (FixRec*)c->d_fixrec, c->d_nrec,
+                                                                c->fix_cap, finalstep);
   k_fixup_apply<<<4 * c->num_sms, 256, 0, c->stream>>>(d, pf, pflag, (const FixRec*)c->d_fixrec, c->d_nrec, c->fix_cap);
   c->launches += 2;
   CK(cudaGetLastError());

@@ -218,23 +218,23 @@ constexpr int kReconUnroll = sizeof(T) == 4 ? 2 : 1;
 
 // CLAMP: for fewer ghost zones than the stencil reaches (recon_narrow); cells beyond the grid are
 // the grid's last one in that direction.  It serves x1 too, whose rows have no ends to stop at.
-template <int DIR, int LIM, typename T, bool CLAMP = false, int TU = HARM_TU>
-__global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
-                                                                             const T* __restrict__ S, T* __restrict__ EL,
-                                                                             T* __restrict__ ER) {
+template <int DIR, int LIM, typename T, bool CLAMP>
+__device__ __forceinline__ void recon_march(const Dims& d, const ReconBox& rb, const double* __restrict__ P,
+                                            const T* __restrict__ S, T* __restrict__ EL, T* __restrict__ ER, int group,
+                                            int chunk, int prim) {
   static_assert(DIR != 1 || CLAMP, "x1: k_recon_x1");
   using V = typename ReconLanes<T>::V;
   constexpr int N = ReconLanes<T>::N, D = ReconWin<LIM>::D;
   constexpr bool HAS_S = ReconWin<LIM>::S;
   const int lane = threadIdx.x & 31;
-  const int line0 = ((int)blockIdx.x * kReconWarps + (int)(threadIdx.x >> 5)) * 32 * N;
+  const int line0 = (group * kReconWarps + (int)(threadIdx.x >> 5)) * 32 * N;
   if (line0 >= rb.nlines) return;
-  const int a = rb.c0 + (int)blockIdx.y * rb.chunk, b = min(a + rb.chunk - 1, rb.c1);
+  const int a = rb.c0 + chunk * rb.chunk, b = min(a + rb.chunk - 1, rb.c1);
   const unsigned stride = (DIR == 1) ? 1u : (DIR == 2) ? (unsigned)d.n1e : (unsigned)d.plane;
   [[maybe_unused]] const int cells_along = (DIR == 1) ? d.n1e : (DIR == 2) ? d.n2e : d.n3e;
-  const double* Pp = P + (size_t)blockIdx.z * d.cells;
-  T* el = EL + (size_t)blockIdx.z * d.cells;
-  T* er = ER + (size_t)blockIdx.z * d.cells;
+  const double* Pp = P + (size_t)prim * d.cells;
+  T* el = EL + (size_t)prim * d.cells;
+  T* er = ER + (size_t)prim * d.cells;
   // offset within one primitive of the newest cell of each line (lines past the last repeat it)
   unsigned at[N];
 #pragma unroll
@@ -314,6 +314,13 @@ __global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dim
   }
 }
 
+template <int DIR, int LIM, typename T, bool CLAMP = false, int TU = HARM_TU>
+__global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon(Dims d, ReconBox rb, const double* __restrict__ P,
+                                                                             const T* __restrict__ S, T* __restrict__ EL,
+                                                                             T* __restrict__ ER) {
+  recon_march<DIR, LIM, T, CLAMP>(d, rb, P, S, EL, ER, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
 // x1: the rows of a plane's lines are one contiguous range of memory, ghost cells included; a warp
 // takes segments of 64 of its cells (positions), wherever rows end in them: the edges of ghost
 // cells beyond c0 .. c1 are computed from whatever is next to them and never read.  WENO5: the
@@ -338,23 +345,19 @@ struct ReconRowSmem {
   T w0[64], w2[64], f[64];
 };
 
-template <int LIM, typename T, int TU = HARM_TU>
-__global__ void __launch_bounds__(32 * kRowWarps, kRowBlocks<T>) k_recon_x1(Dims d, ReconBox rb, FastDiv dseg,
-                                                             const double* __restrict__ P,
-                                                             const T* __restrict__ S, T* __restrict__ EL,
-                                                             T* __restrict__ ER) {
+// the segments it, it + nw, ... of the box
+template <int LIM, typename T>
+__device__ __forceinline__ void recon_rows(const Dims& d, const ReconBox& rb, const FastDiv& dseg,
+                                           const double* __restrict__ P, const T* __restrict__ S, T* __restrict__ EL,
+                                           T* __restrict__ ER, ReconRowSmem<T>& w, int it, int nw, int prim) {
   using R = ReconRow<LIM>;
   constexpr int H = R::H, M = R::M;
   constexpr bool HAS_S = ReconWin<LIM>::S;
-  __shared__ ReconRowSmem<T> rows[kRowWarps];
-  ReconRowSmem<T>& w = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const double* Pp = P + (size_t)blockIdx.z * d.cells;
-  T* el = EL + (size_t)blockIdx.z * d.cells;
-  T* er = ER + (size_t)blockIdx.z * d.cells;
+  const double* Pp = P + (size_t)prim * d.cells;
+  T* el = EL + (size_t)prim * d.cells;
+  T* er = ER + (size_t)prim * d.cells;
   const int items = rb.nlines / rb.nt * (int)dseg.d;  // segments of the box
-  int it = (int)blockIdx.x * kRowWarps + (int)(threadIdx.x >> 5);
-  const int nw = (int)gridDim.x * kRowWarps;
   const unsigned plane = (unsigned)d.plane, row0 = (unsigned)rb.t0 * (unsigned)d.n1e;
   const unsigned ncell = (unsigned)rb.nt * (unsigned)d.n1e, top = (unsigned)d.cells - 1u;
   double nx[3];
@@ -460,15 +463,25 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowBlocks<T>) k_recon_x1(Dims
   }
 }
 
+template <int LIM, typename T, int TU = HARM_TU>
+__global__ void __launch_bounds__(32 * kRowWarps, kRowBlocks<T>) k_recon_x1(Dims d, ReconBox rb, FastDiv dseg,
+                                                             const double* __restrict__ P,
+                                                             const T* __restrict__ S, T* __restrict__ EL,
+                                                             T* __restrict__ ER) {
+  __shared__ ReconRowSmem<T> rows[kRowWarps];
+  const int warp = threadIdx.x >> 5;
+  recon_rows<LIM, T>(d, rb, dseg, P, S, EL, ER, rows[warp], (int)blockIdx.x * kRowWarps + warp, (int)gridDim.x * kRowWarps,
+                     blockIdx.z);
+}
+
 // ------------------------------------------------------------------ per-cell coefficients
 
-// S of direction DIR for the edge cells of a ReconBox, from the cell pass L (k_cellprep): the
+// S of direction DIR for edge cell t of a ReconBox, from the cell pass L (k_cellprep): the
 // strength of WENO5BND's momentum-flux reduction, or PARALINE's flattening coefficient
-template <int DIR, int LIM, typename T, int TU = HARM_TU>
-__global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const double* __restrict__ P,
-                                                    const T* __restrict__ L, T* __restrict__ S) {
+template <int DIR, int LIM, typename T>
+__device__ __forceinline__ void recon_coef(const Dims& d, const ReconBox& rb, const double* __restrict__ P,
+                                           const T* __restrict__ L, T* __restrict__ S, long long t) {
   const int nc = rb.c1 - rb.c0 + 1;
-  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= (long long)nc * rb.nlines) return;
   int c, l;
   if (DIR == 1) { c = (int)(t % nc); l = (int)(t / nc); }
@@ -499,6 +512,11 @@ __global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const d
     S[id] = paraline_fi<T>(v, pp);
   }
 }
+template <int DIR, int LIM, typename T, int TU = HARM_TU>
+__global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const double* __restrict__ P,
+                                                    const T* __restrict__ L, T* __restrict__ S) {
+  recon_coef<DIR, LIM, T>(d, rb, P, L, S, (long long)blockIdx.x * 256 + threadIdx.x);
+}
 
 // ------------------------------------------------------------------ k_face
 
@@ -510,14 +528,14 @@ __global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const d
 template <typename T>
 constexpr int kFaceBlocks = sizeof(T) == 4 ? 5 : 4;
 constexpr int kFaceThreads = 128;
-template <int DIR, typename T, typename GT, int TU = HARM_TU>
-__global__ void __launch_bounds__(kFaceThreads, kFaceBlocks<T>) k_face(Dims d, Phys ph, FaceBox fb, const T* __restrict__ EL,
-                                                              const T* __restrict__ ER, const GT* __restrict__ geom,
-                                                              T* __restrict__ F, unsigned long long* __restrict__ dtslot,
-                                                              int kb) {
-  const int t = (int)blockIdx.x * kFaceThreads + threadIdx.x;
+// Block (bx, by) of a direction's faces: their fluxes, and the minimum of their time-step limits.
+template <int DIR, typename T, typename GT>
+__device__ __forceinline__ void face_block(const Dims& d, const Phys& ph, const FaceBox& fb, const T* __restrict__ EL,
+                                           const T* __restrict__ ER, const GT* __restrict__ geom, T* __restrict__ F,
+                                           unsigned long long* __restrict__ dtslot, int kb, int bx, int by) {
+  const int t = bx * kFaceThreads + (int)threadIdx.x;
   const int i = t % fb.cnt[0] + fb.lo[0], j = t / fb.cnt[0] + fb.lo[1];
-  const int k0 = (int)blockIdx.y * kb, k1 = min(k0 + kb, fb.cnt[2]);
+  const int k0 = by * kb, k1 = min(k0 + kb, fb.cnt[2]);
   constexpr int loc = (DIR == 1) ? HARM_LOC_FACE1 : (DIR == 2) ? HARM_LOC_FACE2 : HARM_LOC_CENT;
   const GT* tab = geom + (size_t)loc * HARM_NGF * d.plane;
   double top = 0.0;
@@ -571,6 +589,77 @@ __global__ void __launch_bounds__(kFaceThreads, kFaceBlocks<T>) k_face(Dims d, P
   }
   block_dt_atomic(top, ph.cour * ((DIR == 1) ? ph.dx1 : (DIR == 2) ? ph.dx2 : ph.dx3), dtslot);
 }
+template <int DIR, typename T, typename GT, int TU = HARM_TU>
+__global__ void __launch_bounds__(kFaceThreads, kFaceBlocks<T>) k_face(Dims d, Phys ph, FaceBox fb, const T* __restrict__ EL,
+                                                              const T* __restrict__ ER, const GT* __restrict__ geom,
+                                                              T* __restrict__ F, unsigned long long* __restrict__ dtslot,
+                                                              int kb) {
+  face_block<DIR, T, GT>(d, ph, fb, EL, ER, geom, F, dtslot, kb, blockIdx.x, blockIdx.y);
+}
+
+// ------------------------------------------------------------------ small grids
+
+// The stages of the three directions in one launch each, for grids whose launches take longer to
+// start than to run (one_launch_fluxes): a block belongs to one direction.
+struct ReconAll {
+  ReconBox rb[3];
+  unsigned blocks[3];  // of each direction (0 without x3)
+  unsigned groups[3];  // of a march's chunk
+  FastDiv dseg;
+};
+struct FaceAll {
+  FaceBox fb[3];
+  unsigned blocks[3], bx[3];
+};
+
+template <int LIM, typename T, int TU = HARM_TU>
+__global__ void __launch_bounds__(256) k_recon_coef_all(Dims d, ReconAll ra, const double* __restrict__ P,
+                                                        const T* __restrict__ L, T* __restrict__ S) {
+  unsigned b = blockIdx.x;
+  if (b < ra.blocks[0]) return recon_coef<1, LIM, T>(d, ra.rb[0], P, L, S, (long long)b * 256 + threadIdx.x);
+  b -= ra.blocks[0];
+  if (b < ra.blocks[1]) return recon_coef<2, LIM, T>(d, ra.rb[1], P, L, S + d.cells, (long long)b * 256 + threadIdx.x);
+  b -= ra.blocks[1];
+  recon_coef<3, LIM, T>(d, ra.rb[2], P, L, S + 2 * d.cells, (long long)b * 256 + threadIdx.x);
+}
+
+// E: [direction][left, right][8][cells]
+template <int LIM, typename T, int TU = HARM_TU>
+__global__ void __launch_bounds__(32 * kReconWarps, kReconBlocks<T>) k_recon_all(Dims d, ReconAll ra, const double* __restrict__ P,
+                                                                                 const T* __restrict__ S, T* __restrict__ E) {
+  __shared__ ReconRowSmem<T> rows[kReconWarps];
+  const size_t ne = (size_t)NPR * d.cells;
+  unsigned b = blockIdx.x;
+  if (b < ra.blocks[0]) {
+    const int warp = threadIdx.x >> 5;
+    return recon_rows<LIM, T>(d, ra.rb[0], ra.dseg, P, S, E, E + ne, rows[warp], (int)b * kReconWarps + warp,
+                              (int)ra.blocks[0] * kReconWarps, blockIdx.y);
+  }
+  b -= ra.blocks[0];
+  if (b < ra.blocks[1])
+    return recon_march<2, LIM, T, false>(d, ra.rb[1], P, S + d.cells, E + 2 * ne, E + 3 * ne, (int)(b % ra.groups[1]),
+                                         (int)(b / ra.groups[1]), blockIdx.y);
+  b -= ra.blocks[1];
+  recon_march<3, LIM, T, false>(d, ra.rb[2], P, S + 2 * d.cells, E + 4 * ne, E + 5 * ne, (int)(b % ra.groups[2]),
+                                (int)(b / ra.groups[2]), blockIdx.y);
+}
+
+template <typename T, typename GT, int TU = HARM_TU>
+__global__ void __launch_bounds__(kFaceThreads, kFaceBlocks<T>) k_face_all(Dims d, Phys ph, FaceAll fa, const T* __restrict__ E,
+                                                                  const GT* __restrict__ geom, T* __restrict__ F1,
+                                                                  T* __restrict__ F2, T* __restrict__ F3,
+                                                                  unsigned long long* __restrict__ slots) {
+  const size_t ne = (size_t)NPR * d.cells;
+  unsigned b = blockIdx.x;
+  if (b < fa.blocks[0])
+    return face_block<1, T, GT>(d, ph, fa.fb[0], E, E + ne, geom, F1, slots + 0, 1, (int)(b % fa.bx[0]), (int)(b / fa.bx[0]));
+  b -= fa.blocks[0];
+  if (b < fa.blocks[1])
+    return face_block<2, T, GT>(d, ph, fa.fb[1], E + 2 * ne, E + 3 * ne, geom, F2, slots + 1, 1, (int)(b % fa.bx[1]),
+                                (int)(b / fa.bx[1]));
+  b -= fa.blocks[1];
+  face_block<3, T, GT>(d, ph, fa.fb[2], E + 4 * ne, E + 5 * ne, geom, F3, slots + 2, 1, (int)(b % fa.bx[2]), (int)(b / fa.bx[2]));
+}
 
 // ------------------------------------------------------------------ launchers
 
@@ -599,12 +688,29 @@ static inline bool recon_narrow(const Dims& d) {
   return recon_may_be_narrow<DIR, LIM> && (DIR == 3 ? d.ng3 : d.ng) <= ReconWin<LIM>::D;
 }
 
-// The two kernels of one direction on a face box; E: scratch of 2 x 8 x cells of T.  The cell
+// Cuts a box's lines into chunks and gives their number.  Each chunk costs its first cell's window
+// again (10 loads and 4 cells' weights for WENO5), so a line is cut only as far as the chip needs
+// blocks: eight per SM (two waves; the other limiters, lighter in registers and bound by the
+// latency of their loads, 24), and at least 12 cells (the others 4: a march of a small grid is a
+// chain of load latencies).
+template <int LIM>
+static inline int cut_marches(ReconBox& rb, int groups, int num_sms) {
+  const int nc = rb.c1 - rb.c0 + 1;
+  constexpr int per_sm = (LIM == HARM_LIM_WENO5) ? 8 : 24;
+  int chunks = (per_sm * num_sms + groups * NPR - 1) / (groups * NPR);
+  chunks = std::max(1, std::min(chunks, nc / ((LIM == HARM_LIM_WENO5) ? 12 : 4)));
+  rb.chunk = (nc + chunks - 1) / chunks;
+  return (nc + rb.chunk - 1) / rb.chunk;
+}
+// the segments of the x1 rows of a plane
+template <int LIM>
+static inline long long row_segments(const Dims& d, const ReconBox& rb) {
+  return ((long long)rb.nt * d.n1e + ReconRow<LIM>::E - 1) / ReconRow<LIM>::E;
+}
+
+// The two kernels of one direction on a face box; E: scratch of 2 x 8 x cells of T, S of cells.  The cell
 // pass L has to be there for the box's stencils (WENO5, PARALINE).
-// Chunks of a march: each costs its first cell's window again (10 loads and 4 cells' weights for
-// WENO5), so a line is cut only as far as the chip needs blocks: eight per SM (two waves; the
-// other limiters, lighter in registers and bound by the latency of their loads, 24), and at least
-// 12 cells (the others 4: a march of a small grid is a chain of load latencies).  x1: segments are independent, and a warp takes the next one's loads under its own.
+// x1: segments are independent, and a warp takes the next one's loads under its own.
 template <int DIR, int LIM, typename T, typename GT>
 static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const FaceBox& fb, const double* P, const GT* geom,
                                           T* F, unsigned long long* slot, cudaStream_t st, const T* L, T* S, T* E,
@@ -626,19 +732,13 @@ static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const F
       k_recon<DIR, LIM, T, true><<<dim3((rb.nlines + LN - 1) / LN, 1, NPR), 32 * kReconWarps, 0, st>>>(d, rb, P, S, EL, ER);
     }
   } else if constexpr (DIR == 1) {
-    const long long range = (long long)rb.nt * d.n1e, nseg = (range + ReconRow<LIM>::E - 1) / ReconRow<LIM>::E;
-    const long long items = nseg * (rb.nlines / rb.nt);
+    const long long nseg = row_segments<LIM>(d, rb), items = nseg * (rb.nlines / rb.nt);
     if (items > 0x7FFFFFFF) return cudaErrorInvalidValue;
     const long long blocks = std::min<long long>((items + kRowWarps - 1) / kRowWarps, 4LL * num_sms);
     k_recon_x1<LIM, T><<<dim3((unsigned)blocks, 1, NPR), 32 * kRowWarps, 0, st>>>(d, rb, fast_div((unsigned)nseg), P, S, EL, ER);
   } else {
     constexpr int LN = 32 * ReconLanes<T>::N * kReconWarps;
-    const int groups = (rb.nlines + LN - 1) / LN;
-    constexpr int per_sm = (LIM == HARM_LIM_WENO5) ? 8 : 24;
-    int chunks = (per_sm * num_sms + groups * NPR - 1) / (groups * NPR);
-    chunks = std::max(1, std::min(chunks, nc / ((LIM == HARM_LIM_WENO5) ? 12 : 4)));
-    rb.chunk = (nc + chunks - 1) / chunks;
-    chunks = (nc + rb.chunk - 1) / rb.chunk;
+    const int groups = (rb.nlines + LN - 1) / LN, chunks = cut_marches<LIM>(rb, groups, num_sms);
     k_recon<DIR, LIM, T><<<dim3(groups, chunks, NPR), 32 * kReconWarps, 0, st>>>(d, rb, P, S, EL, ER);
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -646,6 +746,44 @@ static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const F
   int kb = 1;
   while (kb < 4 && (long long)bx * ((fb.cnt[2] + 2 * kb - 1) / (2 * kb)) >= 16LL * num_sms) kb *= 2;
   k_face<DIR, T, GT><<<dim3(bx, (fb.cnt[2] + kb - 1) / kb), kFaceThreads, 0, st>>>(d, ph, fb, EL, ER, geom, F, slot, kb);
+  launches += 2;
+  return cudaGetLastError();
+}
+
+// The three directions of a small grid, a launch per stage.
+template <int LIM, typename T, typename GT>
+static inline cudaError_t launch_flux_all(const Dims& d, const Phys& ph, const double* P, const GT* geom, T* F1, T* F2, T* F3,
+                                          unsigned long long* slots, cudaStream_t st, int num_sms,
+                                          unsigned long long& launches, const T* L, T* S, T* E) {
+  ReconAll ra{};
+  FaceAll fa{};
+  const int dirs = d.n3 > 1 ? 3 : 2;
+  for (int q = 0; q < dirs; q++) {
+    fa.fb[q] = face_box(d, q + 1);
+    fa.bx[q] = nblk((long long)fa.fb[q].cnt[0] * fa.fb[q].cnt[1], kFaceThreads);
+    fa.blocks[q] = fa.bx[q] * fa.fb[q].cnt[2];
+  }
+  ra.rb[0] = recon_box<1>(d, fa.fb[0]);
+  ra.rb[1] = recon_box<2>(d, fa.fb[1]);
+  if (dirs == 3) ra.rb[2] = recon_box<3>(d, fa.fb[2]);
+  cudaError_t e;
+  if constexpr (ReconWin<LIM>::S) {
+    for (int q = 0; q < dirs; q++) ra.blocks[q] = nblk((long long)(ra.rb[q].c1 - ra.rb[q].c0 + 1) * ra.rb[q].nlines);
+    k_recon_coef_all<LIM, T><<<ra.blocks[0] + ra.blocks[1] + ra.blocks[2], 256, 0, st>>>(d, ra, P, L, S);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    launches++;
+  }
+  const long long nseg = row_segments<LIM>(d, ra.rb[0]), items = nseg * (ra.rb[0].nlines / ra.rb[0].nt);
+  ra.dseg = fast_div((unsigned)nseg);
+  ra.blocks[0] = (unsigned)std::min<long long>((items + kReconWarps - 1) / kReconWarps, 8LL * num_sms);
+  for (int q = 1; q < dirs; q++) {
+    constexpr int LN = 32 * ReconLanes<T>::N * kReconWarps;
+    ra.groups[q] = (ra.rb[q].nlines + LN - 1) / LN;
+    ra.blocks[q] = ra.groups[q] * cut_marches<LIM>(ra.rb[q], ra.groups[q], num_sms);
+  }
+  k_recon_all<LIM, T><<<dim3(ra.blocks[0] + ra.blocks[1] + ra.blocks[2], NPR), 32 * kReconWarps, 0, st>>>(d, ra, P, S, E);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  k_face_all<T, GT><<<fa.blocks[0] + fa.blocks[1] + fa.blocks[2], kFaceThreads, 0, st>>>(d, ph, fa, E, geom, F1, F2, F3, slots);
   launches += 2;
   return cudaGetLastError();
 }
@@ -660,6 +798,8 @@ static inline cudaError_t launch_flux_dirs(const Dims& d, const Phys& ph, const 
     if ((e = launch_cellprep<LIM, T, GT>(d, ph, pb, geom, L, 0, d.n3e, st)) != cudaSuccess) return e;
     launches++;
   }
+  if (one_launch_fluxes(d, LIM, sizeof(T) == 8) && !recon_narrow<1, LIM>(d) && !recon_narrow<2, LIM>(d) && (d.n3 == 1 || !recon_narrow<3, LIM>(d)))
+    return launch_flux_all<LIM, T, GT>(d, ph, pb, geom, F1, F2, F3, slots, st, num_sms, launches, L, S, E);
   const FaceBox b1 = face_box(d, 1), b2 = face_box(d, 2), b3 = face_box(d, 3);
   if ((e = launch_flux_dir<1, LIM, T, GT>(d, ph, b1, pb, geom, F1, slots + 0, st, L, S, E, num_sms, launches)) != cudaSuccess) return e;
   if ((e = launch_flux_dir<2, LIM, T, GT>(d, ph, b2, pb, geom, F2, slots + 1, st, L, S, E, num_sms, launches)) != cudaSuccess) return e;
@@ -683,6 +823,11 @@ static inline cudaError_t launch_flux_slabs(const Dims& d, const Phys& ph, const
   const FaceBox b1 = face_box(d, 1), b2 = face_box(d, 2), b3 = face_box(d, 3);
   int f3 = b3.lo[2];  // first x3 face not launched yet
   cudaError_t e;
+  if (sw.nslab == 1) {
+    if ((e = cudaStreamWaitEvent(st, sw.ev[0], 0)) != cudaSuccess) return e;
+    if (sw.aos && hp_harm_to_soa(sw.ctx, sw.aos, sw.soa, 0, d.n3e)) return cudaErrorLaunchFailure;
+    return launch_flux_dirs<LIM, T, GT>(d, ph, pb, geom, F1, F2, F3, slots, st, num_sms, launches, L, S, E);
+  }
   for (int s = 0; s < sw.nslab; s++) {
     if ((e = cudaStreamWaitEvent(st, sw.ev[s], 0)) != cudaSuccess) return e;
     const int resident = (s + 1) * sw.planes;  // planes [0, resident) are on the device

@@ -1,8 +1,8 @@
 """The flux stage's two kernels at the edges of their ranges: lines shorter than a warp's 32 or 64,
-grids of a few cells, segments and chunks with a remainder, one plane and several, with the
-reduction of WENO5BND (a planted pressure jump) and the PARALINE flattener active.  FP64 against
-the oracle to 1e-12 of each field's largest face value; FP32 (mixed path) against the FP64 path:
-both reconstruct the same state, and a face flux carries the rounding of a few dozen FP32
+grids of a few cells, segments and chunks with a remainder, one plane and several, the directions
+in joint launches and each in its own, with the reduction of WENO5BND (a planted pressure jump) and
+the PARALINE flattener active.  FP64 against the oracle to 1e-12 of each field's largest face value;
+FP32 (mixed path) against the FP64 path: both reconstruct the same state, and a face flux carries the rounding of a few dozen FP32
 operations on the face's largest terms, of which a substep adds dt/dx < 1: 64 half-ulps of a
 field's largest value (of the state's, for the vectors, whose components share their terms)."""
 import ctypes as C
@@ -16,6 +16,9 @@ from harm_harm_b200 import HARM_PREC_FP64, HARM_PREC_MIXED, Grid, Harm
 from oracle import oracle as O
 
 SHAPES = [(5, 7, 1), (59, 9, 1), (33, 21, 6), (64, 13, 7), (131, 8, 12), (17, 70, 9)]
+# grids beyond the size up to which the three directions share their launches; (41, 45, 37) is beyond
+# it for FP64 WENO5 alone
+LARGE = [(131, 70, 33), (29, 37, 230), (790, 480, 1)]
 
 
 def _faces(g, d):
@@ -26,7 +29,7 @@ def _faces(g, d):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("lim", [0, 1, 2, 3])
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", SHAPES + LARGE + [(41, 45, 37)])
 def test_flux_edges(cuda, shape, lim):
     g, geom, conn, aux, P = make_torus(*shape, lim=lim)
     plant_compression(g, P)
