@@ -27,6 +27,9 @@ static int seterr_msg(const char* msg, int code) {
   return code;
 }
 
+// places of d_scal (in doubles) that calls read back
+enum { SC_DT = 8, SC_NDT = 9, SC_STATS = 16, SC_STATUS = 28 };
+
 int hb_setmsg(const char* msg, int code) { return seterr_msg(msg, code); }
 
 extern "C" const char* harm_b200_last_error(void) { return g_errbuf; }
@@ -92,13 +95,13 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   CK(cudaMalloc(&c->d_scal, 64 * sizeof(double)));
   CK(cudaMemset(c->d_scal, 0, 64 * sizeof(double)));
   c->d_dtslots = (unsigned long long*)(c->d_scal + 0);  // 6 slots
-  c->d_dt = c->d_scal + 8;
-  c->d_ndt = c->d_scal + 9;                             // 2
-  c->d_stats = c->d_scal + 16;                          // 5
+  c->d_dt = c->d_scal + SC_DT;
+  c->d_ndt = c->d_scal + SC_NDT;                        // 2
+  c->d_stats = c->d_scal + SC_STATS;                    // 5
   c->d_nrec = (unsigned int*)(c->d_scal + 24);
   c->d_nrare = (unsigned int*)(c->d_scal + 25);
   c->d_nhard = (unsigned int*)(c->d_scal + 26);
-  c->d_status = (unsigned int*)(c->d_scal + 28);
+  c->d_status = (unsigned int*)(c->d_scal + SC_STATUS);
   {
     // FP32 flux tiles: plain coalesced loads (default) or TMA ("tma"); both feed the same
     // arithmetic.  The TMA-staged kernel measured slower on B200 (it needs ~120 registers for
@@ -254,10 +257,18 @@ static int substep(harm_ctx* c, int precision, int guess, int timeorder, int num
   return hp_update_mixed(c, sc, d_pi, d_pb, d_pf, d_pflag, st);
 }
 
-// the device error word, read after a synchronisation (it is cleared when reported)
+// What a call reads back, in one copy at its end: h_scal[SC_DT ..] then mirrors d_scal's dt, ndt,
+// statistics and error word (as three copies, the error word's a synchronous one, a substep of a
+// 24x20 grid took 120 us instead of 102).
+static cudaError_t read_back(harm_ctx* c) {
+  return cudaMemcpyAsync(c->h_scal + SC_DT, c->d_scal + SC_DT, (SC_STATUS + 1 - SC_DT) * sizeof(double),
+                         cudaMemcpyDeviceToHost, c->stream);
+}
+
+// the device error word of the last read_back, after a synchronisation (it is cleared when reported)
 static int check_status(harm_ctx* c) {
   unsigned int st = 0;
-  CK(cudaMemcpy(&st, c->d_status, sizeof(st), cudaMemcpyDeviceToHost));
+  memcpy(&st, c->h_scal + SC_STATUS, sizeof(st));
   if (st) {
     CK(cudaMemset(c->d_status, 0, sizeof(st)));
     if (st & 1u) return seterr_msg("a flux tile's TMA load did not complete (the step's fluxes are incomplete)", 5);
@@ -268,13 +279,13 @@ static int check_status(harm_ctx* c) {
 
 static void add_stats(harm_ctx* c, harm_stats* stats, double inverted, int guess) {
   if (!stats) return;
-  stats->newton_iters += c->h_scal[8];
+  stats->newton_iters += c->h_scal[SC_STATS];
   stats->cells_inverted += inverted;
   // the gated engine counts the cells it gives the learned start; the others give it to all
-  if (guess == HARM_GUESS_MLP) stats->mlp_cells += (c->mlp_tc == 4) ? c->h_scal[9] : inverted;
-  stats->mlp_fallbacks += c->h_scal[10];
-  stats->inversion_failures += c->h_scal[11];
-  stats->floor_hits += c->h_scal[12];
+  if (guess == HARM_GUESS_MLP) stats->mlp_cells += (c->mlp_tc == 4) ? c->h_scal[SC_STATS + 1] : inverted;
+  stats->mlp_fallbacks += c->h_scal[SC_STATS + 2];
+  stats->inversion_failures += c->h_scal[SC_STATS + 3];
+  stats->floor_hits += c->h_scal[SC_STATS + 4];
 }
 
 extern "C" int harm_b200_advance(harm_ctx* c, int precision, int guess, int timeorder, int numtimeorders,
@@ -299,11 +310,10 @@ extern "C" int harm_b200_advance(harm_ctx* c, int precision, int guess, int time
     return 1;
   if (hp_copy_ghosts(c, d_pb, d_pf)) return 1;
   if (hp_finalize_dt(c, nullptr, c->d_ndt, 1)) return 1;
-  CK(cudaMemcpyAsync(c->h_scal + 1, c->d_ndt, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(c->h_scal + 8, c->d_stats, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  CK(read_back(c));
   CK(cudaStreamSynchronize(c->stream));
   if (int rc = check_status(c)) return rc;
-  if (ndt) *ndt = c->h_scal[1];
+  if (ndt) *ndt = c->h_scal[SC_NDT];
   add_stats(c, stats, (double)d.n1 * d.n2 * d.n3, guess);
   return 0;
 }
@@ -327,11 +337,10 @@ extern "C" int harm_b200_advance_u(harm_ctx* c, int precision, int guess, int ti
     return 1;
   if (hp_copy_ghosts(c, d_pb, d_pf)) return 1;
   if (hp_finalize_dt(c, nullptr, c->d_ndt, 1)) return 1;
-  CK(cudaMemcpyAsync(c->h_scal + 1, c->d_ndt, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(c->h_scal + 8, c->d_stats, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  CK(read_back(c));
   CK(cudaStreamSynchronize(c->stream));
   if (int rc = check_status(c)) return rc;
-  if (ndt) *ndt = c->h_scal[1];
+  if (ndt) *ndt = c->h_scal[SC_NDT];
   add_stats(c, stats, (double)d.n1 * d.n2 * d.n3, guess);
   return 0;
 }
@@ -369,11 +378,10 @@ extern "C" int harm_b200_step_n(harm_ctx* c, int precision, int guess, double* d
   if (stats) CK(cudaMemsetAsync(c->d_stats, 0, 5 * sizeof(double), c->stream));
   for (int s = 0; s < nsteps; s++)
     if (enqueue_step(c, precision, guess, d_P, stats != nullptr)) return 1;
-  CK(cudaMemcpyAsync(c->h_scal, c->d_dt, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (stats) CK(cudaMemcpyAsync(c->h_scal + 8, c->d_stats, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  CK(read_back(c));
   CK(cudaStreamSynchronize(c->stream));
   if (int rc = check_status(c)) return rc;
-  *dt = c->h_scal[0];
+  *dt = c->h_scal[SC_DT];
   add_stats(c, stats, 2.0 * nsteps * (double)d.n1 * d.n2 * d.n3, guess);
   return 0;
 }
@@ -456,11 +464,10 @@ static int step_host(harm_ctx* c, int precision, int guess, double* h_P, double*
   } else {
     CK(cudaMemcpyAsync(h_P, c->d_Pdev, bytes, cudaMemcpyDeviceToHost, c->stream));
   }
-  CK(cudaMemcpyAsync(c->h_scal, c->d_dt, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (stats) CK(cudaMemcpyAsync(c->h_scal + 8, c->d_stats, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  CK(read_back(c));
   CK(cudaStreamSynchronize(c->stream));
   if (int rc = check_status(c)) return rc;
-  *dt = c->h_scal[0];
+  *dt = c->h_scal[SC_DT];
   add_stats(c, stats, 2.0 * (double)d.n1 * d.n2 * d.n3, guess);
   return 0;
 }
@@ -510,12 +517,11 @@ extern "C" int harm_b200_step_host_n(harm_ctx* c, int precision, int guess, doub
     if (enqueue_step(c, precision, guess, c->d_Pdev, stats != nullptr, &sw)) return 1;
     if (int rc = d2h_slabs(c, h_P)) return rc;
   }
-  CK(cudaMemcpyAsync(c->h_scal, c->d_dt, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (stats) CK(cudaMemcpyAsync(c->h_scal + 8, c->d_stats, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  CK(read_back(c));
   CK(cudaStreamSynchronize(c->stream));
   CK(cudaStreamSynchronize(c->d2h_stream));
   if (int rc = check_status(c)) return rc;
-  *dt = c->h_scal[0];
+  *dt = c->h_scal[SC_DT];
   add_stats(c, stats, 2.0 * nsteps * (double)d.n1 * d.n2 * d.n3, guess);
   return 0;
 }
@@ -598,6 +604,7 @@ extern "C" int harm_b200_time_stages(harm_ctx* c, int precision, int guess, cons
     }
   }
   CK(cudaMemsetAsync(c->d_dtslots, 0xFF, 6 * sizeof(unsigned long long), c->stream));
+  CK(read_back(c));
   CK(cudaStreamSynchronize(c->stream));
   return check_status(c);
 }
