@@ -55,12 +55,26 @@ __device__ __forceinline__ void load_geo(const S* __restrict__ tab, size_t plane
   g.igdet = (T)tab_ld<LDG>(tab + (size_t)HARM_G_IGDET * plane + c);
 }
 
-// HARM_INVERT_FAST_DIV (harm_path_mixed.cu, harm_path_fp64fma.cu): the FP64 divisions of the
-// inversion and of the cell states by the hardware's reciprocal approximation refined by two
-// Newton-Raphson steps (r <- r + r (1 - b r), quadratic convergence from the approximation's
-// relative error) and a multiply: within an ulp or two of the IEEE quotients for normal operands,
-// with fewer FP64 instructions.  Otherwise IEEE FP64 division (the operations of the C
-// restatement, so the FP64 path matches it to round-off).
+// a/b from b's correctly rounded reciprocal y (P. Markstein, IBM J. Res. Dev. 34, 1990): the
+// quotient estimate q = a y corrected by its exact remainder, q + (a - b q) y.  The corrected
+// value is a/b to within 2^-52 ulp before its rounding, so it is the IEEE quotient unless a/b
+// lies that close to the middle of two doubles (b normal, no overflow or underflow; a = 0
+// gives 0).  Three operations against the dozen of a division: the WENO sums divide several
+// values by one denominator, and several by constants.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+
+// HARM_INVERT_FAST_DIV (harm_path_mixed.cu, harm_path_fp64fma.cu): FP64 divisions by the
+// hardware's reciprocal approximation refined by two Newton-Raphson steps (r <- r + r (1 - b r),
+// quadratic convergence from the approximation's relative error).  frcp and fdiv, inside the
+// Newton iteration of the inversion, whose steps correct one another: within an ulp or two of the
+// IEEE quotients for normal operands.  sdiv, in the cell states and in the inversion's setup and
+// result: corrected by the quotient's remainder (div_by, with y an ulp or so off: the IEEE quotient
+// but for a/b within some 2^-52 ulp of a midpoint), so that those values are what IEEE division
+// gives.  Otherwise IEEE FP64 division (the operations of the C restatement, so the FP64 path
+// matches it to round-off).
 #ifdef HARM_INVERT_FAST_DIV
 constexpr bool kFastDiv = true;
 __device__ __forceinline__ double frcp(double b) {
@@ -72,23 +86,14 @@ __device__ __forceinline__ double frcp(double b) {
   return fma(r, e, r);
 }
 __device__ __forceinline__ double fdiv(double a, double b) { return a * frcp(b); }
+__device__ __forceinline__ double sdiv(double a, double b) { return div_by(a, b, frcp(b)); }
 #else
 constexpr bool kFastDiv = false;
 __device__ __forceinline__ double frcp(double b) { return 1.0 / b; }
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
+__device__ __forceinline__ double sdiv(double a, double b) { return a / b; }
 #endif
-__device__ __forceinline__ float fdiv(float a, float b) { return a / b; }
-
-// a/b from b's correctly rounded reciprocal y (P. Markstein, IBM J. Res. Dev. 34, 1990): the
-// quotient estimate q = a y corrected by its exact remainder, q + (a - b q) y.  The corrected
-// value is a/b to within 2^-52 ulp before its rounding, so it is the IEEE quotient unless a/b
-// lies that close to the middle of two doubles (b normal, no overflow or underflow; a = 0
-// gives 0).  Three operations against the dozen of a division: the WENO sums divide several
-// values by one denominator, and several by constants.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q = a * y;
-  return fma(fma(-b, q, a), y, q);
-}
+__device__ __forceinline__ float sdiv(float a, float b) { return a / b; }
 
 // The reciprocals of several values from one division, each corrected by its own remainder (so,
 // as div_by's quotients, the IEEE value but for operands within 1e-15 of a midpoint): b's values
@@ -169,7 +174,7 @@ __device__ __forceinline__ void ucon_of(const T* pr, const Geo<T>& g, T* ucon, T
   q = (q >= T(0)) ? q : T(0);
   qsq = q;
   gamma = sqrt(T(1) + q);
-  ucon[0] = fdiv(gamma, g.alpha);
+  ucon[0] = sdiv(gamma, g.alpha);
   ucon[1] = pr[HARM_U1] - ucon[0] * g.beta1;
   ucon[2] = pr[HARM_U2] - ucon[0] * g.beta2;
   ucon[3] = pr[HARM_U3] - ucon[0] * g.beta3;
@@ -193,10 +198,10 @@ __device__ __forceinline__ void get_state(const T* pr, const Geo<T>& g, T gam, S
   lower(q.ucon, g, q.ucov);
   T ud0tilde = pr[HARM_U1] * g.gcov[1] + pr[HARM_U2] * g.gcov[2] + pr[HARM_U3] * g.gcov[3];
   T alphasq = g.alpha * g.alpha;
-  q.plus1ud0 = ud0tilde + fdiv(g.gcovpert_tt - alphasq * (g.betasqoalphasq + q.qsq), T(1) + q.gamma * g.alpha);
+  q.plus1ud0 = ud0tilde + sdiv(g.gcovpert_tt - alphasq * (g.betasqoalphasq + q.qsq), T(1) + q.gamma * g.alpha);
   T Bcov[4], Bsq, udotB;
   bdots(pr, g, q.ucov, Bcov, Bsq, udotB);
-  q.bsq = fdiv(Bsq + udotB * udotB, q.ucon[0] * q.ucon[0]);
+  q.bsq = sdiv(Bsq + udotB * udotB, q.ucon[0] * q.ucon[0]);
   q.pressure = (gam - T(1)) * pr[HARM_UU];
 }
 
@@ -219,7 +224,7 @@ __device__ __forceinline__ void primtoflux(const T* pr, const State<T>& q, int d
   for (int mu = 0; mu < 4; mu++)
     em[mu] = Bsq * ud * q.ucov[mu] - Bd * Bcov[mu] - udotB * (Bd * q.ucov[mu] + Bcov[mu] * ud);
   em[dir] += T(0.5) * (Bsq + udotB * udotB);
-  const T ig2 = fdiv(T(1), q.ucon[0] * q.ucon[0]);
+  const T ig2 = sdiv(T(1), q.ucon[0] * q.ucon[0]);
   F[HARM_RHO] = rho * ud * gd;
 #pragma unroll
   for (int mu = 0; mu < 4; mu++) F[HARM_UU + mu] = (ma[mu] + em[mu] * ig2) * gd;

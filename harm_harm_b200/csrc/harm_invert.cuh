@@ -30,8 +30,9 @@ constexpr double kBIG = 1.e100;
 constexpr double kSQRTMIN = 1.4916681462400413e-154;
 constexpr double kSMALL = 1e-300;
 
-// The divisions are fdiv and frcp (harm_device.cuh): IEEE, or on the mixed path the refined
-// hardware reciprocal, shared between the divisions of one residual evaluation.
+// The divisions of the iteration are fdiv and frcp (harm_device.cuh): IEEE, or on the mixed and the
+// FP64 FMA path the refined hardware reciprocal, shared between the divisions of one residual
+// evaluation; those of the setup and the result are sdiv.
 __device__ __forceinline__ double utsq_calc(double W, const InvC& c) {
   double SoW = fdiv(c.QdotB, W);
   double top = c.Qtsq + (c.Bsq + 2.0 * W) * SoW * SoW;
@@ -50,12 +51,15 @@ __device__ __forceinline__ bool coldgrhd(double Qtsq, double D, double& Wp) {
 
 // residual, derivative and Newton step of the hot (E') or cold (P^2) equation
 __device__ __forceinline__ void inv_func(double Wp, const InvC& c, double& resid, double& jac, double& dx, double& f) {
-  if (kFastDiv && !c.cold) {
+  const double Wf = Wp + c.D, Xf = c.Bsq + Wf + kSMALL;
+  // (below, powers of W up to the fourth and of W X up to the third are formed: values beyond
+  // 1e-50 .. 1e50 are left to the divisions further down)
+  if (kFastDiv && !c.cold && Wf > 1e-50 && Xf < 1e50) {
     // The same residual and derivative with four reciprocals instead of the twelve divisions:
     // utsq with numerator and denominator times W^2 (no quotient inside the quotient), one
     // reciprocal for W and X together and one for gamma^2 and 1 + gamma (k_invert<1> at
     // 256x128x64: 248 -> 223 us; compiled for 2 or 4 blocks per SM instead of 3 it is the same).
-    const double W = Wp + c.D, X = c.Bsq + W + kSMALL, W2 = W * W, Y = fma(2.0, W, c.Bsq);
+    const double W = Wf, X = Xf, W2 = W * W, Y = fma(2.0, W, c.Bsq);
     const double bq = c.QdotBsq * Y;
     const double utsq = fma(c.Qtsq, W2, bq) * frcp(fma(fma(c.Bsq + X, W, fma(c.Bsq, c.Bsq, -c.Qtsq)), W2, -bq));
     const double iWX = frcp(W * X), iX = iWX * W, iX2 = iX * iX, iX3 = iX2 * iX;
@@ -230,7 +234,7 @@ static __device__ __forceinline__ void inv_invariants(const double* U, const Geo
   c.QdotB = Qcov[1] * Bcon[1] + Qcov[2] * Bcon[2] + Qcov[3] * Bcon[3];
   c.QdotBsq = c.QdotB * c.QdotB;
   double alpha = g.alpha, alphasq = alpha * alpha;
-  double Dfactor = fdiv(-g.gcovpert_tt + alphasq * g.betasqoalphasq, alphasq + alpha);
+  double Dfactor = sdiv(-g.gcovpert_tt + alphasq * g.betasqoalphasq, alphasq + alpha);
   c.Qdotnp = Qconp[0] * ncov[0] + c.D * Dfactor;
 }
 
@@ -245,14 +249,14 @@ static __device__ int inv_setup(const double* U, const Geo<double>& g, const dou
     for (int j = 1; j < 4; j++) utsq += g.gcov[sym(i, j)] * prim[HARM_U1 + i - 1] * prim[HARM_U1 + j - 1];
   if ((utsq < 0.) && (fabs(utsq) < fabs(-0.9 * c.utsq_too_big))) utsq = 0.0;
   if (!(utsq >= 0. && utsq < c.utsq_too_big)) utsq = 0.0;
-  double gammasq = 1. + utsq, gamma = sqrt(gammasq), rho0 = fdiv(c.D, gamma), u = prim[HARM_UU];
+  double gammasq = 1. + utsq, gamma = sqrt(gammasq), rho0 = sdiv(c.D, gamma), u = prim[HARM_UU];
   double p = (c.gam - 1.) * u;
   double bc[4] = {0.0, prim[HARM_B1], prim[HARM_B2], prim[HARM_B3]}, bcv[4];
   lower(bc, g, bcv);
   double bsq = bc[1] * bcv[1] + bc[2] * bcv[2] + bc[3] * bcv[3];
-  bsq *= fdiv(g.alpha * g.alpha, gammasq);
-  Wp_last = fdiv(c.D * utsq, 1.0 + gamma) + (u + p) * gammasq;
-  double Wpabs = fdiv(fabs(c.D * utsq), 1.0 + fabs(gamma)) + (fabs(u) + fabs(p)) * fabs(gammasq) + kSQRTMIN;
+  bsq *= sdiv(g.alpha * g.alpha, gammasq);
+  Wp_last = sdiv(c.D * utsq, 1.0 + gamma) + (u + p) * gammasq;
+  double Wpabs = sdiv(fabs(c.D * utsq), 1.0 + fabs(gamma)) + (fabs(u) + fabs(p)) * fabs(gammasq) + kSQRTMIN;
   double etaabs = fabs(rho0) + (fabs(u) + fabs(p) + fabs(bsq));
   c.w2 = 1e2 * fabs(rho0);
   if (gammasq * etaabs >= c.w2) {
@@ -292,11 +296,11 @@ static __device__ int inv_verify_guess(double& Wp_last, const InvC& c, int8_t& f
 static __device__ int inv_finish(double Wp, const InvC& c, const double* Qtcon, const double* Bcon, double* prim, int8_t& flag) {
   if (Wp == kBIG) flag = HARM_UTOPRIMFAILCONVRET + 1;
   else if (Wp <= -(c.D)) flag = HARM_UTOPRIMFAILCONVRET + 1;
-  else if (fdiv(Wp, c.w1) > c.gsq_too_big) flag = HARM_UTOPRIMFAILCONVW;
+  else if (Wp / c.w1 > c.gsq_too_big) flag = HARM_UTOPRIMFAILCONVW;
   double W = Wp + c.D;
   double utsq = utsq_calc(W, c), gammasq = 1.0 + utsq, gamma = sqrt(gammasq);
-  double wmrho0 = fdiv(Wp - fdiv(c.D * utsq, 1.0 + gamma), gammasq);
-  double rho0 = fdiv(c.D, gamma);
+  double wmrho0 = sdiv(Wp - sdiv(c.D * utsq, 1.0 + gamma), gammasq);
+  double rho0 = sdiv(c.D, gamma);
   double p = ((c.gam - 1.0) / c.gam) * wmrho0, u = wmrho0 - p;
   if ((rho0 <= 0.) || ((p < 0.) && !c.cold)) {
     if ((rho0 <= 0.) && (p >= 0.)) flag = HARM_UTOPRIMFAILRHONEG;
@@ -307,7 +311,7 @@ static __device__ int inv_finish(double Wp, const InvC& c, const double* Qtcon, 
   out[0] = rho0;
   out[1] = c.cold ? 0.0 : u;
 #pragma unroll
-  for (int i = 1; i < 4; i++) out[1 + i] = fdiv(gamma, W + c.Bsq) * (Qtcon[i] + fdiv(c.QdotB * Bcon[i], W));
+  for (int i = 1; i < 4; i++) out[1 + i] = sdiv(gamma, W + c.Bsq) * (Qtcon[i] + sdiv(c.QdotB * Bcon[i], W));
   bool nan = false;
 #pragma unroll
   for (int i = 0; i < 5; i++) nan |= !isfinite(out[i]);
