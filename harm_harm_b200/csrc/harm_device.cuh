@@ -94,6 +94,14 @@ __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ double sdiv(double a, double b) { return a / b; }
 #endif
 __device__ __forceinline__ float sdiv(float a, float b) { return a / b; }
+// sdiv with an approximate reciprocal y of b at hand (a few ulp do: the correction squares its error)
+__device__ __forceinline__ double sdiv(double a, double b, double y) { return kFastDiv ? div_by(a, b, y) : a / b; }
+// approximate reciprocals of two values from one (their product in range)
+__device__ __forceinline__ void frcp2(double b0, double b1, double& y0, double& y1) {
+  const double r = kFastDiv ? frcp(b0 * b1) : 0.0;
+  y0 = r * b1;
+  y1 = r * b0;
+}
 
 // The reciprocals of several values from one division, each corrected by its own remainder (so,
 // as div_by's quotients, the IEEE value but for operands within 1e-15 of a midpoint): b's values

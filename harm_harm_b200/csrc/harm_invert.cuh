@@ -51,18 +51,16 @@ __device__ __forceinline__ bool coldgrhd(double Qtsq, double D, double& Wp) {
 
 // residual, derivative and Newton step of the hot (E') or cold (P^2) equation
 __device__ __forceinline__ void inv_func(double Wp, const InvC& c, double& resid, double& jac, double& dx, double& f) {
-  const double Wf = Wp + c.D, Xf = c.Bsq + Wf + kSMALL;
-  // (below, powers of W up to the fourth and of W X up to the third are formed: values beyond
-  // 1e-50 .. 1e50 are left to the divisions further down)
-  if (kFastDiv && !c.cold && Wf > 1e-50 && Xf < 1e50) {
-    // The same residual and derivative with four reciprocals instead of the twelve divisions:
-    // utsq with numerator and denominator times W^2 (no quotient inside the quotient), one
-    // reciprocal for W and X together and one for gamma^2 and 1 + gamma (k_invert<1> at
-    // 256x128x64: 248 -> 223 us; compiled for 2 or 4 blocks per SM instead of 3 it is the same).
-    const double W = Wf, X = Xf, W2 = W * W, Y = fma(2.0, W, c.Bsq);
-    const double bq = c.QdotBsq * Y;
-    const double utsq = fma(c.Qtsq, W2, bq) * frcp(fma(fma(c.Bsq + X, W, fma(c.Bsq, c.Bsq, -c.Qtsq)), W2, -bq));
-    const double iWX = frcp(W * X), iX = iWX * W, iX2 = iX * iX, iX3 = iX2 * iX;
+  if (kFastDiv && !c.cold) {
+    // The same residual and derivative with four reciprocals instead of the twelve divisions: one
+    // for W and X together and one for gamma^2 and 1 + gamma (k_invert<1> at 256x128x64, setup and
+    // result included: 248 -> 203 us; compiled for 2 or 4 blocks per SM instead of 3 it is the
+    // same).  No power beyond those of the divisions it replaces: with utsq times W^2 above and
+    // below and (W X)^3 in dv^2 it takes 3 us less, but states of W below 1e-52 do not invert.
+    const double W = Wp + c.D, X = c.Bsq + W + kSMALL;
+    const double iWX = frcp(W * X), iX = iWX * W, iW = iWX * X, iX2 = iX * iX, iX3 = iX2 * iX, iW2 = iW * iW;
+    const double BW = c.QdotBsq * iW2, Y = fma(2.0, W, c.Bsq);
+    const double utsq = fma(Y, BW, c.Qtsq) * frcp(fma(-Y, BW, fma(X, X, -c.Qtsq)));
     const double gammasq = 1.0 + utsq, gamma = sqrt(gammasq), gp1 = 1.0 + gamma;
     const double ig = frcp(gammasq * gp1), igsq = ig * gp1;
     const double wmrho0 = (Wp - c.D * utsq * (ig * gammasq)) * igsq;
@@ -75,7 +73,7 @@ __device__ __forceinline__ void inv_func(double Wp, const InvC& c, double& resid
     const double BQ = c.Bsq * c.Qtsq - c.QdotBsq;
     double Ep = c.Qdotnp + Wp - pofchi + 0.5 * c.Bsq + 0.5 * BQ * iX2;
     if (pofchi != pofchi || Ep != Ep) Ep = -kVERYBIG;
-    const double dvsq = -2.0 * (iWX * iWX * iWX) * (c.Qtsq * (W2 * W) + c.QdotBsq * (3.0 * W * X + c.Bsq * c.Bsq));
+    const double dvsq = -2.0 * iX3 * fma(BW * iW, fma(3.0 * W, X, c.Bsq * c.Bsq), c.Qtsq);
     const double dpdvsq = (c.D * (gamma * 0.5 - 1.0) - Wp) * dpdchi;
     double dE = (1.0 - (igsq * dpdchi + dpdvsq * dvsq)) - BQ * iX3;
     if (dE != dE) dE = 0.0;
@@ -249,14 +247,17 @@ static __device__ int inv_setup(const double* U, const Geo<double>& g, const dou
     for (int j = 1; j < 4; j++) utsq += g.gcov[sym(i, j)] * prim[HARM_U1 + i - 1] * prim[HARM_U1 + j - 1];
   if ((utsq < 0.) && (fabs(utsq) < fabs(-0.9 * c.utsq_too_big))) utsq = 0.0;
   if (!(utsq >= 0. && utsq < c.utsq_too_big)) utsq = 0.0;
-  double gammasq = 1. + utsq, gamma = sqrt(gammasq), rho0 = sdiv(c.D, gamma), u = prim[HARM_UU];
+  double gammasq = 1. + utsq, gamma = sqrt(gammasq), yg, y1, u = prim[HARM_UU];
+  frcp2(gamma, 1.0 + gamma, yg, y1);
+  double rho0 = sdiv(c.D, gamma, yg);
   double p = (c.gam - 1.) * u;
   double bc[4] = {0.0, prim[HARM_B1], prim[HARM_B2], prim[HARM_B3]}, bcv[4];
   lower(bc, g, bcv);
   double bsq = bc[1] * bcv[1] + bc[2] * bcv[2] + bc[3] * bcv[3];
-  bsq *= sdiv(g.alpha * g.alpha, gammasq);
-  Wp_last = sdiv(c.D * utsq, 1.0 + gamma) + (u + p) * gammasq;
-  double Wpabs = sdiv(fabs(c.D * utsq), 1.0 + fabs(gamma)) + (fabs(u) + fabs(p)) * fabs(gammasq) + kSQRTMIN;
+  bsq *= sdiv(g.alpha * g.alpha, gammasq, yg * yg);
+  const double Wpk = sdiv(c.D * utsq, 1.0 + gamma, y1);
+  Wp_last = Wpk + (u + p) * gammasq;
+  double Wpabs = fabs(Wpk) + (fabs(u) + fabs(p)) * gammasq + kSQRTMIN;
   double etaabs = fabs(rho0) + (fabs(u) + fabs(p) + fabs(bsq));
   c.w2 = 1e2 * fabs(rho0);
   if (gammasq * etaabs >= c.w2) {
@@ -296,11 +297,14 @@ static __device__ int inv_verify_guess(double& Wp_last, const InvC& c, int8_t& f
 static __device__ int inv_finish(double Wp, const InvC& c, const double* Qtcon, const double* Bcon, double* prim, int8_t& flag) {
   if (Wp == kBIG) flag = HARM_UTOPRIMFAILCONVRET + 1;
   else if (Wp <= -(c.D)) flag = HARM_UTOPRIMFAILCONVRET + 1;
-  else if (Wp / c.w1 > c.gsq_too_big) flag = HARM_UTOPRIMFAILCONVW;
+  else if (kFastDiv ? Wp > c.gsq_too_big * c.w1 : Wp / c.w1 > c.gsq_too_big) flag = HARM_UTOPRIMFAILCONVW;
   double W = Wp + c.D;
   double utsq = utsq_calc(W, c), gammasq = 1.0 + utsq, gamma = sqrt(gammasq);
-  double wmrho0 = sdiv(Wp - sdiv(c.D * utsq, 1.0 + gamma), gammasq);
-  double rho0 = sdiv(c.D, gamma);
+  double yg, y1, yX, yW;
+  frcp2(gamma, 1.0 + gamma, yg, y1);
+  frcp2(W + c.Bsq, W, yX, yW);
+  double wmrho0 = sdiv(Wp - sdiv(c.D * utsq, 1.0 + gamma, y1), gammasq, yg * yg);
+  double rho0 = sdiv(c.D, gamma, yg);
   double p = ((c.gam - 1.0) / c.gam) * wmrho0, u = wmrho0 - p;
   if ((rho0 <= 0.) || ((p < 0.) && !c.cold)) {
     if ((rho0 <= 0.) && (p >= 0.)) flag = HARM_UTOPRIMFAILRHONEG;
@@ -311,7 +315,7 @@ static __device__ int inv_finish(double Wp, const InvC& c, const double* Qtcon, 
   out[0] = rho0;
   out[1] = c.cold ? 0.0 : u;
 #pragma unroll
-  for (int i = 1; i < 4; i++) out[1 + i] = sdiv(gamma, W + c.Bsq) * (Qtcon[i] + sdiv(c.QdotB * Bcon[i], W));
+  for (int i = 1; i < 4; i++) out[1 + i] = sdiv(gamma, W + c.Bsq, yX) * (Qtcon[i] + sdiv(c.QdotB * Bcon[i], W, yW));
   bool nan = false;
 #pragma unroll
   for (int i = 0; i < 5; i++) nan |= !isfinite(out[i]);
