@@ -118,6 +118,9 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
               : (m && strcmp(m, "mma-fused") == 0) ? 3 : (m && strcmp(m, "mma") == 0) ? 0 : 4;
     c->mlp_gate = mlp_gate;
     CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
+    int pitch = 0;
+    CK(cudaDeviceGetAttribute(&pitch, cudaDevAttrMaxPitch, device));
+    c->max_pitch = (size_t)pitch;
   }
   CK(cudaMemset(c->d_dtslots, 0xFF, 6 * sizeof(unsigned long long)));
   CK(cudaMallocHost(&c->h_scal, 64 * sizeof(double)));
@@ -398,9 +401,20 @@ static int slab_planes(const harm_ctx* c) {
   return std::max((c->g.n3e + HARM_H2D_SLABS - 1) / HARM_H2D_SLABS, least);
 }
 
-// H2D of the state in at most HARM_H2D_SLABS slabs of k-planes (one two-dimensional copy per
-// slab, followed by an event) on the copy stream, after the context
-// stream's earlier work
+// the slab of every primitive, in one copy of eight rows of a primitive's pitch, or row by row
+// where the pitch is beyond a two-dimensional copy's (2^31 - 1 bytes: 268 million cells)
+static cudaError_t copy_slab(const harm_ctx* c, double* dst, const double* src, size_t off, size_t bytes, cudaMemcpyKind kind,
+                             cudaStream_t st) {
+  const size_t pitch = c->cells * sizeof(double);
+  if (pitch <= c->max_pitch) return cudaMemcpy2DAsync(dst + off, pitch, src + off, pitch, bytes, NPR, kind, st);
+  cudaError_t e = cudaSuccess;
+  for (size_t p = 0; p < NPR && e == cudaSuccess; p++)
+    e = cudaMemcpyAsync(dst + p * c->cells + off, src + p * c->cells + off, bytes, kind, st);
+  return e;
+}
+
+// H2D of the state in at most HARM_H2D_SLABS slabs of k-planes (copy_slab, followed by an event)
+// on the copy stream, after the context stream's earlier work
 // harm_layout: h_P is in HARM's [k][j][i][pl] layout (one copy per slab into d_Paos, converted
 // into d_Pdev on the context stream after the slab's event)
 // after_slab (optional): per slab, an event the slab's copy waits for (the previous step's
@@ -424,9 +438,7 @@ static int h2d_slabs(harm_ctx* c, const double* h_P, SlabWait* sw, bool harm_lay
     if (harm_layout) {
       CK(cudaMemcpyAsync(c->d_Paos + NPR * off, h_P + NPR * off, NPR * bytes, cudaMemcpyHostToDevice, c->copy_stream));
     } else {
-      // the slab of every primitive in one copy: eight rows of a primitive's pitch
-      const size_t pitch = c->cells * sizeof(double);
-      CK(cudaMemcpy2DAsync(c->d_Pdev + off, pitch, h_P + off, pitch, bytes, NPR, cudaMemcpyHostToDevice, c->copy_stream));
+      CK(copy_slab(c, c->d_Pdev, h_P, off, bytes, cudaMemcpyHostToDevice, c->copy_stream));
     }
     CK(cudaEventRecord(c->slab_ev[s], c->copy_stream));
   }
@@ -488,8 +500,7 @@ static int d2h_slabs(harm_ctx* c, double* h_P) {
   for (int s = 0; s < nslab; s++) {
     const int z0 = s * planes, z1 = (z0 + planes < n3e) ? z0 + planes : n3e;
     const size_t off = (size_t)z0 * c->plane, bytes = (size_t)(z1 - z0) * c->plane * sizeof(double);
-    const size_t pitch = c->cells * sizeof(double);
-    CK(cudaMemcpy2DAsync(h_P + off, pitch, c->d_Pdev + off, pitch, bytes, NPR, cudaMemcpyDeviceToHost, c->d2h_stream));
+    CK(copy_slab(c, h_P, c->d_Pdev, off, bytes, cudaMemcpyDeviceToHost, c->d2h_stream));
     CK(cudaEventRecord(c->d2h_ev[s], c->d2h_stream));
   }
   return 0;

@@ -32,6 +32,7 @@ struct harm_ctx {
   cudaEvent_t d2h_ev[HARM_H2D_SLABS];   // recorded on d2h_stream after each slab
   cudaEvent_t done_ev;                  // recorded on stream when a step's state is final
   size_t plane, cells;
+  size_t max_pitch;                     // of a two-dimensional copy
   // metric tables (FP64, plus an FP32 copy for the mixed-precision flux path)
   double* d_geom;
   float* d_geomf;
