@@ -76,12 +76,16 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   }
   c->d_edge = (double*)c->d_flux + 3 * nf;
   c->d_edgef = (float*)c->d_flux + 3 * nf;
-  CK(cudaMalloc(&c->d_emf, 3 * d.cells * sizeof(double)));
-  c->d_emff = (float*)c->d_emf;
-  if (g->lim == HARM_LIM_WENO5 || g->lim == HARM_LIM_PARALINE) {
-    const size_t nl = (g->lim == HARM_LIM_WENO5 ? 9 : 4) * d.cells;
-    CK(cudaMalloc(&c->d_line, (nl + ndir * d.cells) * sizeof(double)));
-    c->d_coef = (double*)c->d_line + nl;
+  // the cell pass of the flux stage, the EMFs and post_fixup's records: each is read for the last
+  // time before the next is written, so they share their memory
+  const size_t nl = (g->lim == HARM_LIM_WENO5) ? 9 : (g->lim == HARM_LIM_PARALINE) ? 4 : 0;
+  c->fix_cap = (unsigned int)std::min<size_t>((size_t)d.n1 * d.n2 * d.n3, 0xFFFFFFF0u);
+  CK(cudaMalloc(&c->d_shared, std::max(std::max(nl, (size_t)3) * d.cells * sizeof(double), c->fix_cap * sizeof(FixRec))));
+  c->d_line = c->d_fixrec = c->d_shared;
+  c->d_emf = (double*)c->d_shared;
+  c->d_emff = (float*)c->d_shared;
+  if (nl) {
+    CK(cudaMalloc(&c->d_coef, ndir * d.cells * sizeof(double)));
     // read (and not used) at ghost cells that no pass writes
     CK(cudaMemset(c->d_coef, 0, ndir * d.cells * sizeof(double)));
   }
@@ -90,8 +94,6 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   CK(cudaMalloc(&c->d_rare, (size_t)d.n1 * d.n2 * d.n3 * sizeof(unsigned int)));
   CK(cudaMalloc(&c->d_pflag, d.cells));
   CK(cudaMemset(c->d_pflag, 0, d.cells));
-  c->fix_cap = (unsigned int)std::min<size_t>((size_t)d.n1 * d.n2 * d.n3, 0xFFFFFFF0u);
-  CK(cudaMalloc(&c->d_fixrec, (size_t)c->fix_cap * sizeof(FixRec)));
   CK(cudaMalloc(&c->d_scal, 64 * sizeof(double)));
   CK(cudaMemset(c->d_scal, 0, 64 * sizeof(double)));
   c->d_dtslots = (unsigned long long*)(c->d_scal + 0);  // 6 slots
@@ -165,8 +167,8 @@ extern "C" int harm_b200_destroy(harm_ctx* c) {
   if (!c) return 0;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  void* ptrs[] = {c->d_geom, c->d_geomf, c->d_conn, c->d_aux, c->d_flux, c->d_emf, c->d_line, c->d_Paos,
-                  c->d_pk, c->d_U, c->d_rare, c->d_pflag, c->d_fixrec, c->d_scal, c->d_Pdev, c->d_mlp, c->d_wpg,
+  void* ptrs[] = {c->d_geom, c->d_geomf, c->d_conn, c->d_aux, c->d_flux, c->d_shared, c->d_coef, c->d_Paos,
+                  c->d_pk, c->d_U, c->d_rare, c->d_pflag, c->d_scal, c->d_Pdev, c->d_mlp, c->d_wpg,
                   c->d_mlp_master, c->d_mlp_adam, c->d_mlp_work};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -42,6 +42,7 @@ struct harm_ctx {
   void* d_flux;     // the arrays of the flux stage: d_F and d_edge, or d_Ff and d_edgef
   double* d_F[3];
   float* d_Ff[3];
+  void* d_shared;   // memory of d_line, d_emf / d_emff and d_fixrec, in use one after the other
   double* d_emf;
   float* d_emff;
   void* d_line;     // the flux stage's cell pass: WENO5 [9][cells], PARALINE [4][cells] (FP64 path:
