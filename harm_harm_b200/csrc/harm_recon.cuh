@@ -66,6 +66,7 @@ struct ReconWin {
   static constexpr int D = (LIM == HARM_LIM_WENO5) ? 5 : (LIM == HARM_LIM_MC) ? 1 : 2;
   static constexpr int W = (LIM == HARM_LIM_WENO5) ? 8 : 2 * D + 1;
   static constexpr bool S = (LIM == HARM_LIM_WENO5 || LIM == HARM_LIM_PARALINE);  // a per-cell coefficient
+  static constexpr int R = (LIM == HARM_LIM_PARALINE) ? 3 : D;  // the reach of edges and coefficient
 };
 
 // edges of the cell at y[0] by the limiters that need no weights
@@ -477,8 +478,9 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowBlocks<T>) k_recon_x1(Dims
 // ------------------------------------------------------------------ per-cell coefficients
 
 // S of direction DIR for edge cell t of a ReconBox, from the cell pass L (k_cellprep): the
-// strength of WENO5BND's momentum-flux reduction, or PARALINE's flattening coefficient
-template <int DIR, int LIM, typename T>
+// strength of WENO5BND's momentum-flux reduction, or PARALINE's flattening coefficient (CLAMP: as
+// k_recon's)
+template <int DIR, int LIM, typename T, bool CLAMP = false>
 __device__ __forceinline__ void recon_coef(const Dims& d, const ReconBox& rb, const double* __restrict__ P,
                                            const T* __restrict__ L, T* __restrict__ S, long long t) {
   const int nc = rb.c1 - rb.c0 + 1;
@@ -490,9 +492,8 @@ __device__ __forceinline__ void recon_coef(const Dims& d, const ReconBox& rb, co
   const int tt = rb.t0 + l % rb.nt, o = rb.o0 + l / rb.nt;
   const long long stride = (DIR == 1) ? 1 : (DIR == 2) ? (long long)d.n1e : (long long)d.plane;
   const size_t id = (DIR == 1) ? cidx(d, c, tt, o) : (DIR == 2) ? cidx(d, tt, c, o) : cidx(d, tt, o, c);
-  // the cell q further along the direction, or the grid's last one
-  const int cells_along = (DIR == 1) ? d.n1e : (DIR == 2) ? d.n2e : d.n3e;
-  auto along = [&](int q) { return id + (min(max(c + q, 0), cells_along - 1) - c) * stride; };
+  [[maybe_unused]] const int cells_along = (DIR == 1) ? d.n1e : (DIR == 2) ? d.n2e : d.n3e;
+  auto along = [&](int q) { return id + (CLAMP ? min(max(c + q, 0), cells_along - 1) - c : q) * stride; };
   if constexpr (LIM == HARM_LIM_WENO5) {
     const T* Lq = L + (size_t)3 * (DIR - 1) * d.cells;
     const T* ve = Lq + d.cells;
@@ -512,10 +513,10 @@ __device__ __forceinline__ void recon_coef(const Dims& d, const ReconBox& rb, co
     S[id] = paraline_fi<T>(v, pp);
   }
 }
-template <int DIR, int LIM, typename T, int TU = HARM_TU>
+template <int DIR, int LIM, typename T, bool CLAMP = false, int TU = HARM_TU>
 __global__ void __launch_bounds__(256) k_recon_coef(Dims d, ReconBox rb, const double* __restrict__ P,
                                                     const T* __restrict__ L, T* __restrict__ S) {
-  recon_coef<DIR, LIM, T>(d, rb, P, L, S, (long long)blockIdx.x * 256 + threadIdx.x);
+  recon_coef<DIR, LIM, T, CLAMP>(d, rb, P, L, S, (long long)blockIdx.x * 256 + threadIdx.x);
 }
 
 // ------------------------------------------------------------------ k_face
@@ -685,7 +686,7 @@ template <int DIR, int LIM>
 constexpr bool recon_may_be_narrow = DIR == 3 || LIM == HARM_LIM_MC || LIM == HARM_LIM_PARA;
 template <int DIR, int LIM>
 static inline bool recon_narrow(const Dims& d) {
-  return recon_may_be_narrow<DIR, LIM> && (DIR == 3 ? d.ng3 : d.ng) <= ReconWin<LIM>::D;
+  return recon_may_be_narrow<DIR, LIM> && (DIR == 3 ? d.ng3 : d.ng) <= ReconWin<LIM>::R;
 }
 
 // Cuts a box's lines into chunks and gives their number.  Each chunk costs its first cell's window
@@ -722,7 +723,10 @@ static inline cudaError_t launch_flux_dir(const Dims& d, const Phys& ph, const F
   T* ER = E + (size_t)NPR * d.cells;
   cudaError_t e;
   if constexpr (ReconWin<LIM>::S) {
-    k_recon_coef<DIR, LIM, T><<<nblk((long long)nc * rb.nlines), 256, 0, st>>>(d, rb, P, L, S);
+    auto k = k_recon_coef<DIR, LIM, T>;
+    if constexpr (DIR == 3)
+      if (recon_narrow<DIR, LIM>(d)) k = k_recon_coef<DIR, LIM, T, true>;
+    k<<<nblk((long long)nc * rb.nlines), 256, 0, st>>>(d, rb, P, L, S);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     launches++;
   }
