@@ -105,9 +105,9 @@ static int create_ctx(const harm_grid* g, int device, harm_ctx** out) {
   c->d_nhard = (unsigned int*)(c->d_scal + 26);
   c->d_status = (unsigned int*)(c->d_scal + SC_STATUS);
   {
-    // FP32 flux tiles: plain coalesced loads (default) or TMA ("tma"); both feed the same
-    // arithmetic.  The TMA-staged kernel measured slower on B200 (it needs ~120 registers for
-    // its tile loop, halving the warps that hide the face physics' latency), so it is opt-in.
+    // FP32 flux stage: the reconstruction and face kernels (default) or TMA-staged tiles ("tma"),
+    // with the same arithmetic.  The tiles are slower on B200 (they recompute their halos' weights,
+    // and need ~120 registers for the tile loop), so they are opt-in.
     const char* e = getenv("HARM_B200_FLUX_STAGING");
     c->flux_tma = (e && strcmp(e, "tma") == 0);
     // learned start: by default ("gated") only for the cells whose previous state is a poor

@@ -206,10 +206,12 @@ static inline FaceBox face_box(const Dims& d, int dir) {
 
 // ------------------------------------------------------------------ tiled flux kernel
 //
+// FP64, of the entry point that cannot have the edge values' memory (harm_noalloc_fp64.cu); its
+// tiles' geometry and WENO5 passes also serve the FP32 tiles of harm_flux_tma.cuh.
 // One block of 256 threads = a tile of A = 32 faces of direction DIR times NT = 8 transverse
 // lines, consecutive threads along i so that every global load is coalesced.  VB primitives
-// at a time (all 8 in FP32, 4 in FP64) are staged in shared memory with the stencil halo along
-// DIR; the block then computes every cell's reconstruction once (MC slope, para4, the WENO5
+// at a time (4; in FP32 all 8) are staged in shared memory with the stencil halo along DIR; the
+// block then computes every cell's reconstruction once (MC slope, para4, the WENO5
 // weights and then the edge values, or PARALINE's edges after a pass that computes each
 // staged cell's V and total pressure and each edge cell's flattening coefficient), three
 // barriers per group instead of three per primitive.
@@ -419,7 +421,7 @@ __device__ __forceinline__ void weno_tile_edges(const T* s_y, T* s_w, T* s_el, T
 }
 
 
-// The face physics of k_fluxt: B^DIR continuity, limit_gamma, states, fluxes, wave speeds and
+// The FP64 face physics: B^DIR continuity, limit_gamma, states, fluxes, wave speeds and
 // the HLL flux of one face (flux.c:852, vchar.c:34; LAXF where both speeds vanish or where
 // fluxmethod is LAXF, fluxcompute.c:243) into F at `id`; returns ctop.
 template <int DIR, typename T, typename GT>
@@ -467,9 +469,8 @@ __device__ __forceinline__ double face_dt(const Phys& ph, double ctop) {
   return (dtij > 0.0) ? dtij : 1.e300;
 }
 
-// HARM_FLUXT_MINB: resident blocks per SM the tiled flux kernel is compiled for (the mixed
-// path's FP32 tiles: 3, at most 85 registers with every staging load in flight; the FP64
-// tiles: 2, 128 registers with spills, faster than the ~160 registers and 1 block per SM the
+// HARM_FLUXT_MINB (harm_noalloc_fp64.cu): resident blocks per SM the tiled flux kernel is compiled
+// for (2: 128 registers with spills, faster than the ~160 registers and 1 block per SM the
 // compiler picks on its own); unset, the compiler's choice
 #ifdef HARM_FLUXT_MINB
 #define HARM_FLUXT_LB __launch_bounds__(256, HARM_FLUXT_MINB)
@@ -794,7 +795,7 @@ static inline cudaError_t launch_cellprep(const Dims& d, const Phys& ph, const d
 }
 
 // launch k_fluxt<DIR, LIM, T, GT>; the first launch of an instantiation on a device raises
-// its dynamic shared-memory limit where the tile needs more than 48 KB (FP32 WENO5: 63 KB)
+// its dynamic shared-memory limit where the tile needs more than 48 KB (WENO5: 72 KB)
 template <int DIR, int LIM, typename T, typename GT>
 static inline cudaError_t launch_fluxt(const Dims& d, const Phys& ph, const FaceBox& fb, const double* P,
                                        const GT* geom, T* F, unsigned long long* dtslot, cudaStream_t st) {

@@ -118,35 +118,15 @@ __device__ __forceinline__ void recips(double b0, double b1, double b2, double& 
   y1 = recip_fix(b1, r2 * b0);
   y2 = recip_fix(b2, r * b01);
 }
-__device__ __forceinline__ void recips(float b0, float b1, float& y0, float& y1) {
-  y0 = __fdividef(1.0f, b0);
-  y1 = __fdividef(1.0f, b1);
-}
-__device__ __forceinline__ void recips(float b0, float b1, float b2, float& y0, float& y1, float& y2) {
-  recips(b0, b1, y0, y1);
-  y2 = __fdividef(1.0f, b2);
-}
 
-// Several values over one denominator: one reciprocal, FP64 with the quotients corrected.
+// Several values over one denominator: one reciprocal, the quotients corrected (FP64 only).
 template <typename T>
 struct WScale {
+  static_assert(sizeof(T) == 8, "the FP32 forms are harm_weno_f32x2.cuh's and harm_face_f32x2.cuh's");
   T d, y;
   __device__ __forceinline__ explicit WScale(T den) : d(den), y(T(1) / den) {}
   __device__ __forceinline__ WScale(T den, T rec) : d(den), y(rec) {}
   __device__ __forceinline__ T operator()(T a) const { return div_by(a, d, y); }
-};
-template <>
-struct WScale<float> {
-  float r;
-  __device__ __forceinline__ explicit WScale(float den) {
-#ifdef __CUDA_ARCH__
-    r = __fdividef(1.0f, den);
-#else
-    r = 1.0f / den;  // host pass only parses this; the kernels use the line above
-#endif
-  }
-  __device__ __forceinline__ WScale(float, float rec) : r(rec) {}
-  __device__ __forceinline__ float operator()(float a) const { return a * r; }
 };
 
 template <typename T>
@@ -486,9 +466,10 @@ __device__ __forceinline__ T symsum2(T a0, T a1) {
   return s;
 }
 
-// Division inside the WENO weights.  FP64: IEEE division (the oracle's operations).  FP32
-// (mixed path): the fast reciprocal-multiply form, error of 2 ulp; the weights only steer the
-// stencil combination, so this stays far inside the FP32 reconstruction's own rounding.
+// Division inside the WENO weights.  FP64: IEEE division (the oracle's operations).  FP32 (the
+// lower-order fractions next to a jump in the TMA-staged tiles): the fast reciprocal-multiply
+// form, error of 2 ulp; the fractions only steer the stencil combination, so this stays far
+// inside the FP32 reconstruction's own rounding.
 template <typename T>
 __device__ __forceinline__ T wdiv(T a, T b) {
   return a / b;
@@ -512,20 +493,10 @@ __device__ __forceinline__ float wdivk<float>(float a, float b) {
 template <typename T>
 __device__ __forceinline__ T limit_weight(int order, T w) {
   const T avg = T(1) / T(order), w1 = T(0.2) * avg, w2 = (T(1) - T(0.2)) * avg, w3 = (T(1) + T(0.2)) * avg, w4 = T(1);
-  if constexpr (sizeof(T) == 4) {
-    // FP32: the limiter is continuous and piecewise linear, 0 | ramp to avg | avg | ramp to 1,
-    // so it is the lower ramp clamped to [0, avg] plus the part of the upper ramp above avg:
-    // min/max instead of compares and selects, no divergent branches (the same values away
-    // from the break points, within a rounding at them)
-    const T lo = wdivk<T>(avg * (w - w1), w2 - w1);
-    const T up = wdivk<T>((w - w3) * (w4 - avg), w4 - w3);
-    return fmaxf(fminf(lo, avg), T(0)) + fmaxf(up, T(0));
-  } else {
-    if (w < w1) return T(0);
-    if (w < w2) return wdivk<T>(avg * (w - w1), w2 - w1);
-    if (w < w3) return avg;
-    return wdivk<T>((w - w3) * (w4 - avg), w4 - w3) + avg;
-  }
+  if (w < w1) return T(0);
+  if (w < w2) return wdivk<T>(avg * (w - w1), w2 - w1);
+  if (w < w3) return avg;
+  return wdivk<T>((w - w3) * (w4 - avg), w4 - w3) + avg;
 }
 
 // unoptimised (limited, normalised) weights of the three 3-point stencils of the cell at u

@@ -1,16 +1,17 @@
 // harm_flux_tma.cuh -- the FP32 flux kernel with its stencil tiles staged by TMA.
 //
-// Same tiles and arithmetic as k_fluxt<DIR, LIM, float> (harm_common.cuh), organised as a
-// persistent kernel: each block walks the tiles of a direction; one thread loads a tile's
+// k_fluxt's tiles (harm_common.cuh) in FP32, with the packed WENO5 and face arithmetic of
+// harm_weno_f32x2.cuh and harm_face_f32x2.cuh, as a persistent kernel: each block walks the tiles of a direction; one thread loads a tile's
 // 8 primitives with a single 4-D cp.async.bulk.tensor (x = i, y = j, z = k, w = primitive,
 // zero fill outside the extended grid) completing on an mbarrier, and the load of the next
 // tile is in flight while the block converts, reconstructs and evaluates the current one.
 // The TMA x coordinate (i) must start on a 16-byte boundary, so the box starts at the even
 // i at or below the first staged cell and is one or two doubles wider; the conversion pass
 // reads it from that offset.  Requires 16-byte aligned P and an even n1e (the row pitch is a
-// multiple of 16 bytes); other layouts use k_fluxt.  Opt-in (HARM_B200_FLUX_STAGING=tma): on
-// B200 the staging is not what bounds the flux stage (the WENO5 arithmetic and the face
-// physics are), and the tile loop's registers cost occupancy, so k_fluxt is the default.
+// multiple of 16 bytes); other layouts use the reconstruction and face kernels of
+// harm_recon.cuh, which are the default: the WENO5 arithmetic and the face physics bound the flux
+// stage, not the staging, and tiles compute a quarter more cells' weights.  Opt-in
+// (HARM_B200_FLUX_STAGING=tma).
 #pragma once
 #include <cuda.h>
 #include "harm_async.cuh"

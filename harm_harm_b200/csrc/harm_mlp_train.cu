@@ -3,7 +3,7 @@
 // Training runs in FP32 with hand-written kernels:
 //   k_mlp_grad   forward and backward pass of the 10-64-64-64-2 SiLU network over a
 //                minibatch; each block owns a slice of the samples, keeps the parameters and
-//                activations in shared memory (181 KB) and its gradients in registers, and
+//                activations in shared memory (147 KB) and its gradients in registers, and
 //                writes one partial gradient, so the reduction order is fixed
 //                (deterministic gradients);
 //   k_mlp_adam   sums the partial gradients in a fixed order and applies Adam;

@@ -21,10 +21,12 @@
 //     cudaGetSymbolAddress (with that device current) and caches it;
 //   - the call is synchronous: it copies the CFL minima back to the host and waits for its
 //     own stream before returning ndt.
-// The kernels are the FP64 path's, compiled the same way (no FMA contraction), so the
-// results equal harm_b200_fluxcalc's.
+// The reconstruction and face kernels of harm_b200_fluxcalc keep the edge values of every cell in
+// memory, which this entry point cannot have, so it has a kernel of its own that keeps them in
+// shared memory (k_fluxt, harm_common.cuh); its arithmetic is the same, compiled the same way (no
+// FMA contraction), and so are its results.
 #ifndef HARM_FLUXT_MINB
-#define HARM_FLUXT_MINB 2  // the FP64 flux tiles at 2 blocks per SM, as in harm_path_fp64.cu
+#define HARM_FLUXT_MINB 2  // the flux tiles at 2 blocks per SM
 #endif
 #include <mutex>
 #include "harm_common.cuh"
@@ -66,7 +68,7 @@ static int noalloc_scratch(double** emf, unsigned long long** dtmin) {
   return 0;
 }
 
-// the three directions with the FP64 path's tile kernel (the first launch of an instantiation
+// the three directions with the tile kernel (the first launch of an instantiation
 // on a device raises its shared-memory limit where the tile needs more than 48 KB)
 template <int LIM>
 static cudaError_t noalloc_dirs(const Dims& d, const Phys& ph, const double* geom, const double* pb, double* F1,

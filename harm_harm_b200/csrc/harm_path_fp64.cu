@@ -3,9 +3,11 @@
 // inversions.
 //
 // harm_path_fp64fma.cu compiles this file's flux and update launchers a second time, with
-// FMA contraction and the inversion's shared reciprocals (HARM_FP64_FMA_TU): the FP64 path as
-// fast as the compiler makes it, for comparisons of speed (HARM_PREC_FP64_FMA); this build
-// (HARM_PREC_FP64) performs the CPU restatement's IEEE operations in its order.
+// FMA contraction and the fast divisions of harm_device.cuh (HARM_FP64_FMA_TU): the FP64 path as
+// fast as the compiler makes it, for comparisons of speed (HARM_PREC_FP64_FMA).  This build
+// (HARM_PREC_FP64) performs the CPU restatement's operations in its order, with IEEE divisions, but
+// for the quotients of the reconstruction and of the faces that div_by and recips form: the IEEE
+// value too, unless the exact one lies within some 1e-15 ulp of the middle of two doubles.
 #include <algorithm>
 #include "harm_common.cuh"
 #include "harm_recon.cuh"

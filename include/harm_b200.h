@@ -62,11 +62,16 @@ enum { HARM_LIM_MC = 0, HARM_LIM_PARA = 1, HARM_LIM_WENO5 = 2, HARM_LIM_PARALINE
    where both wave speeds vanish, or LAXF (Rusanov) everywhere */
 enum { HARM_FLUX_HLL = 0, HARM_FLUX_LAXF = 1 };
 
-/* arithmetic of the flux path: FP64 everywhere in the IEEE operations of the reference's C
-   in its order (HARM_PREC_FP64, no FMA contraction), FP32 reconstruction/HLL/CT with the
-   conserved update, inversion and metric kept in FP64 (HARM_PREC_MIXED), or FP64 everywhere
-   compiled with FMA contraction and the inversion's shared reciprocals (HARM_PREC_FP64_FMA:
-   round-off-level differences from HARM_PREC_FP64; the FP64 path at its best speed) */
+/* arithmetic of the flux path: FP64 everywhere in the operations of the reference's C in its
+   order (HARM_PREC_FP64, no FMA contraction; divisions IEEE, or in the reconstruction and the
+   face fluxes quotients from a shared reciprocal corrected by their remainder, which differ from
+   IEEE ones only within some 1e-15 ulp of the middle of two doubles), FP32
+   reconstruction/HLL/CT with the conserved update, inversion and metric kept in FP64
+   (HARM_PREC_MIXED), or FP64 everywhere compiled with FMA contraction (HARM_PREC_FP64_FMA:
+   round-off-level differences from HARM_PREC_FP64; the FP64 path at its best speed).  The last
+   two form the cell states' and the inversion's FP64 quotients from a refined hardware
+   reciprocal, corrected likewise, and inside the Newton iteration, where several divisors share
+   one, to an ulp or two */
 enum { HARM_PREC_FP64 = 0, HARM_PREC_MIXED = 1, HARM_PREC_FP64_FMA = 2 };
 
 /* initial guess of the Newton inversion: the previous primitive (set_guess_Wp,
