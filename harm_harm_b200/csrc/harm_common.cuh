@@ -179,16 +179,18 @@ struct FaceBox {
 
 // Grids whose flux stage takes the three directions in one launch per kernel (harm_recon.cuh), with
 // edge values and coefficients of all three.  A launch that waits for the one before costs three to
-// four microseconds, and a small grid leaves most of the chip idle in each, so the line lies where
-// the joint kernels' larger code and registers cost more.  Full steps, one launch per direction
-// against joint, us, by extended cells:
+// four microseconds, and its last blocks leave the chip idle, so the line lies where the joint
+// kernels' larger code and registers, and three directions' edge values in the L2, cost more.  Full
+// steps, one launch per direction against joint, us, by extended cells:
 //   FP64 WENO5 27 k 550 / 409, 64 k 576 / 488, 112 k 587 / 572, but a 2-D one of 87 k 551 / 562 and
 //   200 k 727 / 813 (its x1 rows take three blocks per SM and 80 registers by themselves);
-//   the others gain up to the largest tried: mixed WENO5 200 k 422 / 380, 358 k 567 / 546, mixed MC
-//   161 k 303 / 278, 297 k 412 / 389, FP64 MC 161 k 384 / 372, 270 k 510 / 507, PARALINE 297 k
-//   mixed 492 / 452, FP64 677 / 646.
+//   mixed WENO5 200 k 422 / 380, 358 k 567 / 546, 808 k 970 / 918, 1.2 M 1302 / 1284, but 1.7 M
+//   1687 / 1723; the others mixed MC 161 k 303 / 278, 705 k 634 / 608, 1.5 M 1137 / 1120, FP64 MC
+//   161 k 384 / 372, 705 k 998 / 961, PARALINE mixed 297 k 492 / 452, 705 k 763 / 708, FP64 705 k
+//   1150 / 1093, 1.5 M 2367 / 2352.
+// The line of a million cells also keeps the two directions' further edge values to 256 MB.
 static inline bool one_launch_fluxes(const Dims& d, int lim, bool fp64) {
-  return d.cells <= ((lim == HARM_LIM_WENO5 && fp64) ? 72000 : 360000);
+  return d.cells <= ((lim == HARM_LIM_WENO5 && fp64) ? 72000 : 1000000);
 }
 
 static inline FaceBox face_box(const Dims& d, int dir) {

@@ -19,9 +19,8 @@ from harm_harm_b200 import _native as N
 from oracle import oracle as O
 
 SHAPES = [(5, 7, 1), (59, 9, 1), (33, 21, 6), (64, 13, 7), (131, 8, 12), (17, 70, 9)]
-# grids beyond the size up to which the three directions share their launches; (41, 45, 37) is beyond
-# it for FP64 WENO5 alone
-LARGE = [(131, 70, 33), (29, 37, 230), (790, 480, 1)]
+# larger ones, of which (41, 45, 37) takes a launch per direction for FP64 WENO5 and the last two do for all
+LARGE = [(131, 70, 33), (29, 37, 230), (41, 45, 37), (133, 70, 90), (1390, 740, 1)]
 
 
 def _faces(g, d):
@@ -32,7 +31,7 @@ def _faces(g, d):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("lim", [0, 1, 2, 3])
-@pytest.mark.parametrize("shape", SHAPES + LARGE + [(41, 45, 37)])
+@pytest.mark.parametrize("shape", SHAPES + LARGE)
 def test_flux_edges(cuda, shape, lim):
     g, geom, conn, aux, P = make_torus(*shape, lim=lim)
     plant_compression(g, P)
