@@ -13,9 +13,10 @@
 // weight through shared memory.  The edge values cost a round trip through memory that the
 // arithmetic hides.  The warps of a block are one primitive: a primitive whose lines take a
 // slower path (zero lines, steep ones) holds up no other's.
-// Measured per substep against the tiles it replaces: FP32 WENO5 at 256x128x64 1221 -> 756 us
-// (recon 159 + 164 + 174, faces 3 x 54, cell pass and coefficients 97), FP64 WENO5 at 192x96x64 3.6 -> 1.9 ms; FP32 PARALINE at 192x96x64 388
-// -> 310 us.
+// Flux stage of a substep (EMFs included) against the tiles it replaces: FP32 WENO5 at 256x128x64
+// 1214 -> 756 us (recon 143 + 161 + 166, faces 3 x 48, cell pass and coefficients 97), FP64 WENO5 at
+// 192x96x64 3550 -> 1412 us, FP32 PARALINE at 192x96x64 404 -> 337 us; with the three directions in
+// joint launches FP32 WENO5 at 120x72x40 287 -> 195 us (212 with separate ones).
 #pragma once
 #include "harm_common.cuh"
 #include "harm_face_f32x2.cuh"

@@ -1,9 +1,10 @@
-"""Utoprimgen over points at the sizes where the split into a common kernel and one for the rest can
-go wrong: one point, the edges of a block of 128 and of a window of 1024 flags, several windows per
-block, and sets dense in points that do not converge within the common kernel's steps (low u/rho at high B^2/rho, whose
-residual rounds more coarsely than the test) or that the hot inversion cannot invert.  FP64 against
-the oracle point by point: the same flags, primitives to 1e-9 of each point's largest (W' of the
-slow points is only defined to 1e-12 of D, 1e-6 of itself and of u)."""
+"""Utoprimgen over points at the sizes where its kernels can go wrong: one point, the edges of a block
+of 128, the line between the one kernel for few points and the two for many, several windows of 1024
+flags per block of the second, and sets dense in points that do not converge within the first's
+steps (low u/rho at high B^2/rho, whose residual rounds more coarsely than the test) or that the hot
+inversion cannot invert.  FP64 against the oracle point by point: the same flags, primitives to 1e-9
+of each point's largest (W' of the slow points is only defined to 1e-12 of D, 1e-6 of itself and of
+u)."""
 import numpy as np
 import pytest
 
@@ -50,18 +51,21 @@ def test_points(cuda, n, kind):
         assert (flag != 0).any()
 
 
+@pytest.mark.parametrize("per_sm,more", [(512, 0), (512, 1), (2 * 2 * 1024, 517)])
 @pytest.mark.parametrize("dense", [0.02, 0.7])
-def test_points_over_several_windows(cuda, dense):
-    """More points than two windows per block: what a block's list carries from one window into the
-    next, full passes with windows still to come (dense) and lists that fill over all of them
-    (sparse).  Slow, failing and plain points, checked against the oracle once, at random places: the
-    kernels' operations on a point do not depend on its place, so its copies are equal bit for bit."""
+def test_many_points(cuda, dense, per_sm, more):
+    """The most points that one kernel takes, the fewest that two do (a window of the second with a
+    remainder), and more than two windows per block of the second: what a block's list carries from
+    one window into the next, full passes with windows still to come (dense) and lists that fill over
+    all of them (sparse).  Slow, failing and plain points, checked against the oracle once, at random
+    places: the kernels' operations on a point do not depend on its place, so its copies are equal bit
+    for bit."""
     g, geom, conn, aux, _ = make_torus(16, 16, 1)
     sets = [_points(g, geom, m, kind, seed=m) for m, kind in ((700, "plain"), (150, "slow"), (400, "failing"))]
     U, rec, guess = (np.concatenate([s[q] for s in sets], axis=1) for q in range(3))
     ref = [O.utoprimgen_point(g, np.ascontiguousarray(rec[:, k]), U[:, k], guess[:, k]) for k in range(U.shape[1])]
-    Pr, fr, ir = (np.array([r[q] for r in ref]) for q in range(3))
-    n = 2 * 2 * cuda.cuda.get_device_properties(0).multi_processor_count * 1024 + 517
+    Pr, fr = (np.array([r[q] for r in ref]) for q in range(2))
+    n = per_sm * cuda.cuda.get_device_properties(0).multi_processor_count + more
     rng = np.random.default_rng(11)
     at = np.where(rng.random(n) < dense, rng.integers(700, U.shape[1], n), rng.integers(0, 700, n))
     idx = cuda.from_numpy(at).cuda()
