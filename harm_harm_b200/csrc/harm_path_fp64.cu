@@ -368,9 +368,8 @@ __global__ void k_bound_x3(Dims d, double* P, int8_t* flag) {
   int ii = (int)(t % d.n1e);
   long long r = t / d.n1e;
   int jj = (int)(r % d.n2e), gq = (int)(r / d.n2e);
-  int kk, ks;
-  if (gq < d.ng3) { kk = gq; ks = kk + d.n3; }
-  else { kk = d.ng3 + d.n3 + (gq - d.ng3); ks = kk - d.n3; }
+  // the active plane it repeats: with n3 < ng3 the plane n3 away is a ghost plane of this launch
+  const int kk = (gq < d.ng3) ? gq : gq + d.n3, ks = d.ng3 + ((kk - d.ng3) % d.n3 + d.n3) % d.n3;
   size_t dst = cidx(d, ii, jj, kk), src = cidx(d, ii, jj, ks);
   if (flag) flag[dst] = flag[src];
   if (P)

@@ -1,8 +1,9 @@
 """bound_prim's single launch and its per-direction path at the edges of their ranges, against the
-oracle: the smallest grids either takes (n2 = ng + 1 and n3 = ng for the single launch, n2 = ng
-for the other), one plane and several.  FP64 in the oracle's operations: equal to the last bits
-of the math library's log and exp.  With n2 = ng the outermost polar ghost row mirrors the other
-pole's first row, which the oracle has already rewritten there: it is left out."""
+oracle: the smallest grids either takes (n2 = ng + 1 and n3 = ng for the single launch, n2 = ng or
+n3 < ng for the other, whose outer x3 ghost planes repeat planes that are ghosts of ghosts), one
+plane and several.  FP64 in the oracle's operations: equal to the last bits of the math library's
+log and exp.  With n2 = ng the outermost polar ghost row mirrors the other pole's first row, which
+the oracle has already rewritten there: it is left out."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n1,n2,n3,lim", [(3, 5, 1, 0), (5, 7, 6, 2), (37, 9, 4, 0), (16, 12, 7, 2), (130, 33, 1, 2),
-                                          (9, 4, 1, 0), (12, 6, 8, 2)])
+                                          (9, 4, 1, 0), (12, 6, 8, 2), (20, 9, 3, 1), (33, 15, 2, 2)])
 def test_bound_edges(cuda, n1, n2, n3, lim):
     g, geom, conn, aux, P = make_torus(n1, n2, n3, lim=lim)
     rng = np.random.default_rng(n1)
